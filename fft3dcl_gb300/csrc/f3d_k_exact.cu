@@ -29,21 +29,84 @@ struct Cfg {
   static constexpr int THREADS = TPB > 128 ? TPB : 128;
   static constexpr int BPC = THREADS / TPB;           // blocks per CTA
   static constexpr int TS = BW + 1;                   // padded row stride
-  static constexpr int FWD_FLOATS = BH * TS + 2 * PS; // input tile + row spectra
-  static constexpr int INV_FLOATS = 2 * PS + 2 * BH * TS;
+  // Shared memory of a block (a multiple of 4 floats): the input tile, then
+  // the row spectra; the filtered spectrum, then the column results.
+  static constexpr int even4(int n) { return (n + 3) / 4 * 4; }
+  static constexpr int FWD_FLOATS = even4(BH * TS > 2 * PS ? BH * TS : 2 * PS);
+  static constexpr int INV_FLOATS = even4(2 * PS > 2 * BH * TS ? 2 * PS : 2 * BH * TS);
   // Loads in flight per thread: the gather takes GB samples (and window
   // values) per round, the Kalman filter KB bins (spectrum, state, tables)
   // before any of their results is stored.
   static constexpr int GB = BW * BH / TPB < 16 ? BW * BH / TPB : 16;
   static constexpr int NJ = (PS + TPB - 1) / TPB;
   static constexpr int KB = NJ < 8 ? NJ : 8;
+  // Resident CTAs per SM the register budget is set for (a transform of TPB
+  // values holds 2 TPB registers).
+  static constexpr int FWD_CTAS = TPB == 64 ? 3 : 6;
+  static constexpr int INV_CTAS = TPB == 64 ? 3 : 5;  // Kalman: one fewer at TPB < 64
 };
 
-// One block: gather with mirror addressing, convert, subtract chroma
-// centering, analysis window (src/cpu/reference.cpp:140-159); row FFTs then
-// the fbw kept column FFTs (src/cpu/fft.cpp:68-86); store the half spectrum.
+// Threads of one block: a block of up to 32 threads lives in one warp.
+template <int TPB>
+__device__ __forceinline__ void block_sync() {
+  if constexpr (TPB <= 32) __syncwarp();
+  else __syncthreads();
+}
+
+// Gather of a block with mirror addressing, sample conversion, chroma
+// centering and analysis window (src/cpu/reference.cpp:140-159) into
+// tile[BH][TS]. Thread t of TPB (a multiple of BW) keeps one column and takes
+// every (TPB / BW)-th row, GB rows in flight. The sample format is fixed
+// outside the loops and blocks inside the plane need no mirroring: with the
+// format switch and the mirror inside the unrolled loop the code was large
+// enough for instruction fetch to stall the kernels (forward, 1080p 10-bit
+// with 32x32 blocks: 53 -> 20 us; 720p float with 64x64 blocks: 30 -> 18 us).
+template <int BW, int BH, int TPB, int GB, int TS, int FMT>
+__device__ __forceinline__ void gather_fmt(const FwdArgs& a, int bx, int by, int t, float* tile) {
+  constexpr int RS = TPB / BW, NR = BH / RS;  // rows per round, rounds
+  static_assert(TPB % BW == 0 && BH % RS == 0 && NR % GB == 0, "row split");
+  const int lx = t % BW, ly0 = t / BW;
+  const float* win = a.win + t;
+  float* dst = tile + ly0 * TS + lx;
+  if (bx >= 0 && by >= 0 && bx + BW <= a.g.W && by + BH <= a.g.H) {
+    const uint8_t* row = a.src + (long long)(by + ly0) * a.pitch;
+    for (int k0 = 0; k0 < NR; k0 += GB) {
+      float v[GB], w[GB];
+#pragma unroll
+      for (int u = 0; u < GB; u++) {
+        v[u] = load_sample(row + (long long)((k0 + u) * RS) * a.pitch, bx + lx, FMT, a.norm);
+        w[u] = win[(k0 + u) * TPB];
+      }
+#pragma unroll
+      for (int u = 0; u < GB; u++) {
+        const float c = v[u] - a.chroma_norm;
+        dst[(k0 + u) * RS * TS] = c * w[u];
+      }
+    }
+  } else {
+    const int x = mirror_i(bx + lx, a.g.W);
+#pragma unroll 4
+    for (int k = 0; k < NR; k++) {
+      const int y = mirror_i(by + ly0 + k * RS, a.g.H);
+      const float c = load_sample(a.src + (long long)y * a.pitch, x, FMT, a.norm) - a.chroma_norm;
+      dst[k * RS * TS] = c * win[k * TPB];
+    }
+  }
+}
+template <int BW, int BH, int TPB, int GB, int TS>
+__device__ __forceinline__ void gather_block(const FwdArgs& a, int b, int t, float* tile) {
+  int bx, by, par;
+  block_origin(a.g, b, bx, by, par);
+  if (a.fmt == FMT_U8) gather_fmt<BW, BH, TPB, GB, TS, FMT_U8>(a, bx, by, t, tile);
+  else if (a.fmt == FMT_U16) gather_fmt<BW, BH, TPB, GB, TS, FMT_U16>(a, bx, by, t, tile);
+  else gather_fmt<BW, BH, TPB, GB, TS, FMT_F32>(a, bx, by, t, tile);
+}
+
+// One block: gather, row FFTs, then the fbw kept column FFTs
+// (src/cpu/fft.cpp:68-86); store the half spectrum. The row spectra take the
+// input tile's place: every row is in registers before any is written.
 template <int BW, int BH>
-__global__ void __launch_bounds__(Cfg<BW, BH>::THREADS)
+__global__ void __launch_bounds__(Cfg<BW, BH>::THREADS, Cfg<BW, BH>::FWD_CTAS)
     k_forward_exact(const __grid_constant__ FwdArgs a) {
   using C = Cfg<BW, BH>;
   extern __shared__ float4 smem4[];
@@ -52,67 +115,121 @@ __global__ void __launch_bounds__(Cfg<BW, BH>::THREADS)
   const int b = blockIdx.x * C::BPC + slot;
   const bool valid = b < a.g.nb;
   float* tile = smem + slot * C::FWD_FLOATS;
-  float2* rows = reinterpret_cast<float2*>(tile + BH * C::TS);
+  float2* rows = reinterpret_cast<float2*>(tile);
+  float2* out = a.spec + (size_t)b * C::PS;
 
-  if (valid) {
-    int bx, by, par;
-    block_origin(a.g, b, bx, by, par);
-    const bool inside = bx >= 0 && by >= 0 && bx + BW <= a.g.W && by + BH <= a.g.H;
-    for (int i0 = 0; i0 < BW * BH; i0 += C::GB * C::TPB) {
-      float v[C::GB], w[C::GB];
+  if (valid) gather_block<BW, BH, C::TPB, C::GB, C::TS>(a, b, t, tile);
+  block_sync<C::TPB>();
+  static_assert(C::TPB >= BH && C::TPB >= C::FBW, "one row, one column per thread");
+  {
+    float2 v[BW];
+    if (t < BH) {
 #pragma unroll
-      for (int u = 0; u < C::GB; u++) {
-        const int idx = i0 + t + u * C::TPB;
-        if (idx >= BW * BH) continue;
-        const int ly = idx / BW, lx = idx - ly * BW;
-        const int y = inside ? by + ly : mirror_i(by + ly, a.g.H);
-        const int x = inside ? bx + lx : mirror_i(bx + lx, a.g.W);
-        v[u] = load_sample(a.src + (long long)y * a.pitch, x, a.fmt, a.norm);
-        w[u] = a.win[idx];
-      }
-#pragma unroll
-      for (int u = 0; u < C::GB; u++) {
-        const int idx = i0 + t + u * C::TPB;
-        if (idx >= BW * BH) continue;
-        const int ly = idx / BW, lx = idx - ly * BW;
-        const float c = v[u] - a.chroma_norm;
-        tile[ly * C::TS + lx] = c * w[u];
-      }
+      for (int c = 0; c < BW; c++) v[c] = make_float2(tile[t * C::TS + c], 0.0f);
     }
-  }
-  __syncthreads();
-  if (valid) {
-    for (int r = t; r < BH; r += C::TPB) {
-      float2 v[BW];
-#pragma unroll
-      for (int c = 0; c < BW; c++) v[c] = make_float2(tile[r * C::TS + c], 0.0f);
+    block_sync<C::TPB>();
+    if (t < BH) {
       fft_r2<BW, false>(v, a.tw.row);
 #pragma unroll
-      for (int c = 0; c < C::FBW; c++) rows[r * C::FBW + c] = v[c];
+      for (int c = 0; c < C::FBW; c++) rows[t * C::FBW + c] = v[c];
     }
   }
-  __syncthreads();
-  if (valid) {
-    float2* out = a.spec + (size_t)b * C::PS;
-    for (int c = t; c < C::FBW; c += C::TPB) {
-      float2 v[BH];
+  block_sync<C::TPB>();
+  if (valid && t < C::FBW) {
+    float2 v[BH];
 #pragma unroll
-      for (int r = 0; r < BH; r++) v[r] = rows[r * C::FBW + c];
-      fft_r2<BH, false>(v, a.tw.col);
+    for (int r = 0; r < BH; r++) v[r] = rows[r * C::FBW + t];
+    fft_r2<BH, false>(v, a.tw.col);
 #pragma unroll
-      for (int r = 0; r < BH; r++) out[r * C::FBW + c] = v[r];
+    for (int r = 0; r < BH; r++) out[r * C::FBW + t] = v[r];
+  }
+}
+
+// The filtered half spectrum of block b (temporal filter + sharpen per bin,
+// src/cpu/reference.cpp:246-409) into F[PS]. NB bins' window spectra (Kalman:
+// and state and tables) are loaded before any of them is filtered: the
+// compiler cannot move a bin's loads above the previous bin's state stores,
+// and the loads of one bin alone leave the memory system idle.
+template <int BM, int PS, int TPB, int NB>
+__device__ __forceinline__ void filter_block(const InvArgs& a, int b, int t, float2* F) {
+  constexpr int NJ = (PS + TPB - 1) / TPB;
+  const size_t base = (size_t)b * PS;
+  const float dc = block_dc(a, b);
+  for (int j0 = 0; j0 < NJ; j0 += NB) {
+    float2 sv[NB][4];
+    KState ks[NB];
+    BinTables tb[NB];
+#pragma unroll
+    for (int u = 0; u < NB; u++) {
+      const int i = t + (j0 + u) * TPB;
+      if (j0 + u >= NJ || i >= PS) continue;
+      load_window<BM>(a, base + i, sv[u]);
+      if (BM == 0) ks[u] = load_kstate(a, base + i);
+      if (BM == 0) tb[u] = bin_tables(a, i);
     }
+#pragma unroll
+    for (int u = 0; u < NB; u++) {
+      const int i = t + (j0 + u) * TPB;
+      if (j0 + u >= NJ || i >= PS) continue;
+      F[i] = filter_vals_ks<BM>(a, dc, BM == 0 ? tb[u] : bin_tables(a, i), base + i, sv[u], ks[u]);
+    }
+  }
+}
+
+// The temporal mode as a template argument (square blocks: one copy of the
+// filter for each mode, of which a launch runs one) or read per bin.
+template <bool KALMAN, bool BY_MODE, int PS, int TPB, int KB>
+__device__ __forceinline__ void filter_block_any(const InvArgs& a, int b, int t, float2* F) {
+  constexpr int KN = 4;  // bins in flight, temporal modes
+  if constexpr (KALMAN) {
+    filter_block<0, PS, TPB, KB>(a, b, t, F);
+  } else if constexpr (BY_MODE) {
+    switch (a.bm) {
+    case 4: filter_block<4, PS, TPB, KN>(a, b, t, F); break;
+    case 3: filter_block<3, PS, TPB, KN>(a, b, t, F); break;
+    case 2: filter_block<2, PS, TPB, KN>(a, b, t, F); break;
+    case 1: filter_block<1, PS, TPB, KN>(a, b, t, F); break;
+    default: filter_block<-1, PS, TPB, KN>(a, b, t, F);
+    }
+  } else {
+    filter_block<kRuntimeBm, PS, TPB, KN>(a, b, t, F);
+  }
+}
+
+// Starts the window spectra of block b moving into L2 (one thread's call).
+template <int PS>
+__device__ __forceinline__ void prefetch_window(const InvArgs& a, int b) {
+  const int nf = a.bm >= 2 ? a.bm : 1;
+  for (int k = 0; k < nf; k++)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.s[k] + (size_t)b * PS), "r"(PS * 8) : "memory");
+}
+
+// Rows of a block's windowed inverse: sample pair j of row r (its two values
+// before the window) at S[r * TS + at(j)], written by the threads of the row
+// transforms, read back here in plane order, so that the window is read and
+// the block written in whole lines. Stored straight from the row transforms
+// each thread walks its own row: 16 to 32 lines per request, and the loads
+// and stores of the block took half of the kernel (inverse, 1080p 10-bit bt=4
+// with 32x32 blocks: 180 -> 99 us; 720p Kalman with 64x64 blocks: 60 -> 35 us).
+template <int BW, int BH, int TPB, int TS, class At>
+__device__ __forceinline__ void store_block(const InvArgs& a, int b, int t, const float2* S, At&& at) {
+  int bx, by, par;
+  block_origin(a.g, b, bx, by, par);
+  const float2* win = reinterpret_cast<const float2*>(par ? a.win_b : a.win_a);
+  float2* out = reinterpret_cast<float2*>(a.blocks + (size_t)b * BW * BH);
+#pragma unroll 8
+  for (int i = t; i < BW * BH / 2; i += TPB) {
+    const float2 v = S[(i / (BW / 2)) * TS + at(i % (BW / 2))], w = win[i];
+    out[i] = make_float2(v.x * w.x, v.y * w.y);
   }
 }
 
 // One block: temporal filter + sharpen per bin, Hermitian completion and
 // column inverse FFTs, row inverse FFTs, real part times the synthesis
-// window (src/cpu/reference.cpp:246-430, src/cpu/fft.cpp:88-119). KALMAN:
-// the Kalman filter (bm 0), whose state loads of KB bins are issued before
-// their updates are stored (the compiler cannot move a bin's loads above the
-// previous bin's state stores); the other modes read bm at run time.
+// window (src/cpu/reference.cpp:246-430, src/cpu/fft.cpp:88-119). G takes
+// F's place: every column is in registers before any is written.
 template <int BW, int BH, bool KALMAN>
-__global__ void __launch_bounds__(Cfg<BW, BH>::THREADS)
+__global__ void __launch_bounds__(Cfg<BW, BH>::THREADS, Cfg<BW, BH>::INV_CTAS - (KALMAN && Cfg<BW, BH>::TPB < 64))
     k_inverse_exact(const __grid_constant__ InvArgs a) {
   using C = Cfg<BW, BH>;
   extern __shared__ float4 smem4[];
@@ -121,83 +238,41 @@ __global__ void __launch_bounds__(Cfg<BW, BH>::THREADS)
   const int b = blockIdx.x * C::BPC + slot;
   const bool valid = b < a.g.nb;
   float2* F = reinterpret_cast<float2*>(smem + slot * C::INV_FLOATS);
-  float2* G = F + C::PS;
+  float2* G = F;
 
-  if (valid && KALMAN) {
-    const size_t base = (size_t)b * C::PS;
-    const float dc = block_dc(a, b);
-    for (int j0 = 0; j0 < C::NJ; j0 += C::KB) {
-      float2 sv[C::KB][4];
-      KState ks[C::KB];
-      BinTables tb[C::KB];
+  if (!KALMAN && valid && t == 0) prefetch_window<C::PS>(a, b);
+  if (valid) filter_block_any<KALMAN, BW == BH, C::PS, C::TPB, C::KB>(a, b, t, F);
+  block_sync<C::TPB>();
+  {
+    float2 v[BH];
+    if (t < C::FBW) {  // column t, kept or completed
 #pragma unroll
-      for (int u = 0; u < C::KB; u++) {
-        const int i = t + (j0 + u) * C::TPB;
-        if (j0 + u >= C::NJ || i >= C::PS) continue;
-        load_window<0>(a, base + i, sv[u]);
-        ks[u] = load_kstate(a, base + i);
-        tb[u] = bin_tables(a, i);
-      }
-#pragma unroll
-      for (int u = 0; u < C::KB; u++) {
-        const int i = t + (j0 + u) * C::TPB;
-        if (j0 + u >= C::NJ || i >= C::PS) continue;
-        F[i] = filter_vals_ks<0>(a, dc, tb[u], base + i, sv[u], ks[u]);
-      }
-    }
-  } else if (valid) {
-    const size_t base = (size_t)b * C::PS;
-    const float dc = block_dc(a, b);
-    const KState none{make_float2(0.0f, 0.0f), 0.0f, 0.0f};
-    constexpr int KN = 4;  // bins whose window spectra are loaded together
-    for (int j0 = 0; j0 < C::NJ; j0 += KN) {
-      float2 sv[KN][4];
-#pragma unroll
-      for (int u = 0; u < KN; u++) {
-        const int i = t + (j0 + u) * C::TPB;
-        if (j0 + u < C::NJ && i < C::PS) load_window<kRuntimeBm>(a, base + i, sv[u]);
-      }
-#pragma unroll
-      for (int u = 0; u < KN; u++) {
-        const int i = t + (j0 + u) * C::TPB;
-        if (j0 + u >= C::NJ || i >= C::PS) continue;
-        F[i] = filter_vals_ks<kRuntimeBm>(a, dc, bin_tables(a, i), base + i, sv[u], none);
-      }
-    }
-  }
-  __syncthreads();
-  if (valid) {
-    for (int c = t; c < BW; c += C::TPB) {
-      float2 v[BH];
+      for (int r = 0; r < BH; r++) v[r] = F[r * C::FBW + t];
+    } else if (t < BW) {
 #pragma unroll
       for (int r = 0; r < BH; r++) {
-        if (c < C::FBW) {
-          v[r] = F[r * C::FBW + c];
-        } else {
-          const float2 m = F[((BH - r) % BH) * C::FBW + (BW - c)];
-          v[r] = make_float2(m.x, -m.y);
-        }
+        const float2 m = F[((BH - r) % BH) * C::FBW + (BW - t)];
+        v[r] = make_float2(m.x, -m.y);
       }
+    }
+    block_sync<C::TPB>();
+    if (t < BW) {
       fft_r2<BH, true>(v, a.tw.col);
 #pragma unroll
-      for (int r = 0; r < BH; r++) G[r * C::TS + c] = v[r];
+      for (int r = 0; r < BH; r++) G[r * C::TS + t] = v[r];
     }
   }
-  __syncthreads();
-  if (valid) {
-    int bx, by, par;
-    block_origin(a.g, b, bx, by, par);
-    const float* win = par ? a.win_b : a.win_a;
-    float* out = a.blocks + (size_t)b * BW * BH;
-    for (int r = t; r < BH; r += C::TPB) {
-      float2 v[BW];
+  block_sync<C::TPB>();
+  if (t < BH) {
+    float2 v[BW];
 #pragma unroll
-      for (int c = 0; c < BW; c++) v[c] = G[r * C::TS + c];
-      fft_r2<BW, true>(v, a.tw.row);
+    for (int c = 0; c < BW; c++) v[c] = G[t * C::TS + c];
+    fft_r2<BW, true>(v, a.tw.row);
 #pragma unroll
-      for (int c = 0; c < BW; c++) out[r * BW + c] = v[c].x * win[r * BW + c];
-    }
+    for (int c = 0; c < BW / 2; c++) G[t * C::TS + c] = make_float2(v[2 * c].x, v[2 * c + 1].x);
   }
+  block_sync<C::TPB>();
+  if (valid) store_block<BW, BH, C::TPB, C::TS>(a, b, t, G, [](int j) { return j; });
 }
 
 // ---- 64 x 64 blocks: each 64-point transform on a lane pair ----------------
@@ -270,7 +345,7 @@ constexpr int kPairTS = 65;        // padded row stride (float or float2)
 // row p), then the 33 kept columns (pair p = column p). The input tile and
 // the row spectra share shared memory: every row is in registers before any
 // row spectrum is written.
-__global__ void __launch_bounds__(kPairThreads) k_forward_exact64(const __grid_constant__ FwdArgs a) {
+__global__ void __launch_bounds__(kPairThreads, 6) k_forward_exact64(const __grid_constant__ FwdArgs a) {
   constexpr int FBW = 33;
   extern __shared__ float4 smem4[];
   float* tile = reinterpret_cast<float*>(smem4);    // [64][kPairTS]
@@ -278,28 +353,7 @@ __global__ void __launch_bounds__(kPairThreads) k_forward_exact64(const __grid_c
   const int t = threadIdx.x, p = t >> 1;
   const bool odd = t & 1;
   const int b = blockIdx.x;
-  int bx, by, par;
-  block_origin(a.g, b, bx, by, par);
-  const bool inside = bx >= 0 && by >= 0 && bx + 64 <= a.g.W && by + 64 <= a.g.H;
-  constexpr int GB = 16;
-  for (int i0 = 0; i0 < 64 * 64; i0 += GB * kPairThreads) {
-    float v[GB], w[GB];
-#pragma unroll
-    for (int u = 0; u < GB; u++) {
-      const int idx = i0 + t + u * kPairThreads;
-      const int ly = idx >> 6, lx = idx & 63;
-      const int y = inside ? by + ly : mirror_i(by + ly, a.g.H);
-      const int x = inside ? bx + lx : mirror_i(bx + lx, a.g.W);
-      v[u] = load_sample(a.src + (long long)y * a.pitch, x, a.fmt, a.norm);
-      w[u] = a.win[idx];
-    }
-#pragma unroll
-    for (int u = 0; u < GB; u++) {
-      const int idx = i0 + t + u * kPairThreads;
-      const float c = v[u] - a.chroma_norm;
-      tile[(idx >> 6) * kPairTS + (idx & 63)] = c * w[u];
-    }
-  }
+  gather_block<64, 64, kPairThreads, 16, kPairTS>(a, b, t, tile);
   __syncthreads();
   float2 r[32];
 #pragma unroll
@@ -329,9 +383,9 @@ __global__ void __launch_bounds__(kPairThreads) k_forward_exact64(const __grid_c
 // Filter + inverse of one 64 x 64 block per CTA: the filtered half spectrum
 // F, column transforms (pair p = column p, Hermitian completion on the fly)
 // into G, which shares F's space once every column is in registers, then
-// row transforms (pair p = row p) times the synthesis window.
+// row transforms (pair p = row p) and the windowed rows in plane order.
 template <bool KALMAN>
-__global__ void __launch_bounds__(kPairThreads) k_inverse_exact64(const __grid_constant__ InvArgs a) {
+__global__ void __launch_bounds__(kPairThreads, 5) k_inverse_exact64(const __grid_constant__ InvArgs a) {
   constexpr int FBW = 33, PS = 64 * FBW;
   extern __shared__ float4 smem4[];
   float2* F = reinterpret_cast<float2*>(smem4);  // [64][FBW]
@@ -339,33 +393,12 @@ __global__ void __launch_bounds__(kPairThreads) k_inverse_exact64(const __grid_c
   const int t = threadIdx.x, p = t >> 1;
   const bool odd = t & 1;
   const int b = blockIdx.x;
-  const size_t base = (size_t)b * PS;
-  if (KALMAN) {
-    const float dc = block_dc(a, b);
-    constexpr int NJ = (PS + kPairThreads - 1) / kPairThreads, KB = 8;
-    for (int j0 = 0; j0 < NJ; j0 += KB) {
-      float2 sv[KB][4];
-      KState ks[KB];
-      BinTables tb[KB];
-#pragma unroll
-      for (int u = 0; u < KB; u++) {
-        const int i = t + (j0 + u) * kPairThreads;
-        if (j0 + u >= NJ || i >= PS) continue;
-        load_window<0>(a, base + i, sv[u]);
-        ks[u] = load_kstate(a, base + i);
-        tb[u] = bin_tables(a, i);
-      }
-#pragma unroll
-      for (int u = 0; u < KB; u++) {
-        const int i = t + (j0 + u) * kPairThreads;
-        if (j0 + u >= NJ || i >= PS) continue;
-        F[i] = filter_vals_ks<0>(a, dc, tb[u], base + i, sv[u], ks[u]);
-      }
-    }
-  } else {
-    for (int i = t; i < PS; i += kPairThreads) F[i] = filter_bin(a, b, i, base + i);
-  }
+  if (!KALMAN && t == 0) prefetch_window<PS>(a, b);
+  filter_block_any<KALMAN, true, PS, kPairThreads, 6>(a, b, t, F);
   __syncthreads();
+  // A row's odd lane puts its 16 sample pairs 24 entries along: in other
+  // banks than its even lane's.
+  constexpr int kOddAt = 24;
   float2 r[32];
   {
     const int c = p;
@@ -388,12 +421,11 @@ __global__ void __launch_bounds__(kPairThreads) k_inverse_exact64(const __grid_c
 #pragma unroll
   for (int q = 0; q < 32; q++) r[q] = G[p * kPairTS + bit_reverse(q, 6) + odd];
   fft64_pair<true>(r, a.tw.row, odd);
-  int bx, by, par;
-  block_origin(a.g, b, bx, by, par);
-  const float* win = (par ? a.win_b : a.win_a) + p * 64 + 32 * odd;
-  float* out = a.blocks + (size_t)b * 64 * 64 + p * 64 + 32 * odd;
+  __syncwarp();  // the pair has read its row
 #pragma unroll
-  for (int q = 0; q < 32; q++) out[q] = r[q].x * win[q];
+  for (int q = 0; q < 16; q++) G[p * kPairTS + kOddAt * odd + q] = make_float2(r[2 * q].x, r[2 * q + 1].x);
+  __syncthreads();
+  store_block<64, 64, kPairThreads, kPairTS>(a, b, t, G, [](int j) { return j < 16 ? j : j + (kOddAt - 16); });
 }
 
 cudaError_t launch_fwd64(const FwdArgs& a, cudaStream_t st) {
