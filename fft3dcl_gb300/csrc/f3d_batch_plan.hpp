@@ -78,6 +78,39 @@ inline bool sweep_batches(const SweepArgs* planes, int n, SweepBatch& Bf, SweepB
   return true;
 }
 
+// Segments of each plane's strips (written to its segs, at most what it comes
+// with) for one launch of all planes' sweeps, `slots` CTAs of which run at a
+// time. A CTA costs its block rows plus about one and a half for its set-up
+// and its seams, and a last wave costs as much as a full one: the rows per
+// segment with the smallest waves x (rows + 1.5), the largest such. Each
+// plane's own plan fills one wave by itself: a 1080p 4:2:0 frame then had 756
+// CTAs of 2 to 3 rows for 456 slots and 56 seams, here 378 CTAs of 5 rows and
+// 25 seams (its step, with the seams finished in the sweep: 123.5 -> 120.7
+// us; ten 4K outputs 1750 -> 1738 us).
+inline void plan_segments(SweepArgs* planes, int n, int slots) {
+  if (slots < 1) return;
+  int most = 1;
+  for (int i = 0; i < n; i++) most = planes[i].cells_y + 1 > most ? planes[i].cells_y + 1 : most;
+  auto segs_of = [&](const SweepArgs& a, int rows) {
+    const int s = (a.cells_y + 1 + rows - 1) / rows;
+    return s < a.segs ? s : a.segs;
+  };
+  int best = 0;
+  long long best_cost = 0;
+  for (int rows = 1; rows <= most; rows++) {
+    long long ctas = 0;
+    int longest = 0;
+    for (int i = 0; i < n; i++) {
+      const int s = segs_of(planes[i], rows), r = (planes[i].cells_y + 1 + s - 1) / s;
+      ctas += (long long)planes[i].strips * s;
+      longest = r > longest ? r : longest;
+    }
+    const long long cost = (ctas + slots - 1) / slots * (2 * longest + 3);
+    if (best == 0 || cost <= best_cost) best = rows, best_cost = cost;
+  }
+  for (int i = 0; i < n; i++) planes[i].segs = segs_of(planes[i], best);
+}
+
 // Autotuner choice among n timed launch shapes (fastest[i]: the fastest of
 // shape i's runs; shape 0 is the default): the fastest shape, unless the
 // default is within `margin` of it (single-step timings vary by about 1 %).

@@ -88,6 +88,29 @@ __device__ __forceinline__ void store_sample(uint8_t* row, int x, float v, int f
   }
 }
 
+// Samples x..x+3 of a plane row (those left of W), with one store where they
+// are whole and aligned.
+__device__ __forceinline__ void store_quad(uint8_t* row, int x, int W, const float (&v)[4], int fmt, float inv_norm,
+                                           float max_pix) {
+  const bool full = x + 4 <= W;
+  const uintptr_t r = reinterpret_cast<uintptr_t>(row);
+  if (full && fmt == FMT_U8 && ((r + x) & 3) == 0) {
+    *reinterpret_cast<uint32_t*>(row + x) =
+        pack_u8(v[0]) | (pack_u8(v[1]) << 8) | (pack_u8(v[2]) << 16) | (pack_u8(v[3]) << 24);
+  } else if (full && fmt == FMT_U16 && ((r + 2 * x) & 7) == 0) {
+    uint32_t p[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) p[k] = pack_u16(v[k], inv_norm, max_pix);
+    *reinterpret_cast<uint2*>(row + 2 * x) = make_uint2(p[0] | (p[1] << 16), p[2] | (p[3] << 16));
+  } else if (full && fmt == FMT_F32 && ((r + 4 * x) & 15) == 0) {
+    *reinterpret_cast<float4*>(row + 4 * x) = make_float4(v[0], v[1], v[2], v[3]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (x + k < W) store_sample(row, x + k, v[k], fmt, inv_norm, max_pix);
+  }
+}
+
 // Wiener shrink of one complex value, src/cpu/reference.cpp:201-209.
 __device__ __forceinline__ void wienner(float& re, float& im, float sx, float sy, float beta_x) {
   float psd = re * re + im * im + 0.0000000000000000000000000000000000001f;
@@ -403,6 +426,54 @@ __device__ __forceinline__ float2 filter_bin_t(const InvArgs& a, float dc, int i
 
 __device__ __forceinline__ float2 filter_bin(const InvArgs& a, int b, int i, size_t gi) {
   return filter_bin_t<kRuntimeBm>(a, block_dc(a, b), i, gi);
+}
+
+// End of a sweep CTA (strip, segment seg): of the two CTAs that share a seam
+// (the last cell row of a segment), the one that ends last finishes the
+// strip's seam cells, ((q1 + q2) + q3) + q4 per sample
+// (src/cpu/reference.cpp:415-430), packed. Nothing waits, and no merge launch
+// follows: at ten 1080p outputs the merge kernel took 43 us beside a sweep of
+// 138 us. Every CTA of the launch calls this once, also one that gave up, so
+// that the counters return to 0. Called by all threads; flags: two ints of
+// shared memory. J0: the strip's first cell, ncell its cells.
+template <int CH, int CW>
+__device__ __forceinline__ void finish_seams(const SweepArgs& sa, int strip, int seg, int J0, int ncell, int* flags) {
+  if (sa.segs < 2) return;
+  __threadfence();  // this CTA's seam rows, before its count
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    const int k = seg - 1 + (int)threadIdx.x;  // the seam above, the seam below
+    int last = 0;
+    if (k >= 0 && k < sa.segs - 1) {
+      int* c = sa.seam_cnt + (size_t)k * sa.strips + strip;
+      last = atomicAdd(c, 1) == 1;
+      if (last) atomicExch(c, 0);
+    }
+    flags[threadIdx.x] = last;
+    __threadfence();
+  }
+  __syncthreads();
+  const int nrow = sa.cells_y + 1;
+#pragma unroll 1
+  for (int w = 0; w < 2; w++) {
+    if (!flags[w]) continue;
+    const int k = seg - 1 + w;
+    const int y0 = ((int)((long long)(k + 1) * nrow / sa.segs) - 1) * CH;
+    const int quads = ncell * (CW / 4);
+    for (int i = threadIdx.x; i < CH * quads; i += blockDim.x) {
+      const int yy = i / quads, x = J0 * CW + 4 * (i - yy * quads);
+      if (y0 + yy >= sa.inv.g.H || x >= sa.inv.g.W) continue;
+      const size_t row = sa.seam_w;
+      const float4 b = __ldcg(reinterpret_cast<const float4*>(sa.seam_b + ((size_t)k * CH + yy) * row + x));
+      const float4 t0 = __ldcg(reinterpret_cast<const float4*>(sa.seam_t + ((size_t)(2 * k) * CH + yy) * row + x));
+      const float4 t1 = __ldcg(reinterpret_cast<const float4*>(sa.seam_t + ((size_t)(2 * k + 1) * CH + yy) * row + x));
+      float v[4] = {(b.x + t0.x) + t1.x, (b.y + t0.y) + t1.y, (b.z + t0.z) + t1.z, (b.w + t0.w) + t1.w};
+      if (sa.chroma_norm != 0.0f)
+#pragma unroll
+        for (int q = 0; q < 4; q++) v[q] += sa.chroma_norm;
+      store_quad(sa.dst + (long long)(y0 + yy) * sa.pitch, x, sa.inv.g.W, v, sa.fmt, sa.inv_norm, sa.max_pix);
+    }
+  }
 }
 
 // One radix-2 DIT stage of length LEN over N register values: butterflies

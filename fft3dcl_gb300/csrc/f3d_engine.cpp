@@ -314,8 +314,7 @@ SweepArgs sweep_args(const f3d_engine* e, const InvArgs& a, uint8_t* ddst, long 
   sa.strips = e->sweep_strips;
   sa.segs = e->sweep_segs;
   sa.seam_w = sa.cells_x * (a.g.bw / 2);
-  sa.seam_b = e->d_seam;
-  sa.seam_t = e->d_seam ? e->d_seam + (size_t)(sa.segs - 1) * (a.g.bh / 2) * sa.seam_w : nullptr;
+  set_seams(sa, e->d_seam, e->sweep_segs);
   sa.prefetch = e->sweep_prefetch;
   sa.tab = e->d_tc;
   sa.err = e->d_err;
@@ -329,7 +328,7 @@ int run_process(f3d_engine* e, const int* window, int n, uint8_t* ddst, long lon
   int rc = inverse_args(e, window, n, a);
   if (rc != F3D_OK) return rc;
   if (e->fused) {
-    // One fused launch (plus the seam merge) writes the packed plane.
+    // The fused launch (tensor-core form: filter, then inverse) writes the packed plane.
     const SweepArgs sa = sweep_args(e, a, ddst, pitch, fmt);
     e->test_skip = false;
     cudaEventRecord(e->ev[2], e->stream);
@@ -542,8 +541,9 @@ int f3d_engine_create(const f3d_script_params* sp, const f3d_plane_geom* geom,
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     sweep_plan(e->inv_form, geo, sms > 0 ? sms : 1, &e->sweep_strips, &e->sweep_segs);
-    e->seam_floats = sweep_seam_floats(geo, e->sweep_segs);
-    if (e->seam_floats && (ce = e->alloc(&e->d_seam, sizeof(float) * e->seam_floats)) != cudaSuccess)
+    e->seam_floats = sweep_seam_floats(geo, e->sweep_strips, e->sweep_segs);
+    if (e->seam_floats && ((ce = e->alloc(&e->d_seam, sizeof(float) * e->seam_floats)) != cudaSuccess ||
+                           (ce = cudaMemsetAsync(e->d_seam, 0, sizeof(float) * e->seam_floats, e->stream)) != cudaSuccess))
       return finish_fail(e->cuda_fail(ce, "seam buffer allocation"));
     if (e->inv_form == F3D_FORM_TC) {
       e->img_bytes = tc_image_bytes(geo, e->sweep_strips);
@@ -914,7 +914,8 @@ int f3d_batch_create(f3d_engine* const* engines, int n, int flags, f3d_batch** o
     b->img_bytes[i] = b->fast ? 0 : e->img_bytes;  // the fast sweep has no operand tiles
     b->seam_bytes[i] = sizeof(float) * e->seam_floats;
     if ((b->img_bytes[i] && cudaMalloc(&b->img[i], b->img_bytes[i]) != cudaSuccess) ||
-        (b->seam_bytes[i] && cudaMalloc(&b->seam[i], b->seam_bytes[i]) != cudaSuccess)) {
+        (b->seam_bytes[i] && (cudaMalloc(&b->seam[i], b->seam_bytes[i]) != cudaSuccess ||
+                              cudaMemsetAsync(b->seam[i], 0, b->seam_bytes[i], b->stream) != cudaSuccess))) {
       cudaGetLastError();
       f3d_batch_destroy(b);
       return fail_thread(F3D_E_NOMEM, "FFT3DCL: batch output buffers could not be allocated");
@@ -1008,8 +1009,7 @@ int f3d_batch_step(f3d_batch* b, const int* fns, const void* const* dev_src, con
     e->test_skip = false;
     if (b->repeat[i]) {  // a repeated engine: this output's own tiles and seam rows
       sa[ns].img = b->img[i];
-      sa[ns].seam_b = b->seam[i];
-      sa[ns].seam_t = b->seam[i] ? b->seam[i] + (size_t)(sa[ns].segs - 1) * (a.g.bh / 2) * sa[ns].seam_w : nullptr;
+      set_seams(sa[ns], b->seam[i], e->sweep_segs);
     }
     ns++;
     mask |= 1ull << (16 + i);
@@ -1028,7 +1028,7 @@ int f3d_batch_step(f3d_batch* b, const int* fns, const void* const* dev_src, con
           for (int k = 0; k < nwin[j]; k++)
             if (windows[j][k] == fns[i]) overlap = false;
   if (overlap) mask |= 1ull << 32;
-  // Filter, inverse and seam merge; timed by events unless being captured.
+  // Filter and inverse; timed by events unless being captured.
   auto sweep = [&](const TcTune& t, cudaEvent_t after_filter) -> cudaError_t {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(b->stream, &cs);

@@ -10,34 +10,18 @@ static std::atomic<unsigned long long> g_launch_count{0};
 void count_launch() { g_launch_count.fetch_add(1, std::memory_order_relaxed); }
 unsigned long long launch_count() { return g_launch_count.load(std::memory_order_relaxed); }
 
+int sm_count() {
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n > 0 ? n : 1;
+}
+
 namespace {
 
 __device__ __forceinline__ int floor_div(int a, int b) {
   int q = a / b;
   return (a % b != 0 && ((a < 0) != (b < 0))) ? q - 1 : q;
-}
-
-// Four finished samples of row y from x on (those inside the plane), with one
-// store where they are whole and aligned.
-__device__ __forceinline__ void store_quad(const OlaArgs& a, int x, int y, const float (&v)[4]) {
-  uint8_t* row = a.dst + (long long)y * a.pitch;
-  const bool full = x + 4 <= a.g.W;
-  const uintptr_t r = reinterpret_cast<uintptr_t>(row);
-  if (full && a.fmt == FMT_U8 && ((r + x) & 3) == 0) {
-    *reinterpret_cast<uint32_t*>(row + x) =
-        pack_u8(v[0]) | (pack_u8(v[1]) << 8) | (pack_u8(v[2]) << 16) | (pack_u8(v[3]) << 24);
-  } else if (full && a.fmt == FMT_U16 && ((r + 2 * x) & 7) == 0) {
-    uint32_t p[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) p[k] = pack_u16(v[k], a.inv_norm, a.max_pix);
-    *reinterpret_cast<uint2*>(row + 2 * x) = make_uint2(p[0] | (p[1] << 16), p[2] | (p[3] << 16));
-  } else if (full && a.fmt == FMT_F32 && ((r + 4 * x) & 15) == 0) {
-    *reinterpret_cast<float4*>(row + 4 * x) = make_float4(v[0], v[1], v[2], v[3]);
-  } else {
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-      if (x + k < a.g.W) store_sample(row, x + k, v[k], a.fmt, a.inv_norm, a.max_pix);
-  }
 }
 
 // The mode-1 blocks covering a sample along one axis: first block and how
@@ -112,7 +96,7 @@ __global__ void __launch_bounds__(256) k_ola(const __grid_constant__ OlaArgs a) 
   if (a.chroma_norm != 0.0f)
 #pragma unroll
     for (int k = 0; k < V; k++) sum[k] += a.chroma_norm;
-  if constexpr (V == 4) store_quad(a, x, y, sum);
+  if constexpr (V == 4) store_quad(a.dst + (long long)y * a.pitch, x, g.W, sum, a.fmt, a.inv_norm, a.max_pix);
   else store_sample(a.dst + (long long)y * a.pitch, x, sum[0], a.fmt, a.inv_norm, a.max_pix);
 }
 

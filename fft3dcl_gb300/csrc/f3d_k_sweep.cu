@@ -21,7 +21,7 @@
 //   - starts cell row m: P = bottom halves of row m.
 // The first cell row of a segment (row M0-1) and its last (M1-1) are shared
 // with the neighbouring segments: their quadrants go to seam buffers and
-// k_seam_merge finishes them in the same order. The next row's window
+// the later of the two CTAs finishes them in the same order. The next row's window
 // spectra can be bulk-prefetched into L2 while row m is processed (off by
 // default: with one wave of CTAs each holding a row, the prefetched rows
 // exceed what L2 keeps and the extra traffic costs more than it hides).
@@ -70,15 +70,11 @@ __device__ __forceinline__ float4 add4(float4 a, float4 b) {
 // Four output samples at x..x+3 of row y (bounds-checked against the plane).
 __device__ __forceinline__ void store4(const SweepArgs& sa, int y, int x, float4 v) {
   if (y >= sa.inv.g.H) return;
-  uint8_t* row = sa.dst + (long long)y * sa.pitch;
-  const float e[4] = {v.x, v.y, v.z, v.w};
+  float e[4] = {v.x, v.y, v.z, v.w};
+  if (sa.chroma_norm != 0.0f)
 #pragma unroll
-  for (int k = 0; k < 4; k++) {
-    if (x + k >= sa.inv.g.W) break;
-    float s = e[k];
-    if (sa.chroma_norm != 0.0f) s += sa.chroma_norm;
-    store_sample(row, x + k, s, sa.fmt, sa.inv_norm, sa.max_pix);
-  }
+    for (int k = 0; k < 4; k++) e[k] += sa.chroma_norm;
+  store_quad(sa.dst + (long long)y * sa.pitch, x, sa.inv.g.W, e, sa.fmt, sa.inv_norm, sa.max_pix);
 }
 
 // CTA `cta` (strip, segment) of plane sa's sweep.
@@ -156,6 +152,8 @@ __device__ __forceinline__ void sweep_fast_cta(const SweepArgs& sa, int cta) {
     }
     __syncthreads();
   }
+  // The tiles are free: two ints of them for the seams.
+  finish_seams<CH, CW>(sa, strip, seg, J0, ncell, reinterpret_cast<int*>(slots));
 }
 
 template <int BW, int BH, int BM>
@@ -176,23 +174,6 @@ __global__ void __launch_bounds__(kSweepThreads, F3D_SWEEP_MINB)
   sweep_fast_cta<BW, BH, BM>(B.p[r0 + local % rl], local / rl);
 }
 
-// Finishes the seam cell rows: ((q1 + q2) + q3) + q4 per sample, packed.
-__global__ void __launch_bounds__(256) k_seam_merge(const __grid_constant__ SweepArgs sa, int ch) {
-  const int x = blockIdx.x * 256 + threadIdx.x;
-  const int yy = blockIdx.y, k = blockIdx.z;  // seam k: cell row M1(k) - 1
-  if (x >= sa.inv.g.W) return;
-  const int nrow = sa.cells_y + 1;
-  const int m1 = (int)((long long)(k + 1) * nrow / sa.segs);
-  const int y = (m1 - 1) * ch + yy;
-  if (y >= sa.inv.g.H) return;
-  const size_t o = ((size_t)k * ch + yy) * sa.seam_w + x;
-  const size_t ot = ((size_t)(k * 2) * ch + yy) * sa.seam_w + x;
-  float v = sa.seam_b[o] + sa.seam_t[ot];
-  v = v + sa.seam_t[ot + (size_t)ch * sa.seam_w];
-  if (sa.chroma_norm != 0.0f) v += sa.chroma_norm;
-  store_sample(sa.dst + (long long)y * sa.pitch, x, v, sa.fmt, sa.inv_norm, sa.max_pix);
-}
-
 template <int BW, int BH, int BM>
 cudaError_t launch_bm(const SweepArgs& a, cudaStream_t st, cudaEvent_t mark) {
   using S_ = SCfg<BW, BH>;
@@ -205,7 +186,7 @@ cudaError_t launch_bm(const SweepArgs& a, cudaStream_t st, cudaEvent_t mark) {
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (mark) cudaEventRecord(mark, st);
-  return launch_seam_merge(a, st);
+  return cudaSuccess;
 }
 
 template <int BW, int BH, int BM>
@@ -247,11 +228,12 @@ cudaError_t launch_size(const SweepArgs& a, cudaStream_t st, cudaEvent_t mark) {
 }  // namespace
 
 cudaError_t launch_sweep_fast_batch(const SweepArgs* planes, int n, cudaStream_t st, cudaEvent_t mark) {
+  if (n < 1 || n > kMaxBatch) return cudaErrorInvalidValue;
+  SweepArgs p[kMaxBatch];
+  std::copy(planes, planes + n, p);
+  plan_segments(p, n, F3D_SWEEP_MINB * sm_count());
   SweepBatch Bf, Bs, Bm;
-  if (!sweep_batches(planes, n, Bf, Bs, Bm, false))
-    return n < 1 || n > kMaxBatch ? cudaErrorInvalidValue : cudaErrorNotSupported;
-  int maxw = 0;
-  for (int i = 0; i < n; i++) maxw = std::max(maxw, planes[i].inv.g.W);
+  if (!sweep_batches(p, n, Bf, Bs, Bm, false)) return cudaErrorNotSupported;
   cudaError_t e;
   switch (planes[0].inv.g.bw) {
   case 8: e = launch_batch_size<8, 8>(Bs, n, st); break;
@@ -261,15 +243,7 @@ cudaError_t launch_sweep_fast_batch(const SweepArgs* planes, int n, cudaStream_t
   }
   if (e != cudaSuccess) return e;
   if (mark) cudaEventRecord(mark, st);
-  return launch_seam_merge_batch(Bm, n, maxw, planes[0].inv.g.bh / 2, st);
-}
-
-cudaError_t launch_seam_merge(const SweepArgs& a, cudaStream_t st) {
-  if (a.segs < 2) return cudaSuccess;
-  dim3 grid((a.inv.g.W + 255) / 256, a.inv.g.bh / 2, a.segs - 1);
-  k_seam_merge<<<grid, 256, 0, st>>>(a, a.inv.g.bh / 2);
-  count_launch();
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 bool sweep_supported(int form, const Geo& g, int bm) {
@@ -282,7 +256,7 @@ bool sweep_supported(int form, const Geo& g, int bm) {
   return g.xoff == -g.bw / 2 && g.xstep == g.bw / 2 && g.yoff == -g.bh / 2 && g.ystep == g.bh / 2;
 }
 
-void sweep_plan(int form, const Geo& g, int sm_count, int* strips, int* segs) {
+void sweep_plan(int form, const Geo& g, int sms, int* strips, int* segs) {
   const int tj = form == F3D_FORM_TC ? tc_sweep_cells(g.bw) : kSweepThreads / g.bw - 1;
   const int per_sm = form == F3D_FORM_TC ? kTcSweepCtasPerSm : F3D_SWEEP_MINB;
   const int cells_x = (g.W + g.bw / 2 - 1) / (g.bw / 2);
@@ -290,15 +264,15 @@ void sweep_plan(int form, const Geo& g, int sm_count, int* strips, int* segs) {
   *strips = (cells_x + tj - 1) / tj;
   // At most one wave of resident CTAs (a partial second wave would double the
   // time), segments of at least two block rows.
-  int s = per_sm * sm_count / *strips;
+  int s = per_sm * sms / *strips;
   const int maxseg = (cells_y + 1) / 2;
   if (s > maxseg) s = maxseg;
   *segs = s < 1 ? 1 : s;
 }
 
-size_t sweep_seam_floats(const Geo& g, int segs) {
+size_t sweep_seam_floats(const Geo& g, int strips, int segs) {
   const int cells_x = (g.W + g.bw / 2 - 1) / (g.bw / 2);
-  return (size_t)(segs > 1 ? segs - 1 : 0) * 3 * (g.bh / 2) * (size_t)cells_x * (g.bw / 2);
+  return (size_t)(segs > 1 ? segs - 1 : 0) * (3 * (g.bh / 2) * (size_t)cells_x * (g.bw / 2) + strips);
 }
 
 cudaError_t launch_sweep(int form, const SweepArgs& a, cudaStream_t st, cudaEvent_t mark) {

@@ -1029,18 +1029,13 @@ __global__ void __launch_bounds__(kTcThreads, kTcSweepCtasPerSm) k_sweep_tc(cons
   __syncthreads();
   tc::fence_after_sync();
   if (warp == 0) tc::tmem_dealloc(st.tmem, C::TMEM_COLS);
+  // The partial sums are done with: two ints of them for the seams.
+  finish_seams<S::CH, S::CW>(sa, strip, seg, J0, ncell, reinterpret_cast<int*>(sm + S::P));
 }
 
 template <class K>
 cudaError_t prepare(K k, size_t smem) {
   return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-}
-
-int sm_count() {
-  int dev = 0, n = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  return n > 0 ? n : 1;
 }
 
 // Host-side fp16 hi/lo split of a double.
@@ -1221,33 +1216,11 @@ cudaError_t launch_filter(const SweepBatch& B, int bm, cudaStream_t st) {
   return B.p[0].inv.half ? launch_filter_h<N, MINB, true>(B, bm, st) : launch_filter_h<N, MINB, false>(B, bm, st);
 }
 
-// Finishes the seam cell rows of every plane of the batch: blockIdx.z runs
-// over all planes' seams (prefix in cta0), the sum as in k_seam_merge
-// (f3d_k_sweep.cu): ((q1 + q2) + q3) + q4, packed.
-__global__ void __launch_bounds__(256) k_seam_merge_batch(const __grid_constant__ SweepBatch B, int ch) {
-  const int pl = plane_of(B, B.cta0, blockIdx.z);
-  const SweepArgs& sa = B.p[pl];
-  const int k = blockIdx.z - B.cta0[pl];
-  const int x = blockIdx.x * 256 + threadIdx.x;
-  const int yy = blockIdx.y;
-  if (x >= sa.inv.g.W) return;
-  const int nrow = sa.cells_y + 1;
-  const int m1 = (int)((long long)(k + 1) * nrow / sa.segs);
-  const int y = (m1 - 1) * ch + yy;
-  if (y >= sa.inv.g.H) return;
-  const size_t o = ((size_t)k * ch + yy) * sa.seam_w + x;
-  const size_t ot = ((size_t)(k * 2) * ch + yy) * sa.seam_w + x;
-  float v = sa.seam_b[o] + sa.seam_t[ot];
-  v = v + sa.seam_t[ot + (size_t)ch * sa.seam_w];
-  if (sa.chroma_norm != 0.0f) v += sa.chroma_norm;
-  store_sample(sa.dst + (long long)y * sa.pitch, x, v, sa.fmt, sa.inv_norm, sa.max_pix);
-}
-
 namespace {
 
 template <int N>
-cudaError_t launch_sweep_n(const SweepBatch& Bf, const SweepBatch& B, const SweepBatch& Bm, int n, int maxw,
-                           const TcTune& t, cudaStream_t st, cudaEvent_t mark, cudaEvent_t after_filter) {
+cudaError_t launch_sweep_n(const SweepBatch& Bf, const SweepBatch& B, int n, const TcTune& t, cudaStream_t st,
+                           cudaEvent_t mark, cudaEvent_t after_filter) {
   using S = SwpCfg<N>;
   const int bm = B.p[0].inv.bm;
   constexpr size_t smem = S::BYTES;
@@ -1264,35 +1237,30 @@ cudaError_t launch_sweep_n(const SweepBatch& Bf, const SweepBatch& B, const Swee
   if (e != cudaSuccess) return e;
   k_sweep_tc<N><<<B.cta0[n], kTcThreads, smem, st>>>(B);
   count_launch();
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  // Seam rows of all planes.
-  if (Bm.cta0[n] == 0) return cudaSuccess;
-  dim3 grid((maxw + 255) / 256, S::CH, Bm.cta0[n]);
-  k_seam_merge_batch<<<grid, 256, 0, st>>>(Bm, S::CH);
-  count_launch();
   return cudaGetLastError();
+}
+
+// The filter's and the inverse kernel's batch parameters, with the segments
+// planned for one launch of all planes.
+cudaError_t tc_sweep_batches(const SweepArgs* planes, int n, SweepBatch& Bf, SweepBatch& B) {
+  if (n < 1 || n > kMaxBatch) return cudaErrorInvalidValue;
+  SweepArgs p[kMaxBatch];
+  std::copy(planes, planes + n, p);
+  plan_segments(p, n, kTcSweepCtasPerSm * sm_count());
+  SweepBatch Bm;
+  return sweep_batches(p, n, Bf, B, Bm) ? cudaSuccess : cudaErrorNotSupported;
 }
 
 }  // namespace
 
-cudaError_t launch_seam_merge_batch(const SweepBatch& Bm, int n, int maxw, int ch, cudaStream_t st) {
-  if (Bm.cta0[n] == 0) return cudaSuccess;
-  dim3 grid((maxw + 255) / 256, ch, Bm.cta0[n]);
-  k_seam_merge_batch<<<grid, 256, 0, st>>>(Bm, ch);
-  count_launch();
-  return cudaGetLastError();
-}
-
 cudaError_t launch_sweep_tc_batch(const SweepArgs* planes, int n, const TcTune& t, cudaStream_t st,
                                   cudaEvent_t mark, cudaEvent_t after_filter) {
-  SweepBatch Bf, B, Bm;
-  if (!sweep_batches(planes, n, Bf, B, Bm)) return n < 1 || n > kMaxBatch ? cudaErrorInvalidValue : cudaErrorNotSupported;
-  int maxw = 0;
-  for (int i = 0; i < n; i++) maxw = std::max(maxw, planes[i].inv.g.W);
+  SweepBatch Bf, B;
+  cudaError_t e = tc_sweep_batches(planes, n, Bf, B);
+  if (e != cudaSuccess) return e;
   static_assert(SwpCfg<32>::TJ == 7 && SwpCfg<16>::TJ == 15, "cells per strip");
-  return planes[0].inv.g.bw == 16 ? launch_sweep_n<16>(Bf, B, Bm, n, maxw, t, st, mark, after_filter)
-                                  : launch_sweep_n<32>(Bf, B, Bm, n, maxw, t, st, mark, after_filter);
+  return planes[0].inv.g.bw == 16 ? launch_sweep_n<16>(Bf, B, n, t, st, mark, after_filter)
+                                  : launch_sweep_n<32>(Bf, B, n, t, st, mark, after_filter);
 }
 
 cudaError_t launch_sweep_tc(const SweepArgs& a, cudaStream_t st, cudaEvent_t mark) {
@@ -1321,22 +1289,22 @@ bool is_forward(const void* f) {
 cudaError_t tc_graph_update(cudaGraphExec_t exec, cudaGraph_t graph, const TcFwdArgs* fwd, int nf,
                             const SweepArgs* sw, int ns) {
   TcFwdBatch Bw{};
-  SweepBatch Bf, Bs, Bm;
+  SweepBatch Bf, Bs;
+  cudaError_t e = cudaSuccess;
   if (nf > 0 && !forward_batch(fwd, nf, Bw)) return cudaErrorNotSupported;
-  if (ns > 0 && !sweep_batches(sw, ns, Bf, Bs, Bm)) return cudaErrorNotSupported;
+  if (ns > 0 && (e = tc_sweep_batches(sw, ns, Bf, Bs)) != cudaSuccess) return e;
   size_t cnt = 0;
-  cudaError_t e = cudaGraphGetNodes(graph, nullptr, &cnt);
+  e = cudaGraphGetNodes(graph, nullptr, &cnt);
   if (e != cudaSuccess) return e;
   std::vector<cudaGraphNode_t> nodes(cnt);
   if ((e = cudaGraphGetNodes(graph, nodes.data(), &cnt)) != cudaSuccess) return e;
-  int ch = (ns > 0 ? sw[0].inv.g.bh : 32) / 2;
   for (cudaGraphNode_t node : nodes) {
     cudaGraphNodeType ty;
     if ((e = cudaGraphNodeGetType(node, &ty)) != cudaSuccess) return e;
     if (ty != cudaGraphNodeTypeKernel) continue;
     cudaKernelNodeParams kp{};
     if ((e = cudaGraphKernelNodeGetParams(node, &kp)) != cudaSuccess) return e;
-    void* args[2] = {nullptr, &ch};
+    void* args[1] = {nullptr};
     const void* f = kp.func;
     if (is_forward<32>(f) || is_forward<16>(f))
       args[0] = &Bw;
@@ -1344,8 +1312,6 @@ cudaError_t tc_graph_update(cudaGraphExec_t exec, cudaGraph_t graph, const TcFwd
       args[0] = &Bf;
     else if (f == (const void*)k_sweep_tc<32> || f == (const void*)k_sweep_tc<16>)
       args[0] = &Bs;
-    else if (f == (const void*)k_seam_merge_batch)
-      args[0] = &Bm;
     else
       return cudaErrorInvalidValue;
     kp.kernelParams = args;

@@ -85,7 +85,7 @@ struct OlaArgs {
 // block rows, adding each row's windowed blocks to the cells in shared
 // memory in the reference's block order, and writes finished cells straight
 // to the output plane. Cell rows on the boundary between two segments are
-// finished by a merge pass from the seam buffers.
+// finished from the seam buffers by whichever of the two CTAs ends last.
 struct SweepArgs {
   InvArgs inv;
   uint8_t* dst;          // output plane
@@ -98,6 +98,7 @@ struct SweepArgs {
   int prefetch;          // L2 prefetch of the next block row: 0 off, 1 at row start, 2 after the filter
   float* seam_b;         // [segs-1][bh/2][seam_w]: first two quadrants of each seam cell, summed
   float* seam_t;         // [segs-1][2][bh/2][seam_w]: third and fourth quadrants
+  int* seam_cnt;         // [segs-1][strips]: CTAs of the seam that are done, 0 between launches
   const uint8_t* tab;    // tensor-core form: device copy of tc_tables()
   int* err;              // tensor-core form: bits set when a wait gives up (kErrWait*)
   uint8_t* img;          // tensor-core form: filtered column-inverse operands, one tile per (row, strip)
@@ -112,11 +113,19 @@ enum : int {
   kErrWaitRow = 8       // inverse: the row-inverse products
 };
 
-// Whether the sweep handles this geometry and form; its CTA grid; the seam
-// scratch it needs (floats); and the launches (sweep, then merge).
+// Whether the sweep handles this geometry and form; its CTA grid (the most
+// segments it may be run with); the seam scratch that needs (floats, zeroed
+// before its first use: rows, then the counters); and the launch.
 bool sweep_supported(int form, const Geo& g, int bm);
-void sweep_plan(int form, const Geo& g, int sm_count, int* strips, int* segs);
-size_t sweep_seam_floats(const Geo& g, int segs);
+void sweep_plan(int form, const Geo& g, int sms, int* strips, int* segs);
+size_t sweep_seam_floats(const Geo& g, int strips, int segs);
+// Points sa at seam scratch for at most max_segs segments (null: none).
+inline void set_seams(SweepArgs& sa, float* scratch, int max_segs) {
+  const size_t rows = (size_t)(max_segs - 1) * (sa.inv.g.bh / 2) * sa.seam_w;
+  sa.seam_b = scratch;
+  sa.seam_t = scratch ? scratch + rows : nullptr;
+  sa.seam_cnt = scratch ? reinterpret_cast<int*>(scratch + 3 * rows) : nullptr;
+}
 // `mark` (optional) is recorded after the first kernel: the fast-form sweep,
 // or the tensor-core filter kernel.
 cudaError_t launch_sweep(int form, const SweepArgs& a, cudaStream_t st, cudaEvent_t mark = nullptr);
@@ -218,18 +227,18 @@ cudaError_t launch_sweep_tc_batch(const SweepArgs* planes, int n, const TcTune& 
 cudaError_t tc_graph_update(cudaGraphExec_t exec, cudaGraph_t graph, const TcFwdArgs* fwd, int nf,
                             const SweepArgs* sw, int ns);
 // Tensor-core sweep: cells per strip, CTAs per SM, and the launches (filter,
-// inverse + overlap-add, seam merge of f3d_k_sweep.cu).
+// inverse + overlap-add).
 int tc_sweep_cells(int n);  // 7 for 32 x 32 blocks, 15 for 16 x 16
 constexpr int kTcSweepCtasPerSm = 3;
 cudaError_t launch_sweep_tc(const SweepArgs& a, cudaStream_t st, cudaEvent_t mark);
 // The fast form's fused sweeps of n planes (8x8 to 32x32 blocks, one
-// temporal mode) in one launch, then their seam rows in one more; `mark` is
-// recorded between the two.
+// temporal mode) in one launch; `mark` is recorded after it.
 cudaError_t launch_sweep_fast_batch(const SweepArgs* planes, int n, cudaStream_t st, cudaEvent_t mark);
-cudaError_t launch_seam_merge_batch(const SweepBatch& Bm, int n, int maxw, int ch, cudaStream_t st);
 // Bytes of SweepArgs::img for this geometry and strip count.
 size_t tc_image_bytes(const Geo& g, int strips);
-cudaError_t launch_seam_merge(const SweepArgs& a, cudaStream_t st);
+
+// SMs of the current device.
+int sm_count();
 
 // Counts one kernel launch made by this library (all engines, all threads).
 void count_launch();
