@@ -111,6 +111,26 @@ inline void plan_segments(SweepArgs* planes, int n, int slots) {
   for (int i = 0; i < n; i++) planes[i].segs = segs_of(planes[i], best);
 }
 
+// The filter's batch parameter of the planes of a sweep batch (sweep_batches):
+// the same runs, with the prefix of the planes' groups of `group` blocks.
+// Returns the CTAs (groups) of the launch.
+inline int filter_batch(const SweepBatch& S, int group, FilterBatch& F) {
+  F.n = S.n;
+  F.shifted = S.shifted;
+  F.cta0[0] = 0;
+  for (int i = 0; i < S.n; i++) {
+    const SweepArgs& a = S.p[i];
+    F.p[i].f = a.inv;
+    F.p[i].img = a.img;
+    F.p[i].nblk = (a.cells_y + 1) * a.inv.g.ncols;
+    F.run[i] = S.run[i];
+    F.rlen[i] = S.rlen[i];
+    F.cta0[i + 1] = F.cta0[i] + (F.p[i].nblk + group - 1) / group;
+  }
+  for (int i = S.n + 1; i <= kMaxBatch; i++) F.cta0[i] = F.cta0[S.n];
+  return F.cta0[S.n];
+}
+
 // Autotuner choice among n timed launch shapes (fastest[i]: the fastest of
 // shape i's runs; shape 0 is the default): the fastest shape, unless the
 // default is within `margin` of it (single-step timings vary by about 1 %).

@@ -121,6 +121,16 @@ __device__ __forceinline__ void wienner(float& re, float& im, float sx, float sy
   im *= mul;
 }
 
+// a * b, in the fast forms rounded by itself: without it the compiler may
+// fuse the product into a following addition or not, depending on the code
+// around it (whether the filter's switches are read at run time, for one), and
+// the forms' kernels would round differently.
+template <bool FAST>
+__device__ __forceinline__ float prod(float a, float b) {
+  if constexpr (FAST) return __fmul_rn(a, b);
+  else return a * b;
+}
+
 // The same shrink for the fast forms. With sx = beta * sy (both the plain
 // and the pattern sigmas are built that way) the factor 1 - sy/psd passes
 // beta_x = 1 - 1/beta exactly at psd = sx and grows with psd, so the
@@ -133,8 +143,8 @@ __device__ __forceinline__ void wienner_t(float& re, float& im, float sx, float 
   }
   const float psd = fmaf(re, re, im * im);
   const float mul = fmaxf(fmaf(-sy, 1.0f / psd, 1.0f), beta_x);
-  re *= mul;
-  im *= mul;
+  re = prod<true>(re, mul);
+  im = prod<true>(im, mul);
 }
 
 // Fast forms, temporal modes 2-4: the Wiener gain of one temporal
@@ -163,7 +173,7 @@ struct BinTables {
   float2 gs;
   float pat, shp;
 };
-__device__ __forceinline__ BinTables bin_tables(const InvArgs& a, int i) {
+__device__ __forceinline__ BinTables bin_tables(const FilterArgs& a, int i) {
   BinTables t{make_float2(0.0f, 0.0f), 0.0f, 0.0f};
   if (a.dg) t.gs = a.gs[i];
   if (a.pat) t.pat = a.pattern[i];
@@ -176,7 +186,7 @@ struct KState {
   float2 last;
   float cov, proc;
 };
-__device__ __forceinline__ KState load_kstate(const InvArgs& a, size_t gi) {
+__device__ __forceinline__ KState load_kstate(const FilterArgs& a, size_t gi) {
   KState k{make_float2(0.0f, 0.0f), 0.0f, 0.0f};
   if (!a.kalman_init) {
     k.last = a.klast[gi];
@@ -197,13 +207,13 @@ __device__ __forceinline__ KState load_kstate(const InvArgs& a, size_t gi) {
 // ks: the bin's Kalman state (bm 0) as load_kstate read it, so that a
 // caller can issue the loads of several bins before their updates.
 template <int BM, bool FAST = false>
-__device__ __forceinline__ float2 filter_vals_ks(const InvArgs& a, float dc, const BinTables& tb, size_t gi,
+__device__ __forceinline__ float2 filter_vals_ks(const FilterArgs& a, float dc, const BinTables& tb, size_t gi,
                                                  const float2 (&sv)[4], const KState& ks) {
   float d_re = 0.0f, d_im = 0.0f;
   if (a.dg) {
     const float2 g = tb.gs;
-    d_re = dc * g.x;
-    d_im = dc * g.y;
+    d_re = prod<FAST>(dc, g.x);
+    d_im = prod<FAST>(dc, g.y);
   }
   float sx = a.sigma_x, sy = a.sigma_y;
   if (a.pat) {
@@ -377,11 +387,12 @@ __device__ __forceinline__ float2 filter_vals_ks(const InvArgs& a, float dc, con
       re -= d_re;
       im -= d_im;
     }
-    float psd = re * re + im * im + 0.0000000000000000000000000000000000001f;
+    float psd = FAST ? fmaf(re, re, prod<FAST>(im, im)) : re * re + im * im;
+    psd += 0.0000000000000000000000000000000000001f;
     float factor = tb.shp;
     float g = 1.0f + factor * sqrtf(psd * a.ssmax / ((psd + a.ssmin) * (psd + a.ssmax)));
-    re *= g;
-    im *= g;
+    re = prod<FAST>(re, g);
+    im = prod<FAST>(im, g);
     if (a.dg) {
       re += d_re;
       im += d_im;
@@ -394,7 +405,7 @@ __device__ __forceinline__ float2 filter_vals_ks(const InvArgs& a, float dc, con
 
 // filter_vals_ks with the Kalman state read here.
 template <int BM, bool FAST = false>
-__device__ __forceinline__ float2 filter_vals_t(const InvArgs& a, float dc, const BinTables& tb, size_t gi,
+__device__ __forceinline__ float2 filter_vals_t(const FilterArgs& a, float dc, const BinTables& tb, size_t gi,
                                                 const float2 (&sv)[4]) {
   const int bm = BM == kRuntimeBm ? a.bm : BM;
   KState ks{make_float2(0.0f, 0.0f), 0.0f, 0.0f};
@@ -403,13 +414,13 @@ __device__ __forceinline__ float2 filter_vals_t(const InvArgs& a, float dc, cons
 }
 
 template <int BM, bool FAST = false>
-__device__ __forceinline__ float2 filter_vals(const InvArgs& a, float dc, int i, size_t gi, const float2 (&sv)[4]) {
+__device__ __forceinline__ float2 filter_vals(const FilterArgs& a, float dc, int i, size_t gi, const float2 (&sv)[4]) {
   return filter_vals_t<BM, FAST>(a, dc, bin_tables(a, i), gi, sv);
 }
 
 // The window's spectra of bin gi, in temporal order (frames the mode reads).
 template <int BM>
-__device__ __forceinline__ void load_window(const InvArgs& a, size_t gi, float2 (&sv)[4]) {
+__device__ __forceinline__ void load_window(const FilterArgs& a, size_t gi, float2 (&sv)[4]) {
   const int bm = BM == kRuntimeBm ? a.bm : BM;
   const int nf = bm >= 2 ? bm : 1;
 #pragma unroll
@@ -418,7 +429,7 @@ __device__ __forceinline__ void load_window(const InvArgs& a, size_t gi, float2 
 }
 
 template <int BM, bool FAST = false>
-__device__ __forceinline__ float2 filter_bin_t(const InvArgs& a, float dc, int i, size_t gi) {
+__device__ __forceinline__ float2 filter_bin_t(const FilterArgs& a, float dc, int i, size_t gi) {
   float2 sv[4];
   load_window<BM>(a, gi, sv);
   return filter_vals<BM, FAST>(a, dc, i, gi, sv);

@@ -546,7 +546,7 @@ int f3d_engine_create(const f3d_script_params* sp, const f3d_plane_geom* geom,
                            (ce = cudaMemsetAsync(e->d_seam, 0, sizeof(float) * e->seam_floats, e->stream)) != cudaSuccess))
       return finish_fail(e->cuda_fail(ce, "seam buffer allocation"));
     if (e->inv_form == F3D_FORM_TC) {
-      e->img_bytes = tc_image_bytes(geo, e->sweep_strips);
+      e->img_bytes = tc_image_bytes(geo);
       if ((ce = e->alloc(&e->d_img, e->img_bytes)) != cudaSuccess)
         return finish_fail(e->cuda_fail(ce, "tensor-core operand buffer allocation"));
     }
@@ -1081,7 +1081,7 @@ int f3d_batch_step(f3d_batch* b, const int* fns, const void* const* dev_src, con
   // 1-3 % slower in steady state at eight and ten outputs.
   const uint64_t all = (1ull << n) - 1;
   if (!b->fast && (b->flags & F3D_BATCH_AUTOTUNE) && !b->tuned && (mask & 0xFFFFFFFFull) == (all | (all << 16))) {
-    const TcTune cands[] = {{3, 5}, {2, 5}, {1, 5}, {3, 4}, {2, 4}, {1, 4}, {3, 3}, {2, 3}, {1, 3}};
+    const TcTune cands[] = {{3, 5}, {2, 5}, {1, 5}, {3, 4}, {2, 4}, {1, 4}};
     constexpr int kCands = sizeof(cands) / sizeof(cands[0]);
     cudaEvent_t t0, t1;
     cudaEventCreate(&t0);

@@ -91,10 +91,6 @@ __device__ __forceinline__ uint64_t a2_desc(uint32_t base, int ks) {
 }
 
 constexpr int kTcThreads = 256;
-// Filter-kernel variants: CTAs per SM (minb) and filter_batch(minb), the
-// blocks of a group whose spectra loads are in flight together; fewer CTAs
-// leave registers for deeper batches.
-__host__ __device__ constexpr int filter_batch(int minb) { return minb >= 5 ? 1 : 2; }
 constexpr uint64_t kWaitNs = 1000000000ull;  // one second
 
 // ---- forward ---------------------------------------------------------------
@@ -474,22 +470,20 @@ __global__ void __launch_bounds__(kTcThreads, kFwdMaxCtasPerSm) k_forward_tc(con
 
 // ---- sweep: filter, then inverse + overlap-add -------------------------------
 //
-// The tensor-core counterpart of the fast-form sweep (f3d_k_sweep.cu). The
-// plane is cut into strips of TJ = 7 cells; the group of a strip in block row
-// m is block columns J0..J0+7 (the last one the strip's right neighbour).
+// The tensor-core counterpart of the fast-form sweep (f3d_k_sweep.cu).
 //
-// k_filter_tc, one CTA per (row, strip) group:
-//   F: the temporal filter (filter_vals, fast form) of the group's 8 x 544
-//      bins, contiguous in HBM, into shared memory;
-//   R: rows (k', block) of the column-inverse operand, k' = 0 packing the
-//      Hermitian parts of columns 0 and n/2 as H0 + i H(n/2), scaled by
-//      kInvPre and split hi/lo, written to HBM as the exact shared-memory
-//      image (SWIZZLE_128B) the inverse kernel loads with one bulk copy.
-// With no tensor-memory phases to wait for, it runs at five CTAs per SM.
+// k_filter_tc: the temporal filter (filter_vals, fast form) of every block's
+// bins; the block's part of the column-inverse operand, rows k' (k' = 0
+// packing the Hermitian parts of columns 0 and n/2 as H0 + i H(n/2)), scaled
+// by kInvPre and split hi/lo, leaves as the block's image (BlkImg): the exact
+// shared-memory bytes, so that the images of consecutive blocks are an operand
+// tile.
 //
-// k_sweep_tc, one CTA per (strip, segment of block rows), per row:
-//   the operand tile arrives by bulk copy (issued while the previous row's
-//   transforms ran);
+// k_sweep_tc: the plane is cut into strips of TJ = 7 cells, covered by block
+// columns J0..J0+7 (the last one the strip's right neighbour). One CTA per
+// (strip, segment of block rows), per row:
+//   the images of the row's 8 blocks arrive by one bulk copy (issued while the
+//   previous row's transforms ran);
 //   step 2': V[y][k'] = sum_ky e^(2 pi i ky y/n) sy[y] F[ky][k'] (tensor cores);
 //   V: V into the row-inverse operand, rows (y, block slot) of two tiles
 //      that hold the even and the odd block columns;
@@ -500,41 +494,55 @@ __global__ void __launch_bounds__(kTcThreads, kFwdMaxCtasPerSm) k_forward_tc(con
 //      reference's block order (src/cpu/reference.cpp:415-436), finished cell
 //      rows packed straight to the output plane; segment seams as in the
 //      fast-form sweep.
+
+// A block's operand image: rows k' = 0..n/2-1, K = 2 ky + (re, im), in 8-row
+// atoms, each atom's hi part followed by its lo part, so that the atoms of
+// consecutive blocks are evenly spaced. n = 32: two SWIZZLE_128B atoms of
+// 1024 bytes; n = 16: one interleaved atom of 512.
+template <int N>
+struct BlkImg {
+  static constexpr uint32_t BYTES = 4 * N * N;
+  static constexpr uint32_t LO = N == 32 ? 1024 : 512;  // from a hi part to its lo part
+  static constexpr uint32_t SBO = 2 * LO;               // from atom to atom
+};
+template <int N>
+__host__ __device__ constexpr uint32_t img_off(int kp, int ky) {
+  return (kp >> 3) * BlkImg<N>::SBO + (N == 32 ? tc::off_sw128(kp & 7, 2 * ky) : tc::off_il(kp & 7, 2 * ky, 2 * N));
+}
+// Descriptor of K-step ks (16 columns) of the hi parts of a tile of images at base.
+template <int N>
+__device__ __forceinline__ uint64_t img_desc(uint32_t base, int ks) {
+  if constexpr (N == 32) return tc::sdesc(base + ks * 32, 16, BlkImg<N>::SBO, tc::LAYOUT_SW128);
+  else return tc::sdesc(base + ks * 256, 128, BlkImg<N>::SBO, tc::LAYOUT_INTERLEAVE);
+}
+
 template <int N>
 struct SwpCfg {
   using C = TcCfg<N>;
   static constexpr int TJ = C::G - 1;        // cells per strip
   static constexpr int CH = N / 2, CW = N / 2;
-  // Filtered-bin stride per block (float2), padded: in R a half-warp reads
-  // the same bin of 8 blocks for 2 k', which fall in 16 distinct bank pairs
-  // when FS / 2 is odd.
-  static constexpr int FS = C::PS + 2;
-  static_assert(FS % 4 == 2, "R-phase loads free of bank conflicts");
   static constexpr int PR = CW + 4;          // partial-sum row stride (floats), padded
   static constexpr int PC = CH * PR + 4;     // partial-sum cell stride (floats), padded
-  static constexpr uint32_t TILE = 2 * C::A2_BYTES;                  // operand image: hi, lo
+  static constexpr uint32_t TILE = C::G * BlkImg<N>::BYTES;          // operand tile: the images of a row's blocks
   // Inverse kernel shared memory.
   static constexpr uint32_t C2 = 0;                                  // hi, lo
   static constexpr uint32_t C1 = C2 + 2 * C::B2_BYTES;               // A hi, A lo, B hi, B lo
-  static constexpr uint32_t A2 = (C1 + 4 * C::B1_BYTES + 1023) / 1024 * 1024;  // hi, lo (SWIZZLE_128B)
+  static constexpr uint32_t A2 = (C1 + 4 * C::B1_BYTES + 1023) / 1024 * 1024;  // the operand tile
   // A1 shares A2's space: step 2' has read the operand tile before V writes
   // A1, and the next tile is loaded once step 1' has read A1. Three CTAs fit
   // on an SM.
-  static constexpr uint32_t A1 = A2;                                 // [tile][hi, lo] (INTERLEAVE)
-  // The second tile starts 64 B further than its hi + lo: in V the lanes of
-  // the two tiles store to the same offsets, which then fall in different
-  // banks.
-  static constexpr uint32_t A1_STRIDE = 2 * C::A1_BYTES + 64;
-  static constexpr uint32_t P = A2 + (C::T1 - 1) * A1_STRIDE + 2 * C::A1_BYTES;  // [2][TJ][PC] floats
+  static constexpr uint32_t A1 = A2;                                 // [tile][hi, lo] (SWIZZLE_64B / 32B)
+  static constexpr uint32_t A1_STRIDE = 2 * C::A1_BYTES;
+  // The row of (y, slot) in the second tile, against the first: in V half the
+  // lanes store to each tile, whose rows then fall in different banks.
+  static constexpr int FLIP = N == 32 ? 1 : 2;
+  static constexpr uint32_t P = A2 + TILE;                           // [2][TJ][PC] floats
   static constexpr uint32_t BAR = P + 2 * TJ * PC * 4;               // operand load, step 2', step 1'
   static constexpr uint32_t TSLOT = BAR + 24;
   static constexpr uint32_t BYTES = TSLOT + 8 + 1024;
-  // Filter kernel shared memory.
-  static constexpr uint32_t F_DC = C::G * FS * 8;
-  static constexpr uint32_t F_BYTES = F_DC + C::G * 4;
   static_assert(C::T1 == 2, "one tile per block-column parity");
-  static_assert(P >= A2 + TILE, "the operand tile fits below the partial sums");
-  static_assert(A1_STRIDE % 16 == 0, "operand start addresses are 16-byte aligned");
+  static_assert(A1_STRIDE * C::T1 <= TILE, "the row-inverse operand fits in the operand tile's space");
+  static_assert(A1_STRIDE % 512 == 0 && C::A1_BYTES % 512 == 0, "swizzle atoms");
   static_assert(BAR % 8 == 0 && P % 16 == 0, "alignment");
 };
 
@@ -590,93 +598,61 @@ __device__ __forceinline__ float2 spec_at(const float2* s, size_t j) {
   else return s[j];
 }
 
-// R. Row (k', block), K = 2 ky + (re, im) of the operand image of a group
-// from its filtered bins fbuf[block][bin], in 16-byte chunks of 4 ky, into
-// img. prev (optional) also receives block 0, as the previous strip's block
-// 7; with skip_last the group's block 7 is not written (the next strip
-// writes it).
+// Filter kernel: one CTA per group of G consecutive blocks (8 of 32 x 32, 16
+// of 16 x 16), whose spectra and images are contiguous. It is bound by the
+// instructions per bin (75 % of the issue slots with ten outputs in a launch)
+// and, with one output, by HBM (5.3 TB/s of reads and image writes). Each
+// result goes straight to its place in the group's images, which leave by one
+// bulk copy; the results of columns 0 and n/2 pass through `side`. Figures,
+// 1080p 10-bit bt=4 with sharpen, ten outputs / one: 251 / 42.8 us with the
+// switches read per bin and the results transposed through a buffer of
+// filtered bins (131 instructions per bin), 173 / 36.1 us now (108).
 template <int N>
-__device__ __forceinline__ void tile_rows(uint8_t* img, uint8_t* prev, bool skip_last, const float2* fbuf,
-                                          int tid) {
+struct FltCfg {
   using C = TcCfg<N>;
-  using S = SwpCfg<N>;
-  const int r2 = tid & 127, h = tid >> 7;
-  const int kp = r2 / C::G, bl = r2 % C::G;
-  if (bl == C::G - 1 && skip_last) return;
-  const float2* fb = fbuf + bl * S::FS;
-#pragma unroll
-  for (int cq = 0; cq < C::NY / 4; cq++) {
-    uint32_t hi[4], lo[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int ky = C::NY * h + 4 * cq + u;
-      float2 z;
-      if (kp == 0) {
-        const int kym = (N - ky) & (N - 1);
-        const float2 f0 = fb[ky * C::FBW], f0m = fb[kym * C::FBW];
-        const float2 fn = fb[ky * C::FBW + C::NY], fnm = fb[kym * C::FBW + C::NY];
-        const float h0x = 0.5f * (f0.x + f0m.x), h0y = 0.5f * (f0.y - f0m.y);
-        const float hnx = 0.5f * (fn.x + fnm.x), hny = 0.5f * (fn.y - fnm.y);
-        z = make_float2(h0x - hny, h0y + hnx);
-      } else {
-        z = fb[ky * C::FBW + kp];
-      }
-      tc::split_pair(z.x * kInvPre, z.y * kInvPre, hi[u], lo[u]);
-    }
-    const uint32_t o = a2_off<N>(r2, 2 * (C::NY * h + 4 * cq));
-    *reinterpret_cast<uint4*>(img + o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    *reinterpret_cast<uint4*>(img + C::A2_BYTES + o) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-    if (bl == 0 && prev) {
-      const uint32_t op = a2_off<N>(r2 + C::G - 1, 2 * (C::NY * h + 4 * cq));
-      *reinterpret_cast<uint4*>(prev + op) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-      *reinterpret_cast<uint4*>(prev + C::A2_BYTES + op) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-    }
+  static constexpr uint32_t IMG = BlkImg<N>::BYTES;
+  static constexpr uint32_t SIDE = C::G * IMG;                   // float2 [G][2][N]: columns 0 and n/2
+  static constexpr uint32_t DC = SIDE + C::G * 2 * N * 8;        // float [G]
+  static constexpr uint32_t BYTES = DC + C::G * 4;
+};
+
+// The switches of the temporal filter as the kernel is built for them: the
+// two usual sets fixed at compile time, or read per bin (about ten
+// instructions of branches per bin). Products that are added later are
+// rounded by themselves (prod), so the three give the same bits.
+enum FilterSwitches { kSwPlain = 0, kSwSharpen = 1, kSwAny = 2 };  // degrid; degrid + sharpen; any
+template <int SW>
+__device__ __forceinline__ void fix_switches(FilterArgs& f) {
+  if constexpr (SW != kSwAny) {
+    f.dg = 1;
+    f.pat = 0;
+    f.shp = SW == kSwSharpen;
   }
 }
 
-// The operand image of group (m, strip) in HBM: block 0 also goes to the
-// previous strip's tile as its block 7; this tile's block 7 comes from the
-// next strip.
+// One bin's result into the image at img (offset `at` of its hi part), or,
+// of columns 0 and n/2, into side.
 template <int N>
-__device__ __forceinline__ void operand_tile(const SweepArgs& sa, int m, int strip, const float2* fbuf, int tid) {
-  using S = SwpCfg<N>;
-  uint8_t* img = sa.img + ((size_t)m * sa.strips + strip) * S::TILE;
-  tile_rows<N>(img, strip > 0 ? img - S::TILE : nullptr, strip != sa.strips - 1, fbuf, tid);
-}
-
-// Start of a group's filter: its window spectra begin moving into L2 as
-// whole runs (of shifted windows, only the newest frame: the others are an
-// earlier output's), and the current frame's DC of each block (the degrid
-// correction's scale) goes to dcs. gb0: the group's first bin; nvbin: the
-// bins filtered.
-template <int N, int NF, bool HALF>
-__device__ __forceinline__ void group_start(const SweepArgs& sa, size_t gb0, int nvbin, bool shifted, int m, int J0,
-                                            float* dcs, int tid) {
-  using C = TcCfg<N>;
-  const InvArgs& a = sa.inv;
-  constexpr uint32_t BIN_BYTES = HALF ? 4 : 8;
-  const bool pull = !shifted || tid == NF - 1;
-  if (tid < NF && nvbin > 0 && pull)
-    tc::prefetch_l2(reinterpret_cast<const uint8_t*>(a.s[tid]) + gb0 * BIN_BYTES, (uint32_t)(nvbin * BIN_BYTES));
-  if (tid < C::G) {
-    const int n = J0 + tid;
-    dcs[tid] = (a.dg && n <= sa.cells_x && n < a.g.ncols)
-                   ? spec_at<HALF>(a.s[a.cur], (size_t)(m * a.g.ncols + n) * C::PS).x
-                   : 0.0f;
+__device__ __forceinline__ void put_bin(uint8_t* img, float2* side, bool packed, uint32_t at, int side_at, float2 f) {
+  if (packed) {
+    side[side_at] = f;
+  } else {
+    uint32_t hi, lo;
+    tc::split_pair(f.x * kInvPre, f.y * kInvPre, hi, lo);
+    *reinterpret_cast<uint32_t*>(img + at) = hi;
+    *reinterpret_cast<uint32_t*>(img + at + BlkImg<N>::LO) = lo;
   }
 }
 
-// F. The temporal filter (filter_vals, fast form) of a group's nvb blocks
-// into fbuf[block][bin] (blocks nvb.. get zeros). Thread t filters bin
-// li = t + 256 r (r < NL) of every block of the group, the bin's tables read
-// once for all blocks, then tail item q: bin NL * 256 + e % TAIL of block
-// e / TAIL, e = t + 256 q. The spectra loads of BATCH blocks are issued
-// together; every index is the thread's base plus a constant.
+// The temporal filter (filter_vals, fast form) of a group's nvb blocks.
+// Thread t filters bin li = t + 256 r (r < NL) of every block of the group,
+// the bin's tables read once for all blocks, then tail item q: bin NL * 256 +
+// e % TAIL of block e / TAIL, e = t + 256 q. The spectra loads of BATCH blocks
+// are issued together; every index is the thread's base plus a constant.
 template <int N, int BM, int BATCH, bool HALF>
-__device__ __forceinline__ void filter_group(const InvArgs& a, size_t gb0, int nvb, const float* dcs, float2* fbuf,
-                                             int tid) {
+__device__ __forceinline__ void filter_group(const FilterArgs& a, size_t gb0, int nvb, const float* dcs, uint8_t* img,
+                                             float2* side, int tid) {
   using C = TcCfg<N>;
-  using S = SwpCfg<N>;
   constexpr int NF = BM >= 2 ? BM : 1;
   constexpr int NL = C::PS / kTcThreads;
   constexpr int TAIL = C::PS - NL * kTcThreads;
@@ -686,8 +662,17 @@ __device__ __forceinline__ void filter_group(const InvArgs& a, size_t gb0, int n
   const size_t gt = gb0 + tid;
   if constexpr (NL > 0) {
     BinTables tb[NL];
+    uint32_t at[NL];
+    int side_at[NL];
+    bool packed[NL];
 #pragma unroll
-    for (int r = 0; r < NL; r++) tb[r] = bin_tables(a, tid + kTcThreads * r);
+    for (int r = 0; r < NL; r++) {
+      const int li = tid + kTcThreads * r, ky = li / C::FBW, kx = li - ky * C::FBW;
+      tb[r] = bin_tables(a, li);
+      at[r] = img_off<N>(kx & (C::NY - 1), ky);
+      side_at[r] = (kx ? N : 0) + ky;
+      packed[r] = kx == 0 || kx == C::NY;
+    }
 #pragma unroll
     for (int b0 = 0; b0 < C::G; b0 += BATCH) {
       float2 sv[BATCH][NL][4];
@@ -703,14 +688,12 @@ __device__ __forceinline__ void filter_group(const InvArgs& a, size_t gb0, int n
 #pragma unroll
       for (int u = 0; u < BATCH; u++) {
         const int b = b0 + u;
+        if (b >= nvb) continue;
         const float dc = dcs[b];
 #pragma unroll
-        for (int r = 0; r < NL; r++) {
-          const int li = tid + kTcThreads * r;
-          float2 f = make_float2(0.0f, 0.0f);
-          if (b < nvb) f = filter_vals_t<BM, true>(a, dc, tb[r], gb0 + (size_t)b * C::PS + li, sv[u][r]);
-          fbuf[b * S::FS + li] = f;
-        }
+        for (int r = 0; r < NL; r++)
+          put_bin<N>(img + b * BlkImg<N>::BYTES, side + b * 2 * N, packed[r], at[r], side_at[r],
+                     filter_vals_t<BM, true>(a, dc, tb[r], 0, sv[u][r]));
       }
     }
   }
@@ -718,21 +701,22 @@ __device__ __forceinline__ void filter_group(const InvArgs& a, size_t gb0, int n
   for (int q = 0; q < NT; q++) {
     const int e = tid + kTcThreads * q;
     const int b = e / TAIL, li = NL * kTcThreads + e % TAIL;
-    float2 f = make_float2(0.0f, 0.0f);
-    if (b < nvb) {
-      float2 sv[4];
+    if (b >= nvb) continue;
+    const int ky = li / C::FBW, kx = li - ky * C::FBW;
+    float2 sv[4];
 #pragma unroll
-      for (int k = 0; k < NF; k++) sv[k] = spec_at<HALF>(a.s[k], gb0 + (size_t)b * C::PS + li);
-      f = filter_vals_t<BM, true>(a, dcs[b], bin_tables(a, li), gb0 + (size_t)b * C::PS + li, sv);
-    }
-    fbuf[b * S::FS + li] = f;
+    for (int k = 0; k < NF; k++) sv[k] = spec_at<HALF>(a.s[k], gb0 + (size_t)b * C::PS + li);
+    put_bin<N>(img + b * BlkImg<N>::BYTES, side + b * 2 * N, kx == 0 || kx == C::NY, img_off<N>(kx & (C::NY - 1), ky),
+               (kx ? N : 0) + ky, filter_vals_t<BM, true>(a, dcs[b], bin_tables(a, li), 0, sv));
   }
 }
 
-template <int N, int BM, int MINB, bool HALF>
-__global__ void __launch_bounds__(kTcThreads, MINB) k_filter_tc(const __grid_constant__ SweepBatch B) {
+template <int N, int BM, int MINB, int SW, bool HALF>
+__global__ void __launch_bounds__(kTcThreads, MINB) k_filter_tc(const __grid_constant__ FilterBatch B) {
   using C = TcCfg<N>;
-  using S = SwpCfg<N>;
+  using K = FltCfg<N>;
+  constexpr int NF = BM >= 2 ? BM : 1;  // window frames read
+  constexpr uint32_t BLK = C::PS * (HALF ? 4 : 8);
   // A run of planes of one geometry (e.g. consecutive frames of a plane)
   // runs the same group of each of its planes back to back, so that the
   // window spectra they share are read from L2 the second time.
@@ -740,29 +724,40 @@ __global__ void __launch_bounds__(kTcThreads, MINB) k_filter_tc(const __grid_con
   const int rl = B.rlen[r0];
   const int local = (int)blockIdx.x - B.cta0[r0];
   const int pl = r0 + local % rl;
-  const SweepArgs& sa = B.p[pl];
-  const int cta = local / rl;
-  const InvArgs& a = sa.inv;
-  extern __shared__ __align__(16) uint8_t smem_f[];
-  float2* fbuf = reinterpret_cast<float2*>(smem_f);
-  float* dcs = reinterpret_cast<float*>(smem_f + S::F_DC);
+  const FilterPlane& P = B.p[pl];
+  FilterArgs a = P.f;
+  fix_switches<SW>(a);
+  extern __shared__ __align__(128) uint8_t smem_f[];
+  float2* side = reinterpret_cast<float2*>(smem_f + K::SIDE);
+  float* dcs = reinterpret_cast<float*>(smem_f + K::DC);
   const int tid = threadIdx.x;
-  const int strip = cta % sa.strips, m = cta / sa.strips;
-  const int J0 = strip * S::TJ;
-  const int ncols = a.g.ncols;
-  // A tile's eighth block is the next strip's first: that strip filters it
-  // and writes it into both tiles, so each block is filtered once. The last
-  // strip filters its own eighth block.
-  const bool last_strip = strip == sa.strips - 1;
-  const int own = last_strip ? C::G : C::G - 1;
-  const int nvb = max(0, min(own, min(sa.cells_x + 1, ncols) - J0));  // blocks filtered here
-  constexpr int NF = BM >= 2 ? BM : 1;  // window frames read
-  const size_t gb0 = ((size_t)m * ncols + J0) * C::PS;
-  group_start<N, NF, HALF>(sa, gb0, nvb * C::PS, (B.shifted >> pl) & 1, m, J0, dcs, tid);
+  const int b0 = local / rl * C::G, nvb = min(C::G, P.nblk - b0);
+  const size_t gb0 = (size_t)b0 * C::PS;
+  // The window spectra begin moving into L2 as whole runs (of shifted
+  // windows, only the newest frame: the others are an earlier output's).
+  if (tid < NF && (!((B.shifted >> pl) & 1) || tid == NF - 1))
+    tc::prefetch_l2(reinterpret_cast<const uint8_t*>(P.f.s[tid]) + b0 * (size_t)BLK, nvb * BLK);
+  // The current frame's DC of each block (the degrid correction's scale).
+  if (tid < nvb) dcs[tid] = a.dg ? spec_at<HALF>(P.f.s[P.f.cur], (size_t)(b0 + tid) * C::PS).x : 0.0f;
   __syncthreads();
-  filter_group<N, BM, filter_batch(MINB), HALF>(a, gb0, nvb, dcs, fbuf, tid);
+  filter_group<N, BM, MINB >= 5 ? 1 : 2, HALF>(a, gb0, nvb, dcs, smem_f, side, tid);
   __syncthreads();
-  operand_tile<N>(sa, m, strip, fbuf, tid);
+  {  // Row k' = 0 of block tid / N: the Hermitian parts of columns 0 and n/2, H0 + i H(n/2).
+    const int ky = tid % N, kym = (N - ky) & (N - 1);
+    const float2* f0 = side + tid / N * 2 * N;
+    const float2* fn = f0 + N;
+    const float2 p = f0[ky], pm = f0[kym], n = fn[ky], nm = fn[kym];
+    const float h0x = 0.5f * (p.x + pm.x), h0y = 0.5f * (p.y - pm.y);
+    const float hnx = 0.5f * (n.x + nm.x), hny = 0.5f * (n.y - nm.y);
+    put_bin<N>(smem_f + tid / N * K::IMG, nullptr, false, img_off<N>(0, ky), 0, make_float2(h0x - hny, h0y + hnx));
+  }
+  tc::fence_async_smem();
+  __syncthreads();
+  if (tid == 0) {
+    tc::bulk_store(P.img + (size_t)b0 * K::IMG, smem_f, nvb * K::IMG);
+    tc::bulk_commit();
+    tc::bulk_wait();
+  }
 }
 
 // Shared-memory and barrier state of the inverse phases of one CTA.
@@ -798,8 +793,8 @@ __device__ __forceinline__ bool inverse_row(const SweepArgs& sa, InvState& st, i
     const uint32_t sbo_b = (C::K2 / 8) * 128;
     const uint32_t d = tmem + C::D2_COL;
     for (int ks = 0; ks < C::K2 / 16; ks++) {
-      const uint64_t ah = a2_desc<N>(sbase + S::A2, ks);
-      const uint64_t al = a2_desc<N>(sbase + S::A2 + C::A2_BYTES, ks);
+      const uint64_t ah = img_desc<N>(sbase + S::A2, ks);
+      const uint64_t al = img_desc<N>(sbase + S::A2 + BlkImg<N>::LO, ks);
       const uint64_t bh = tc::sdesc(sbase + S::C2 + ks * 256, 128, sbo_b, tc::LAYOUT_INTERLEAVE);
       const uint64_t bl = tc::sdesc(sbase + S::C2 + C::B2_BYTES + ks * 256, 128, sbo_b, tc::LAYOUT_INTERLEAVE);
       tc::mma_f16(d, ah, bh, id2, ks > 0);
@@ -818,8 +813,8 @@ __device__ __forceinline__ bool inverse_row(const SweepArgs& sa, InvState& st, i
   {
     const int s = warp & 3, h = warp >> 2;
     const int r2 = 32 * s + lane;
-    const int kp = r2 / C::G, bl = r2 % C::G;
-    const int tile = (J0 + bl) & 1, slot = bl >> 1;
+    const int kp = r2 % C::NY, bl = r2 / C::NY;
+    const int tile = (J0 + bl) & 1, slot = (bl >> 1) ^ (tile ? S::FLIP : 0);
     uint8_t* t0 = sm + S::A1 + tile * S::A1_STRIDE;
     float v[N];  // half of the N2 = 2N columns: NY values of y, (re, im)
     tc::tmem_ld<N>(tmem + ((uint32_t)(32 * s) << 16) + C::D2_COL + N * h, v);
@@ -828,7 +823,7 @@ __device__ __forceinline__ bool inverse_row(const SweepArgs& sa, InvState& st, i
       const int y = C::NY * h + j;
       uint32_t hi, lo;
       tc::split_pair(v[2 * j], v[2 * j + 1], hi, lo);
-      const uint32_t o = tc::off_il((C::G / 2) * y + slot, 2 * kp, C::K1);
+      const uint32_t o = tc::off_sw_k<C::K1>((C::G / 2) * y + slot, 2 * kp);
       *reinterpret_cast<uint32_t*>(t0 + o) = hi;
       *reinterpret_cast<uint32_t*>(t0 + C::A1_BYTES + o) = lo;
     }
@@ -847,8 +842,8 @@ __device__ __forceinline__ bool inverse_row(const SweepArgs& sa, InvState& st, i
       const uint32_t b_hi = sbase + S::C1 + t * 2 * C::B1_BYTES, b_lo = b_hi + C::B1_BYTES;
       const uint32_t d = tmem + C::D1_COL + t * C::N1;
       for (int ks = 0; ks < C::K1 / 16; ks++) {
-        const uint64_t ah = tc::sdesc(a_hi + ks * 256, 128, sbo, tc::LAYOUT_INTERLEAVE);
-        const uint64_t al = tc::sdesc(a_lo + ks * 256, 128, sbo, tc::LAYOUT_INTERLEAVE);
+        const uint64_t ah = tc::sdesc(a_hi + ks * 32, 16, 16 * N, N == 32 ? tc::LAYOUT_SW64 : tc::LAYOUT_SW32);
+        const uint64_t al = tc::sdesc(a_lo + ks * 32, 16, 16 * N, N == 32 ? tc::LAYOUT_SW64 : tc::LAYOUT_SW32);
         const uint64_t bh = tc::sdesc(b_hi + ks * 256, 128, sbo, tc::LAYOUT_INTERLEAVE);
         const uint64_t bl = tc::sdesc(b_lo + ks * 256, 128, sbo, tc::LAYOUT_INTERLEAVE);
         tc::mma_f16(d, ah, bh, id1, ks > 0);
@@ -874,7 +869,7 @@ __device__ __forceinline__ bool inverse_row(const SweepArgs& sa, InvState& st, i
     const int t = warp >> 2, s = warp & 3;
     const int r = 32 * s + lane;
     const int y = r / (C::G / 2), slot = r % (C::G / 2);
-    const int bl = 2 * slot + ((t ^ J0) & 1);
+    const int bl = 2 * (slot ^ (t ? S::FLIP : 0)) + ((t ^ J0) & 1);
     float v[N];
     tc::tmem_ld<N>(tmem + ((uint32_t)(32 * s) << 16) + C::D1_COL + t * C::N1, v);
 #pragma unroll
@@ -990,16 +985,19 @@ __global__ void __launch_bounds__(kTcThreads, kTcSweepCtasPerSm) k_sweep_tc(cons
   const int M0 = (int)((long long)seg * nrow / sa.segs);
   const int M1 = (int)((long long)(seg + 1) * nrow / sa.segs);
   const int ncell = min(S::TJ, sa.cells_x - J0);
-  auto tile_of = [&](int m) { return sa.img + ((size_t)m * sa.strips + strip) * S::TILE; };
+  // Operand tile of row m: the images of the strip's blocks (the last strip
+  // may have fewer; the operand rows of the others are never looked at).
+  auto tile_of = [&](int m) { return sa.img + ((size_t)m * sa.inv.g.ncols + J0) * BlkImg<N>::BYTES; };
+  const uint32_t tile_bytes = (ncell + 1) * BlkImg<N>::BYTES;
 
   inverse_setup<N>(sa, sm, bar, tslot);
   if (tid == 0) {
     tc::fence_async_smem();
     if (M0 < M1) {
-      tc::mbar_expect_tx(&bar[0], S::TILE);
+      tc::mbar_expect_tx(&bar[0], tile_bytes);
       // A test of the bounded wait leaves this copy out: nothing is then in
       // flight on the barrier, the wait below gives up and the CTA leaves.
-      if (!(sa.test_skip && cta == 0)) tc::bulk_load(sm + S::A2, tile_of(M0), S::TILE, &bar[0]);
+      if (!(sa.test_skip && cta == 0)) tc::bulk_load(sm + S::A2, tile_of(M0), tile_bytes, &bar[0]);
     }
   }
   tc::fence_before_sync();
@@ -1019,8 +1017,8 @@ __global__ void __launch_bounds__(kTcThreads, kTcSweepCtasPerSm) k_sweep_tc(cons
     // next row's tile starts moving in while the overlap-add runs.
     const bool ok = inverse_row<N>(sa, st, m, M0, M1, seg, J0, ncell, [&] {
       if (tid == 0 && m + 1 < M1) {
-        tc::mbar_expect_tx(&bar[0], S::TILE);
-        tc::bulk_load(sm + S::A2, tile_of(m + 1), S::TILE, &bar[0]);
+        tc::mbar_expect_tx(&bar[0], tile_bytes);
+        tc::bulk_load(sm + S::A2, tile_of(m + 1), tile_bytes, &bar[0]);
       }
     });
     if (!ok) break;
@@ -1186,50 +1184,84 @@ cudaError_t launch_forward_tc_batch(const TcFwdArgs* planes, int n, const TcTune
 
 cudaError_t launch_forward_tc(const TcFwdArgs& a, cudaStream_t st) { return launch_forward_tc_batch(&a, 1, TcTune{}, st); }
 
-template <int N, int BM, int MINB, bool HALF>
-cudaError_t launch_filter_bm(const SweepBatch& B, cudaStream_t st) {
-  constexpr size_t smem = SwpCfg<N>::F_BYTES;
-  auto k = k_filter_tc<N, BM, MINB, HALF>;
-  cudaError_t e = prepare(k, smem);
-  if (e != cudaSuccess) return e;
-  if (B.cta0[B.n] == 0) return cudaSuccess;
-  k<<<B.cta0[B.n], kTcThreads, smem, st>>>(B);
-  count_launch();
-  return cudaGetLastError();
-}
+namespace {
 
-template <int N, int MINB, bool HALF>
-cudaError_t launch_filter_h(const SweepBatch& B, int bm, cudaStream_t st) {
+template <int N, int BM, int MINB, int SW>
+const void* filter_kernel_h(bool half) {
+  return half ? (const void*)k_filter_tc<N, BM, MINB, SW, true> : (const void*)k_filter_tc<N, BM, MINB, SW, false>;
+}
+template <int N, int MINB, int SW>
+const void* filter_kernel_bm(int bm, bool half) {
   switch (bm) {
-  case -1: return launch_filter_bm<N, -1, MINB, HALF>(B, st);
-  case 1: return launch_filter_bm<N, 1, MINB, HALF>(B, st);
-  case 2: return launch_filter_bm<N, 2, MINB, HALF>(B, st);
-  case 3: return launch_filter_bm<N, 3, MINB, HALF>(B, st);
-  case 4: return launch_filter_bm<N, 4, MINB, HALF>(B, st);
-  default: return cudaErrorNotSupported;
+  case -1: return filter_kernel_h<N, -1, MINB, SW>(half);
+  case 1: return filter_kernel_h<N, 1, MINB, SW>(half);
+  case 2: return filter_kernel_h<N, 2, MINB, SW>(half);
+  case 3: return filter_kernel_h<N, 3, MINB, SW>(half);
+  case 4: return filter_kernel_h<N, 4, MINB, SW>(half);
+  default: return nullptr;
   }
 }
-
-// The planes of a batch store their spectra alike, fp32 or fp16 (sweep_batches checks).
 template <int N, int MINB>
-cudaError_t launch_filter(const SweepBatch& B, int bm, cudaStream_t st) {
-  return B.p[0].inv.half ? launch_filter_h<N, MINB, true>(B, bm, st) : launch_filter_h<N, MINB, false>(B, bm, st);
+const void* filter_kernel_n(int sw, int bm, bool half) {
+  return sw == kSwPlain     ? filter_kernel_bm<N, MINB, kSwPlain>(bm, half)
+         : sw == kSwSharpen ? filter_kernel_bm<N, MINB, kSwSharpen>(bm, half)
+                            : filter_kernel_bm<N, MINB, kSwAny>(bm, half);
 }
+template <int N>
+const void* filter_kernel(int minb, int sw, int bm, bool half) {
+  return minb >= 5 ? filter_kernel_n<N, 5>(sw, bm, half) : filter_kernel_n<N, 4>(sw, bm, half);
+}
+
+// The switches all planes of a batch share.
+int filter_switches(const SweepBatch& S) {
+  int sw = -1;
+  for (int i = 0; i < S.n; i++) {
+    const FilterArgs& f = S.p[i].inv;
+    const int s = !f.dg || f.pat ? kSwAny : (f.shp ? kSwSharpen : kSwPlain);
+    sw = sw < 0 || sw == s ? s : kSwAny;
+  }
+  return sw;
+}
+
+// The filter launch of a batch (one CTA per group of blocks).
+struct FilterLaunch {
+  const void* kernel = nullptr;
+  int grid = 0;
+  size_t smem = 0;
+};
+FilterLaunch filter_launch(const SweepBatch& S, int minb, FilterBatch& F) {
+  const bool n16 = S.p[0].inv.g.bw == 16;
+  FilterLaunch l;
+  l.grid = filter_batch(S, n16 ? TcCfg<16>::G : TcCfg<32>::G, F);
+  const int sw = filter_switches(S), bm = S.p[0].inv.bm;
+  const bool half = S.p[0].inv.half;  // the planes store their spectra alike (sweep_batches checks)
+  l.kernel = n16 ? filter_kernel<16>(minb, sw, bm, half) : filter_kernel<32>(minb, sw, bm, half);
+  l.smem = n16 ? FltCfg<16>::BYTES : FltCfg<32>::BYTES;
+  return l;
+}
+
+}  // namespace
 
 namespace {
 
 template <int N>
-cudaError_t launch_sweep_n(const SweepBatch& Bf, const SweepBatch& B, int n, const TcTune& t, cudaStream_t st,
-                           cudaEvent_t mark, cudaEvent_t after_filter) {
+cudaError_t launch_sweep_n(const SweepBatch& B, int n, const TcTune& t, cudaStream_t st, cudaEvent_t mark,
+                           cudaEvent_t after_filter) {
   using S = SwpCfg<N>;
-  const int bm = B.p[0].inv.bm;
   constexpr size_t smem = S::BYTES;
   static_assert(kTcSweepCtasPerSm * (S::BYTES + 1024) <= 228 * 1024, "CTAs per SM");
-  // Filter: one CTA per (row, strip) group of every plane.
-  cudaError_t e = t.filter_minb == 3   ? launch_filter<N, 3>(Bf, bm, st)
-                  : t.filter_minb == 4 ? launch_filter<N, 4>(Bf, bm, st)
-                                       : launch_filter<N, 5>(Bf, bm, st);
-  if (e != cudaSuccess) return e;
+  FilterBatch F;
+  const FilterLaunch l = filter_launch(B, t.filter_minb, F);
+  if (!l.kernel) return cudaErrorNotSupported;
+  cudaError_t e = cudaSuccess;
+  if (l.grid > 0) {
+    e = prepare(l.kernel, l.smem);
+    if (e != cudaSuccess) return e;
+    void* args[1] = {&F};
+    e = cudaLaunchKernel(l.kernel, dim3(l.grid), dim3(kTcThreads), args, l.smem, st);
+    if (e != cudaSuccess) return e;
+    count_launch();
+  }
   if (mark) cudaEventRecord(mark, st);
   if (after_filter && (e = cudaEventRecord(after_filter, st)) != cudaSuccess) return e;
   // Inverse + overlap-add: one CTA per (strip, segment) of every plane.
@@ -1240,14 +1272,14 @@ cudaError_t launch_sweep_n(const SweepBatch& Bf, const SweepBatch& B, int n, con
   return cudaGetLastError();
 }
 
-// The filter's and the inverse kernel's batch parameters, with the segments
-// planned for one launch of all planes.
-cudaError_t tc_sweep_batches(const SweepArgs* planes, int n, SweepBatch& Bf, SweepBatch& B) {
+// The inverse kernel's batch parameters, with the segments planned for one
+// launch of all planes.
+cudaError_t tc_sweep_batch(const SweepArgs* planes, int n, SweepBatch& B) {
   if (n < 1 || n > kMaxBatch) return cudaErrorInvalidValue;
   SweepArgs p[kMaxBatch];
   std::copy(planes, planes + n, p);
   plan_segments(p, n, kTcSweepCtasPerSm * sm_count());
-  SweepBatch Bm;
+  SweepBatch Bf, Bm;
   return sweep_batches(p, n, Bf, B, Bm) ? cudaSuccess : cudaErrorNotSupported;
 }
 
@@ -1255,12 +1287,12 @@ cudaError_t tc_sweep_batches(const SweepArgs* planes, int n, SweepBatch& Bf, Swe
 
 cudaError_t launch_sweep_tc_batch(const SweepArgs* planes, int n, const TcTune& t, cudaStream_t st,
                                   cudaEvent_t mark, cudaEvent_t after_filter) {
-  SweepBatch Bf, B;
-  cudaError_t e = tc_sweep_batches(planes, n, Bf, B);
+  SweepBatch B;
+  const cudaError_t e = tc_sweep_batch(planes, n, B);
   if (e != cudaSuccess) return e;
   static_assert(SwpCfg<32>::TJ == 7 && SwpCfg<16>::TJ == 15, "cells per strip");
-  return planes[0].inv.g.bw == 16 ? launch_sweep_n<16>(Bf, B, n, t, st, mark, after_filter)
-                                  : launch_sweep_n<32>(Bf, B, n, t, st, mark, after_filter);
+  return planes[0].inv.g.bw == 16 ? launch_sweep_n<16>(B, n, t, st, mark, after_filter)
+                                  : launch_sweep_n<32>(B, n, t, st, mark, after_filter);
 }
 
 cudaError_t launch_sweep_tc(const SweepArgs& a, cudaStream_t st, cudaEvent_t mark) {
@@ -1268,17 +1300,6 @@ cudaError_t launch_sweep_tc(const SweepArgs& a, cudaStream_t st, cudaEvent_t mar
 }
 
 namespace {
-template <int N, int MINB, bool HALF>
-bool is_filter_h(const void* f) {
-  return f == (const void*)k_filter_tc<N, -1, MINB, HALF> || f == (const void*)k_filter_tc<N, 1, MINB, HALF> ||
-         f == (const void*)k_filter_tc<N, 2, MINB, HALF> || f == (const void*)k_filter_tc<N, 3, MINB, HALF> ||
-         f == (const void*)k_filter_tc<N, 4, MINB, HALF>;
-}
-template <int N>
-bool is_filter(const void* f) {
-  return is_filter_h<N, 3, false>(f) || is_filter_h<N, 3, true>(f) || is_filter_h<N, 4, false>(f) ||
-         is_filter_h<N, 4, true>(f) || is_filter_h<N, 5, false>(f) || is_filter_h<N, 5, true>(f);
-}
 template <int N>
 bool is_forward(const void* f) {
   return f == (const void*)k_forward_tc<N, 1, false> || f == (const void*)k_forward_tc<N, 2, false> ||
@@ -1289,10 +1310,15 @@ bool is_forward(const void* f) {
 cudaError_t tc_graph_update(cudaGraphExec_t exec, cudaGraph_t graph, const TcFwdArgs* fwd, int nf,
                             const SweepArgs* sw, int ns) {
   TcFwdBatch Bw{};
-  SweepBatch Bf, Bs;
+  SweepBatch Bs;
+  FilterBatch F;
+  FilterLaunch fl[2];
   cudaError_t e = cudaSuccess;
   if (nf > 0 && !forward_batch(fwd, nf, Bw)) return cudaErrorNotSupported;
-  if (ns > 0 && (e = tc_sweep_batches(sw, ns, Bf, Bs)) != cudaSuccess) return e;
+  if (ns > 0) {
+    if ((e = tc_sweep_batch(sw, ns, Bs)) != cudaSuccess) return e;
+    for (int v = 0; v < 2; v++) fl[v] = filter_launch(Bs, 4 + v, F);
+  }
   size_t cnt = 0;
   e = cudaGraphGetNodes(graph, nullptr, &cnt);
   if (e != cudaSuccess) return e;
@@ -1306,14 +1332,15 @@ cudaError_t tc_graph_update(cudaGraphExec_t exec, cudaGraph_t graph, const TcFwd
     if ((e = cudaGraphKernelNodeGetParams(node, &kp)) != cudaSuccess) return e;
     void* args[1] = {nullptr};
     const void* f = kp.func;
-    if (is_forward<32>(f) || is_forward<16>(f))
+    if (is_forward<32>(f) || is_forward<16>(f)) {
       args[0] = &Bw;
-    else if (is_filter<32>(f) || is_filter<16>(f))
-      args[0] = &Bf;
-    else if (f == (const void*)k_sweep_tc<32> || f == (const void*)k_sweep_tc<16>)
+    } else if (ns > 0 && (f == fl[0].kernel || f == fl[1].kernel)) {
+      args[0] = &F;
+    } else if (f == (const void*)k_sweep_tc<32> || f == (const void*)k_sweep_tc<16>) {
       args[0] = &Bs;
-    else
+    } else {
       return cudaErrorInvalidValue;
+    }
     kp.kernelParams = args;
     kp.extra = nullptr;
     if ((e = cudaGraphExecKernelNodeSetParams(exec, node, &kp)) != cudaSuccess) return e;
@@ -1321,10 +1348,9 @@ cudaError_t tc_graph_update(cudaGraphExec_t exec, cudaGraph_t graph, const TcFwd
   return cudaSuccess;
 }
 
-size_t tc_image_bytes(const Geo& g, int strips) {
+size_t tc_image_bytes(const Geo& g) {
   const int cells_y = (g.H + g.bh / 2 - 1) / (g.bh / 2);
-  const size_t tile = g.bw == 16 ? SwpCfg<16>::TILE : SwpCfg<32>::TILE;
-  return (size_t)(cells_y + 1) * strips * tile;
+  return (size_t)(cells_y + 1) * g.ncols * (g.bw == 16 ? BlkImg<16>::BYTES : BlkImg<32>::BYTES);
 }
 
 }  // namespace f3d

@@ -45,9 +45,8 @@ struct FwdArgs {
   const float2* twc;
 };
 
-struct InvArgs {
-  Geo g;
-  Twiddles tw;
+// The temporal filter of one output.
+struct FilterArgs {
   const float2* s[4];  // window spectra in temporal order (__half2 pairs when half)
   int half;            // spectra stored as fp16 pairs (tensor-core filter only)
   int cur;             // index of the current frame in s
@@ -60,10 +59,16 @@ struct InvArgs {
   float2* klast;       // Kalman state, nb x bh x fbw
   float* kcov;
   float* kproc;
+  float sigma_x, sigma_y, beta_x, beta, ssmin, ssmax, kalman_cn, kr2;
+};
+
+// Filter and inverse of one output.
+struct InvArgs : FilterArgs {
+  Geo g;
+  Twiddles tw;
   const float* win_a;  // synthesis window of even-parity blocks (mode 0: analysis window)
   const float* win_b;  // synthesis window of odd-parity blocks
   float* blocks;       // out: nb x bh x bw windowed blocks
-  float sigma_x, sigma_y, beta_x, beta, ssmin, ssmax, kalman_cn, kr2;
   const float2* twr;   // blocks above 64: device twiddles, bw/2 and bh/2 entries,
   const float2* twc;   //   and nb x bh x bw complex work space
   float2* work;
@@ -101,7 +106,7 @@ struct SweepArgs {
   int* seam_cnt;         // [segs-1][strips]: CTAs of the seam that are done, 0 between launches
   const uint8_t* tab;    // tensor-core form: device copy of tc_tables()
   int* err;              // tensor-core form: bits set when a wait gives up (kErrWait*)
-  uint8_t* img;          // tensor-core form: filtered column-inverse operands, one tile per (row, strip)
+  uint8_t* img;          // tensor-core form: filtered column-inverse operands, one image per block
   int test_skip;         // tests only: the plane's first CTA skips its first operand-tile copy
 };
 
@@ -211,6 +216,19 @@ struct SweepBatch {
   int shifted;  // filter: bit i set when plane i's window is plane i-1's (same run) moved on by one frame
   SweepArgs p[kMaxBatch];
 };
+// Filter of the tensor-core form, with the runs of a SweepBatch.
+struct FilterPlane {
+  FilterArgs f;
+  uint8_t* img;
+  int nblk;  // blocks that the output reads: rows 0..cells_y of the block grid
+};
+struct FilterBatch {
+  int n;
+  int cta0[kMaxBatch + 1];
+  int run[kMaxBatch], rlen[kMaxBatch];
+  int shifted;
+  FilterPlane p[kMaxBatch];
+};
 // Launch shape of the tensor-core kernels, picked by the autotuner.
 struct TcTune {
   int fwd_ctas_per_sm = 3;  // persistent forward grid: CTAs per SM (1 to 3; 2 at most with the split)
@@ -234,8 +252,8 @@ cudaError_t launch_sweep_tc(const SweepArgs& a, cudaStream_t st, cudaEvent_t mar
 // The fast form's fused sweeps of n planes (8x8 to 32x32 blocks, one
 // temporal mode) in one launch; `mark` is recorded after it.
 cudaError_t launch_sweep_fast_batch(const SweepArgs* planes, int n, cudaStream_t st, cudaEvent_t mark);
-// Bytes of SweepArgs::img for this geometry and strip count.
-size_t tc_image_bytes(const Geo& g, int strips);
+// Bytes of SweepArgs::img for this geometry.
+size_t tc_image_bytes(const Geo& g);
 
 // SMs of the current device.
 int sm_count();

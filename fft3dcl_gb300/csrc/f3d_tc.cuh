@@ -12,9 +12,12 @@
 //  - SWIZZLE_128B: rows of 64 elements (128 bytes); 8-row atoms of 1024 bytes,
 //    the 16-byte chunk c of row r stored at chunk position c ^ (r % 8). Atoms
 //    are SBO = 1024 bytes apart and the tile base is 1024-byte aligned.
+//  - SWIZZLE_64B, SWIZZLE_32B: the same with rows of 64 or 32 bytes and atoms
+//    of 512 or 256 bytes (SBO): chunk c of row r at c ^ (r / 2 % 4), or at
+//    c ^ (r / 4 % 2).
 // Each MMA instruction consumes K = 16 elements: the descriptor start
-// advances by 2*LBO per step for INTERLEAVE and by 32 bytes inside the
-// 128-byte row for SWIZZLE_128B.
+// advances by 2*LBO per step for INTERLEAVE and by 32 bytes inside the row
+// for the swizzled layouts.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -97,7 +100,7 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[M]) {
 }
 
 // ---- MMA -----------------------------------------------------------------
-enum : uint32_t { LAYOUT_INTERLEAVE = 0, LAYOUT_SW128 = 2 };
+enum : uint32_t { LAYOUT_INTERLEAVE = 0, LAYOUT_SW128 = 2, LAYOUT_SW64 = 4, LAYOUT_SW32 = 6 };
 
 // Shared-memory matrix descriptor: start, leading and stride byte offsets
 // (16-byte units, 14 bits each), the fixed version field 0b001 at bit 46,
@@ -210,6 +213,14 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint3
 // Byte offset of element (row, k) in an INTERLEAVE K-major tile with K columns.
 __host__ __device__ constexpr uint32_t off_il(int row, int k, int K) {
   return static_cast<uint32_t>((row >> 3) * (K / 8) * 128 + (k >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2);
+}
+// Byte offset of element (row, k) in a SWIZZLE_64B (K = 32) or SWIZZLE_32B
+// (K = 16) K-major tile.
+template <int K>
+__host__ __device__ constexpr uint32_t off_sw_k(int row, int k) {
+  static_assert(K == 16 || K == 32, "row of 32 or 64 bytes");
+  const int sw = K == 32 ? (row >> 1) & 3 : (row >> 2) & 1;
+  return static_cast<uint32_t>(row * (2 * K) + (((k >> 3) ^ sw) << 4) + (k & 7) * 2);
 }
 // Byte offset of element (row, k) in a SWIZZLE_128B K-major tile (K = 64).
 __host__ __device__ constexpr uint32_t off_sw128(int row, int k) {
