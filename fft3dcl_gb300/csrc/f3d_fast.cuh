@@ -291,6 +291,68 @@ __device__ __forceinline__ void inverse_block_sq(const InvArgs& a, int b, int t,
   __syncwarp();
 }
 
+// ---- 64 x 64 blocks: each 64-point transform on a lane pair ------------------
+//
+// One thread per 64-point transform holds 128 registers of data, which leaves
+// 12 warps on an SM. As a pair (lanes 2p, 2p + 1), the even lane holds
+// positions 0..31 of the bit-reversed array and the odd lane 32..63; the
+// stages up to 32 stay inside a lane (f3d_k_exact.cu does the same), the last
+// one pairs position j with j + 32 through a shuffle. Every value comes from
+// the operations of fft_fast<64>.
+
+// Stages LEN..32 of one half of a 64-point transform.
+template <int LEN, bool INV>
+__device__ __forceinline__ void fast_half_stage64(float2 (&a)[32], const float2* tw) {
+  constexpr int half = LEN / 2, step = 64 / LEN;
+#pragma unroll
+  for (int i = 0; i < 32; i += LEN) {
+#pragma unroll
+    for (int j = 0; j < half; j++) {
+      const float2 b = a[i + j + half];
+      float2 t;
+      if (j == 0) {
+        t = b;
+      } else if (j * step == 16) {
+        t = INV ? make_float2(-b.y, b.x) : make_float2(b.y, -b.x);
+      } else {
+        const float2 w = tw[j * step];
+        const float wy = INV ? -w.y : w.y;
+        t.x = fmaf(w.x, b.x, -wy * b.y);
+        t.y = fmaf(w.x, b.y, wy * b.x);
+      }
+      const float2 u = a[i + j];
+      a[i + j] = make_float2(u.x + t.x, u.y + t.y);
+      a[i + j + half] = make_float2(u.x - t.x, u.y - t.y);
+    }
+  }
+  if constexpr (LEN < 32) fast_half_stage64<LEN * 2, INV>(a, tw);
+}
+
+__device__ __forceinline__ float2 shfl_pair(float2 v) {
+  return make_float2(__shfl_xor_sync(0xffffffffu, v.x, 1), __shfl_xor_sync(0xffffffffu, v.y, 1));
+}
+
+// Forward transform of 64 values on a lane pair: a holds positions
+// 32 * odd + q of the bit-reversed input, then values 32 * odd + q. Every lane
+// of the warp takes part.
+__device__ __forceinline__ void fft64_fast_pair(float2 (&a)[32], const float2* tw, bool odd) {
+  fast_half_stage64<2, false>(a, tw);
+#pragma unroll
+  for (int j = 0; j < 32; j++) {
+    const float2 b = a[j];
+    float2 t = b;
+    if (j == 16) {
+      t = make_float2(b.y, -b.x);
+    } else if (j > 0) {
+      const float2 w = tw[j];
+      t.x = fmaf(w.x, b.x, -w.y * b.y);
+      t.y = fmaf(w.x, b.y, w.y * b.x);
+    }
+    const float2 r = shfl_pair(odd ? t : b);
+    a[j] = odd ? make_float2(r.x - t.x, r.y - t.y) : make_float2(b.x + r.x, b.y + r.y);
+  }
+}
+
 // Bulk prefetch of `bytes` (a multiple of 16, 16-byte aligned) into L2.
 __device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");

@@ -22,10 +22,56 @@
 //             complex FFT whose real and imaginary parts are the two rows.
 #include "f3d_fast.cuh"
 
+#include <type_traits>
+
 namespace f3d {
 namespace {
 
 constexpr int kThreads = 128;
+
+// The samples of block b, converted and windowed, into tile[BH][TS], by TPB
+// threads.
+template <int BW, int BH, int TPB, int TS>
+__device__ __forceinline__ void gather_block(const FwdArgs& a, int b, int t, float* tile) {
+  int bx, by, par;
+  block_origin(a.g, b, bx, by, par);
+  const bool inside = bx >= 0 && by >= 0 && bx + BW <= a.g.W && by + BH <= a.g.H;
+  const int bps = a.fmt == FMT_U8 ? 1 : (a.fmt == FMT_U16 ? 2 : 4);
+  const uintptr_t row0 = reinterpret_cast<uintptr_t>(a.src) + (long long)by * a.pitch + (long long)bx * bps;
+  const bool vec = inside && ((row0 | (uintptr_t)a.pitch) & 15) == 0 && (BW * bps) % 16 == 0;
+  if (vec) {
+    // 16-byte loads: a row is BW*bps/16 chunks, the group covers them all.
+    const int cpr = BW * bps / 16, spc = 16 / bps;
+    for (int q = t; q < BH * cpr; q += TPB) {
+      const int ly = q / cpr, ch = q - ly * cpr;
+      const uint8_t* p = reinterpret_cast<const uint8_t*>(row0 + (long long)ly * a.pitch) + ch * 16;
+      const uint4 u = *reinterpret_cast<const uint4*>(p);
+      const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
+      float* dst = tile + ly * TS + ch * spc;
+      const float* win = a.win + ly * BW + ch * spc;
+      if (a.fmt == FMT_U8) {
+#pragma unroll
+        for (int k = 0; k < 16; k++)
+          dst[k] = ((float)((w4[k >> 2] >> (8 * (k & 3))) & 0xffu) * (1.0f / 255.0f) - a.chroma_norm) * win[k];
+      } else if (a.fmt == FMT_U16) {
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          dst[k] = ((float)((w4[k >> 1] >> (16 * (k & 1))) & 0xffffu) * a.norm - a.chroma_norm) * win[k];
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++) dst[k] = (__uint_as_float(w4[k]) - a.chroma_norm) * win[k];
+      }
+    }
+  } else {
+    for (int idx = t; idx < BW * BH; idx += TPB) {
+      const int ly = idx / BW, lx = idx - ly * BW;
+      const int y = inside ? by + ly : mirror_i(by + ly, a.g.H);
+      const int x = inside ? bx + lx : mirror_i(bx + lx, a.g.W);
+      tile[ly * TS + lx] =
+          (load_sample(a.src + (long long)y * a.pitch, x, a.fmt, a.norm) - a.chroma_norm) * a.win[idx];
+    }
+  }
+}
 
 template <int BW, int BH>
 __global__ void __launch_bounds__(128) k_forward_fast(const __grid_constant__ FwdArgs a) {
@@ -38,46 +84,7 @@ __global__ void __launch_bounds__(128) k_forward_fast(const __grid_constant__ Fw
   float2* S = reinterpret_cast<float2*>(smem4) + slot * C::SMEM_F2;
   float* tile = reinterpret_cast<float*>(S);  // input tile [BH][TS], aliased with S
 
-  if (valid) {
-    int bx, by, par;
-    block_origin(a.g, b, bx, by, par);
-    const bool inside = bx >= 0 && by >= 0 && bx + BW <= a.g.W && by + BH <= a.g.H;
-    const int bps = a.fmt == FMT_U8 ? 1 : (a.fmt == FMT_U16 ? 2 : 4);
-    const uintptr_t row0 = reinterpret_cast<uintptr_t>(a.src) + (long long)by * a.pitch + (long long)bx * bps;
-    const bool vec = inside && ((row0 | (uintptr_t)a.pitch) & 15) == 0 && (BW * bps) % 16 == 0;
-    if (vec) {
-      // 16-byte loads: a row is BW*bps/16 chunks, the group covers them all.
-      const int cpr = BW * bps / 16, spc = 16 / bps;
-      for (int q = t; q < BH * cpr; q += C::TPB) {
-        const int ly = q / cpr, ch = q - ly * cpr;
-        const uint8_t* p = reinterpret_cast<const uint8_t*>(row0 + (long long)ly * a.pitch) + ch * 16;
-        const uint4 u = *reinterpret_cast<const uint4*>(p);
-        const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
-        float* dst = tile + ly * C::TS + ch * spc;
-        const float* win = a.win + ly * BW + ch * spc;
-        if (a.fmt == FMT_U8) {
-#pragma unroll
-          for (int k = 0; k < 16; k++)
-            dst[k] = ((float)((w4[k >> 2] >> (8 * (k & 3))) & 0xffu) * (1.0f / 255.0f) - a.chroma_norm) * win[k];
-        } else if (a.fmt == FMT_U16) {
-#pragma unroll
-          for (int k = 0; k < 8; k++)
-            dst[k] = ((float)((w4[k >> 1] >> (16 * (k & 1))) & 0xffffu) * a.norm - a.chroma_norm) * win[k];
-        } else {
-#pragma unroll
-          for (int k = 0; k < 4; k++) dst[k] = (__uint_as_float(w4[k]) - a.chroma_norm) * win[k];
-        }
-      }
-    } else {
-      for (int idx = t; idx < BW * BH; idx += C::TPB) {
-        const int ly = idx / BW, lx = idx - ly * BW;
-        const int y = inside ? by + ly : mirror_i(by + ly, a.g.H);
-        const int x = inside ? bx + lx : mirror_i(bx + lx, a.g.W);
-        tile[ly * C::TS + lx] =
-            (load_sample(a.src + (long long)y * a.pitch, x, a.fmt, a.norm) - a.chroma_norm) * a.win[idx];
-      }
-    }
-  }
+  if (valid) gather_block<BW, BH, C::TPB, C::TS>(a, b, t, tile);
   __syncwarp();
   float2 z[BW];
   const bool rows = valid && t < BH / 2;
@@ -156,38 +163,272 @@ __global__ void __launch_bounds__(128) k_inverse_fast(const __grid_constant__ In
   }, [] {});
 }
 
-template <int BW, int BH>
-cudaError_t launch_fwd(const FwdArgs& a, cudaStream_t st) {
-  using C = FCfg<BW, BH>;
-  constexpr int BPC = kThreads / C::TPB;
-  const size_t smem = sizeof(float2) * C::SMEM_F2 * BPC;
-  auto k = k_forward_fast<BW, BH>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+// ---- 64 x 64 blocks -----------------------------------------------------------
+//
+// One block per CTA of 64 threads, each 64-point transform on a lane pair:
+// half the registers a thread and 24 warps on an SM instead of 12. The
+// inverse's windowed rows go back to shared memory and leave in plane order;
+// from the row transforms each thread would walk its own row, a line per
+// lane and request. 1080p 8-bit bt=3 (2,232 blocks for 1,824 CTA slots: the
+// latency of one block counts twice): forward 73 -> 50 us, inverse 79 -> 67.
+constexpr int kPairThreads = 64, kPairCtas = 12;
+
+// gather_block for 64 x 64 blocks whose rows are aligned: four samples per
+// thread and load, so that samples and window are read in whole lines (with
+// 16 bytes of 8-bit samples per thread each window read touched 24 sectors).
+template <int FMT, int TS>
+__device__ __forceinline__ void gather_quads64(const FwdArgs& a, uintptr_t row0, int t, float* tile) {
+  constexpr int BPS = FMT == FMT_U8 ? 1 : (FMT == FMT_U16 ? 2 : 4);
+  using Raw = typename std::conditional<BPS == 1, uint32_t, typename std::conditional<BPS == 2, uint2, uint4>::type>::type;
+  constexpr int NB = 8;  // loads in flight
+  const int lx = (t & 15) * 4, ly0 = t >> 4;
+  const float4* win = reinterpret_cast<const float4*>(a.win) + t;
+#pragma unroll 1
+  for (int i0 = 0; i0 < 16; i0 += NB) {
+    Raw raw[NB];
+    float4 w[NB];
+#pragma unroll
+    for (int i = 0; i < NB; i++) {
+      raw[i] = *reinterpret_cast<const Raw*>(row0 + (long long)(ly0 + 4 * (i0 + i)) * a.pitch + lx * BPS);
+      w[i] = win[(i0 + i) * kPairThreads];
+    }
+#pragma unroll
+    for (int i = 0; i < NB; i++) {
+      float* dst = tile + (ly0 + 4 * (i0 + i)) * TS + lx;
+      const float wk[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        if constexpr (FMT == FMT_U8) {
+          dst[k] = ((float)((raw[i] >> (8 * k)) & 0xffu) * (1.0f / 255.0f) - a.chroma_norm) * wk[k];
+        } else if constexpr (FMT == FMT_U16) {
+          const uint32_t v = k < 2 ? raw[i].x : raw[i].y;
+          dst[k] = ((float)((v >> (16 * (k & 1))) & 0xffffu) * a.norm - a.chroma_norm) * wk[k];
+        } else {
+          const uint32_t v = k == 0 ? raw[i].x : (k == 1 ? raw[i].y : (k == 2 ? raw[i].z : raw[i].w));
+          dst[k] = (__uint_as_float(v) - a.chroma_norm) * wk[k];
+        }
+      }
+    }
   }
-  const int grid = (a.g.nb + BPC - 1) / BPC;
-  if (grid == 0) return cudaSuccess;
-  k<<<grid, kThreads, smem, st>>>(a);
+}
+
+__global__ void __launch_bounds__(kPairThreads, kPairCtas) k_forward_fast64(const __grid_constant__ FwdArgs a) {
+  using C = FCfg<64, 64>;
+  constexpr int SB = C::SB, FBW = C::FBW, NY = C::NY;
+  extern __shared__ float4 smem4[];
+  float2* S = reinterpret_cast<float2*>(smem4);
+  float* tile = reinterpret_cast<float*>(S);  // input tile [64][TS], aliased with S
+  const int t = threadIdx.x, p = t >> 1, b = blockIdx.x;
+  const bool odd = t & 1;
+  {
+    int bx, by, par;
+    block_origin(a.g, b, bx, by, par);
+    const int bps = a.fmt == FMT_U8 ? 1 : (a.fmt == FMT_U16 ? 2 : 4);
+    const uintptr_t row0 = reinterpret_cast<uintptr_t>(a.src) + (long long)by * a.pitch + (long long)bx * bps;
+    const bool quads = bx >= 0 && by >= 0 && bx + 64 <= a.g.W && by + 64 <= a.g.H &&
+                       ((row0 | (uintptr_t)a.pitch) & 15) == 0;
+    if (!quads) gather_block<64, 64, kPairThreads, C::TS>(a, b, t, tile);
+    else if (a.fmt == FMT_U8) gather_quads64<FMT_U8, C::TS>(a, row0, t, tile);
+    else if (a.fmt == FMT_U16) gather_quads64<FMT_U16, C::TS>(a, row0, t, tile);
+    else gather_quads64<FMT_F32, C::TS>(a, row0, t, tile);
+  }
+  __syncthreads();
+  float2 z[32];
+  // Rows 2p and 2p + 1 as one complex transform.
+#pragma unroll
+  for (int q = 0; q < 32; q++) {
+    const int c = bit_reverse(q, 6) + odd;
+    z[q] = make_float2(tile[(2 * p) * C::TS + c], tile[(2 * p + 1) * C::TS + c]);
+  }
+  __syncthreads();  // the tile is dead from here on; S reuses its storage
+  fft64_fast_pair(z, a.tw.row, odd);
+  // Split Z = X_2p + i X_2p+1 (k_forward_fast): columns 0..16 on the even
+  // lane, 32..17 on the odd one. Z[64 - k] of the even lane's k is the odd
+  // lane's entry 32 - k, and the other way round.
+  tile_pair<SB>(S, odd ? NY : 0, 2 * p) =
+      make_float4(0.5f * (z[0].x + z[0].x), 0.5f * (z[0].y - z[0].y), 0.5f * (z[0].y + z[0].y), 0.5f * (z[0].x - z[0].x));
+#pragma unroll
+  for (int i = 1; i <= 16; i++) {
+    const float2 r = shfl_pair(z[32 - i]);
+    const float2 A = odd ? r : z[i], B = odd ? z[i] : r;
+    if (i < 16 || !odd)
+      tile_pair<SB>(S, odd ? NY - i : i, 2 * p) =
+          make_float4(0.5f * (A.x + B.x), 0.5f * (A.y - B.y), 0.5f * (A.y + B.y), 0.5f * (B.x - A.x));
+  }
+  __syncthreads();
+  // Column p; pair 0: columns 0 and 32, which are real, together.
+#pragma unroll
+  for (int q = 0; q < 32; q++) {
+    const int r = bit_reverse(q, 6) + odd;
+    z[q] = p ? S[p * SB + r] : make_float2(S[r].x, S[NY * SB + r].x);
+  }
+  fft64_fast_pair(z, a.tw.col, odd);
+  float2* out = a.spec + (size_t)b * C::PS + (odd ? 32 * FBW : 0);
+  if (t < 32) {  // the warp of pair 0
+#pragma unroll
+    for (int i = 0; i < 32; i++) {
+      const float2 A = z[i], B = i ? shfl_pair(z[32 - i]) : z[0];
+      if (p == 0) {
+        out[i * FBW] = make_float2(0.5f * (A.x + B.x), 0.5f * (A.y - B.y));
+        out[i * FBW + NY] = make_float2(0.5f * (A.y + B.y), 0.5f * (B.x - A.x));
+      }
+    }
+  }
+  if (p) {
+#pragma unroll
+    for (int i = 0; i < 32; i++) out[i * FBW + p] = z[i];
+  }
+}
+
+// inverse_block (f3d_fast.cuh) with 64 threads: thread (c, h) = (t / 2, t % 2)
+// filters rows 32 h .. 32 h + 31 of column c and row t of column 32, then
+// inverts column c's even (h = 0) or odd inputs, combined through a shuffle
+// (as inverse_block_sq), then the row at tile position t.
+template <int BM>
+__global__ void __launch_bounds__(kPairThreads, kPairCtas) k_inverse_fast64(const __grid_constant__ InvArgs a) {
+  using C = FCfg<64, 64>;
+  constexpr int SB = C::SB, FBW = C::FBW, NY = C::NY, H = 32;
+  extern __shared__ float4 smem4[];
+  float2* S = reinterpret_cast<float2*>(smem4);
+  const int t = threadIdx.x, c = t >> 1, h = t & 1, b = blockIdx.x;
+  const size_t base = (size_t)b * C::PS;
+  {
+    constexpr int NF = BM >= 2 ? BM : 1;
+    if (t < NF) prefetch_l2(a.s[t] + base, C::PS * sizeof(float2));
+    const float dc = block_dc(a, b);
+    // Four bins' spectra and tables are loaded together.
+#pragma unroll 1
+    for (int k = 0; k < H; k += 4) {
+      const int r = h * H + k;
+      float2 sv[4][4], f[4];
+      BinTables tb[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        load_window<BM>(a, base + (r + u) * FBW + c, sv[u]);
+        tb[u] = bin_tables(a, (r + u) * FBW + c);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) f[u] = filter_vals_t<BM, true>(a, dc, tb[u], 0, sv[u]);
+      tile_pair<SB>(S, c, r) = make_float4(f[0].x, f[0].y, f[1].x, f[1].y);
+      tile_pair<SB>(S, c, r + 2) = make_float4(f[2].x, f[2].y, f[3].x, f[3].y);
+    }
+    S[NY * SB + t] = filter_bin_t<BM, true>(a, dc, t * FBW + NY, base + t * FBW + NY);
+  }
+  __syncthreads();
+  if (t <= 32) {  // Hermitian parts of columns 0 and 32, packed into column 0
+    const int r = t, m = (64 - t) % 64;
+    const float2 zr = S[r], zm = S[m];
+    const float2 nr = S[NY * SB + r], nm = S[NY * SB + m];
+    const float ar = 0.5f * (zr.x + zm.x), ai = 0.5f * (zr.y - zm.y);
+    const float qr = 0.5f * (nr.x + nm.x), qi = 0.5f * (nr.y - nm.y);
+    S[r] = make_float2(ar - qi, ai + qr);
+    if (m != r) S[m] = make_float2(ar + qi, qr - ai);
+  }
+  __syncthreads();
+  float2 e[H];
+#pragma unroll
+  for (int j = 0; j < H; j++) e[j] = S[c * SB + 2 * j + h];
+  fft_fast<H, true, 2>(e, a.tw.col);
+  __syncwarp();  // the pair has read its column
+#pragma unroll
+  for (int y = 0; y < H; y++) {
+    const float2 w = a.tw.col[y];
+    // e^{+2 pi i y/64} O[y] on h = 1
+    const float2 o = make_float2(fmaf(e[y].x, w.x, e[y].y * w.y), fmaf(e[y].y, w.x, -e[y].x * w.y));
+    const float2 v = h ? o : e[y], q = shfl_pair(v);
+    // h = 0: x[y] = E + P at slot 2y; h = 1: x[y + 32] = E - P at slot 2y + 1
+    const float2 x = h ? make_float2(q.x - v.x, q.y - v.y) : make_float2(v.x + q.x, v.y + q.y);
+    if (c == 0) {  // real inverses of columns 0 and 32
+      S[2 * y + h] = make_float2(x.x, 0.0f);
+      S[NY * SB + 2 * y + h] = make_float2(x.y, 0.0f);
+    } else {
+      S[c * SB + 2 * y + h] = x;
+    }
+  }
+  __syncthreads();
+  {
+#pragma unroll
+    for (int k = 0; k < H; k++) {
+      const float2 yk = S[k * SB + t], ym = S[(H - k) * SB + t];
+      const float ax = yk.x + ym.x, ay = yk.y - ym.y;
+      const float bx = yk.x - ym.x, by = yk.y + ym.y;
+      const float2 w = a.tw.row[k];  // e^{-2 pi i k/64}; the conjugate is used
+      const float px = fmaf(bx, w.x, by * w.y), py = fmaf(by, w.x, -bx * w.y);
+      e[k] = make_float2(ax - py, ay + px);
+    }
+    fft_fast<H, true, 2>(e, a.tw.row);
+    // Only this thread reads or writes the entries at tile position t.
+#pragma unroll
+    for (int k = 0; k < H; k++) S[k * SB + t] = e[k];
+  }
+  __syncthreads();
+  int bx, by, par;
+  block_origin(a.g, b, bx, by, par);
+  const float2* win = reinterpret_cast<const float2*>(par ? a.win_b : a.win_a);
+  float2* out = reinterpret_cast<float2*>(a.blocks + (size_t)b * 64 * 64);
+  constexpr float inv_n = 1.0f / (64 * 64);
+#pragma unroll 8
+  for (int i = t; i < 64 * H; i += kPairThreads) {
+    const float2 v = S[(i % H) * SB + yperm<64>(i / H)], w = win[i];
+    out[i] = make_float2(v.x * inv_n * w.x, v.y * inv_n * w.y);
+  }
+}
+
+cudaError_t launch_fwd64(const FwdArgs& a, cudaStream_t st) {
+  if (a.g.nb == 0) return cudaSuccess;
+  k_forward_fast64<<<a.g.nb, kPairThreads, sizeof(float2) * FCfg<64, 64>::SMEM_F2, st>>>(a);
   count_launch();
   return cudaGetLastError();
 }
 
-template <int BW, int BH, int BM>
-cudaError_t launch_inv_bm(const InvArgs& a, cudaStream_t st) {
-  using C = FCfg<BW, BH>;
-  constexpr int BPC = kThreads / C::TPB;
-  const size_t smem = sizeof(float2) * C::SMEM_F2 * BPC;
-  auto k = k_inverse_fast<BW, BH, BM>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  const int grid = (a.g.nb + BPC - 1) / BPC;
-  if (grid == 0) return cudaSuccess;
-  k<<<grid, kThreads, smem, st>>>(a);
+template <int BM>
+cudaError_t launch_inv64(const InvArgs& a, cudaStream_t st) {
+  if (a.g.nb == 0) return cudaSuccess;
+  k_inverse_fast64<BM><<<a.g.nb, kPairThreads, sizeof(float2) * FCfg<64, 64>::SMEM_F2, st>>>(a);
   count_launch();
   return cudaGetLastError();
+}
+
+template <int BW, int BH>
+cudaError_t launch_fwd(const FwdArgs& a, cudaStream_t st) {
+  if constexpr (BW == 64 && BH == 64) {
+    return launch_fwd64(a, st);
+  } else {
+    using C = FCfg<BW, BH>;
+    constexpr int BPC = kThreads / C::TPB;
+    const size_t smem = sizeof(float2) * C::SMEM_F2 * BPC;
+    auto k = k_forward_fast<BW, BH>;
+    if (smem > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+    }
+    const int grid = (a.g.nb + BPC - 1) / BPC;
+    if (grid == 0) return cudaSuccess;
+    k<<<grid, kThreads, smem, st>>>(a);
+    count_launch();
+    return cudaGetLastError();
+  }
+}
+
+template <int BW, int BH, int BM>
+cudaError_t launch_inv_bm(const InvArgs& a, cudaStream_t st) {
+  if constexpr (BW == 64 && BH == 64) {
+    return launch_inv64<BM>(a, st);
+  } else {
+    using C = FCfg<BW, BH>;
+    constexpr int BPC = kThreads / C::TPB;
+    const size_t smem = sizeof(float2) * C::SMEM_F2 * BPC;
+    auto k = k_inverse_fast<BW, BH, BM>;
+    if (smem > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+    }
+    const int grid = (a.g.nb + BPC - 1) / BPC;
+    if (grid == 0) return cudaSuccess;
+    k<<<grid, kThreads, smem, st>>>(a);
+    count_launch();
+    return cudaGetLastError();
+  }
 }
 
 template <int BW, int BH>
