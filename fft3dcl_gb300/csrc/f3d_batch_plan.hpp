@@ -78,6 +78,14 @@ inline bool sweep_batches(const SweepArgs* planes, int n, SweepBatch& Bf, SweepB
   return true;
 }
 
+// The switches all planes of a batch share (kSwAny where they differ).
+inline int filter_switches(const SweepBatch& S) {
+  int sw = filter_switches(S.p[0].inv);
+  for (int i = 1; i < S.n; i++)
+    if (filter_switches(S.p[i].inv) != sw) sw = kSwAny;
+  return sw;
+}
+
 // Segments of each plane's strips (written to its segs, at most what it comes
 // with) for one launch of all planes' sweeps, `slots` CTAs of which run at a
 // time. A CTA costs its block rows plus about one and a half for its set-up

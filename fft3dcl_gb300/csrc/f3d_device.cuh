@@ -181,6 +181,20 @@ __device__ __forceinline__ BinTables bin_tables(const FilterArgs& a, int i) {
   return t;
 }
 
+// Fixes a kernel's copy of the filter arguments to the switches it is built
+// for. Read at run time they cost about ten instructions of branches per bin,
+// and table loads behind a branch cannot be issued with the spectra's.
+// Products that are added later are rounded by themselves (prod), so the bits
+// are the same.
+template <int SW>
+__device__ __forceinline__ void fix_switches(FilterArgs& f) {
+  if constexpr (SW != kSwAny) {
+    f.dg = 1;
+    f.pat = 0;
+    f.shp = SW == kSwSharpen;
+  }
+}
+
 // Kalman state of one bin as read before its update (a.kalman_init: unused).
 struct KState {
   float2 last;

@@ -214,23 +214,34 @@ __device__ __forceinline__ void inverse_block(const InvArgs& a, int b, int t, bo
 //            first (thread r <= N/2 does rows r and -r);
 //   rows     thread t inverts row t as an N/2-point complex FFT.
 // Tile positions, emit and filtered() are those of inverse_block.
-template <int N, int BM, class Emit, class Filtered>
-__device__ __forceinline__ void inverse_block_sq(const InvArgs& a, int b, int t, bool valid, float2* S,
-                                                 Emit&& emit, Filtered&& filtered) {
+// fa: the filter arguments of a (fix_switches). The spectra and tables of U
+// bins are loaded together.
+template <int N, int BM, int U, class Emit, class Filtered>
+__device__ __forceinline__ void inverse_block_sq(const InvArgs& a, const FilterArgs& fa, int b, int t, bool valid,
+                                                 float2* S, Emit&& emit, Filtered&& filtered) {
   using C = FCfg<N, N>;
   constexpr int NY = N / 2, H = N / 2, SB = C::SB, FBW = C::FBW;
   const size_t base = (size_t)b * C::PS;
   const int c = t % NY, h = t / NY;
   if (valid) {
-    const float dc = block_dc(a, b);
-    F3D_UNROLL(F3D_FILTER_UNROLL)
-    for (int k = 0; k < H; k += 2) {
+    const float dc = fa.dg ? block_dc(a, b) : 0.0f;
+#pragma unroll 1
+    for (int k = 0; k < H; k += U) {
       const int r = h * H + k;
-      const float2 f0 = filter_bin_t<BM, true>(a, dc, r * FBW + c, base + r * FBW + c);
-      const float2 f1 = filter_bin_t<BM, true>(a, dc, (r + 1) * FBW + c, base + (r + 1) * FBW + c);
-      tile_pair<SB>(S, c, r) = make_float4(f0.x, f0.y, f1.x, f1.y);
+      float2 sv[U][4], f[U];
+      BinTables tb[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        load_window<BM>(fa, base + (r + u) * FBW + c, sv[u]);
+        tb[u] = bin_tables(fa, (r + u) * FBW + c);
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) f[u] = filter_vals_t<BM, true>(fa, dc, tb[u], 0, sv[u]);
+#pragma unroll
+      for (int u = 0; u < U; u += 2)
+        tile_pair<SB>(S, c, r + u) = make_float4(f[u].x, f[u].y, f[u + 1].x, f[u + 1].y);
     }
-    S[NY * SB + t] = filter_bin_t<BM, true>(a, dc, t * FBW + NY, base + t * FBW + NY);
+    S[NY * SB + t] = filter_bin_t<BM, true>(fa, dc, t * FBW + NY, base + t * FBW + NY);
   }
   filtered();
   __syncwarp();
@@ -291,57 +302,57 @@ __device__ __forceinline__ void inverse_block_sq(const InvArgs& a, int b, int t,
   __syncwarp();
 }
 
-// ---- 64 x 64 blocks: each 64-point transform on a lane pair ------------------
+// ---- N-point transforms on a lane pair -----------------------------------------
 //
-// One thread per 64-point transform holds 128 registers of data, which leaves
-// 12 warps on an SM. As a pair (lanes 2p, 2p + 1), the even lane holds
-// positions 0..31 of the bit-reversed array and the odd lane 32..63; the
-// stages up to 32 stay inside a lane (f3d_k_exact.cu does the same), the last
-// one pairs position j with j + 32 through a shuffle. Every value comes from
-// the operations of fft_fast<64>.
+// One thread per transform of the forward (two real rows or one column) holds
+// 2 N registers of data and leaves few warps (64 x 64 blocks: 12 on an SM). As
+// a pair (lanes 2p, 2p + 1), the even lane holds positions 0..N/2-1 of the
+// bit-reversed array and the odd lane the others; the stages up to N/2 stay
+// inside a lane, the last one pairs position j with j + N/2 through a shuffle.
+// Every value comes from the operations of fft_fast<N>.
 
-// Stages LEN..32 of one half of a 64-point transform.
-template <int LEN, bool INV>
-__device__ __forceinline__ void fast_half_stage64(float2 (&a)[32], const float2* tw) {
-  constexpr int half = LEN / 2, step = 64 / LEN;
+// Stages LEN..N/2 of one half of an N-point transform.
+template <int N, int LEN>
+__device__ __forceinline__ void fast_half_stage(float2 (&a)[N / 2], const float2* tw) {
+  constexpr int half = LEN / 2, step = N / LEN;
 #pragma unroll
-  for (int i = 0; i < 32; i += LEN) {
+  for (int i = 0; i < N / 2; i += LEN) {
 #pragma unroll
     for (int j = 0; j < half; j++) {
       const float2 b = a[i + j + half];
       float2 t;
       if (j == 0) {
         t = b;
-      } else if (j * step == 16) {
-        t = INV ? make_float2(-b.y, b.x) : make_float2(b.y, -b.x);
+      } else if (j * step == N / 4) {
+        t = make_float2(b.y, -b.x);
       } else {
         const float2 w = tw[j * step];
-        const float wy = INV ? -w.y : w.y;
-        t.x = fmaf(w.x, b.x, -wy * b.y);
-        t.y = fmaf(w.x, b.y, wy * b.x);
+        t.x = fmaf(w.x, b.x, -w.y * b.y);
+        t.y = fmaf(w.x, b.y, w.y * b.x);
       }
       const float2 u = a[i + j];
       a[i + j] = make_float2(u.x + t.x, u.y + t.y);
       a[i + j + half] = make_float2(u.x - t.x, u.y - t.y);
     }
   }
-  if constexpr (LEN < 32) fast_half_stage64<LEN * 2, INV>(a, tw);
+  if constexpr (LEN < N / 2) fast_half_stage<N, LEN * 2>(a, tw);
 }
 
 __device__ __forceinline__ float2 shfl_pair(float2 v) {
   return make_float2(__shfl_xor_sync(0xffffffffu, v.x, 1), __shfl_xor_sync(0xffffffffu, v.y, 1));
 }
 
-// Forward transform of 64 values on a lane pair: a holds positions
-// 32 * odd + q of the bit-reversed input, then values 32 * odd + q. Every lane
-// of the warp takes part.
-__device__ __forceinline__ void fft64_fast_pair(float2 (&a)[32], const float2* tw, bool odd) {
-  fast_half_stage64<2, false>(a, tw);
+// Forward transform of N values on a lane pair: a holds positions N/2 * odd +
+// q of the bit-reversed input, then values N/2 * odd + q. Every lane of the
+// warp takes part.
+template <int N>
+__device__ __forceinline__ void fft_fast_pair(float2 (&a)[N / 2], const float2* tw, bool odd) {
+  fast_half_stage<N, 2>(a, tw);
 #pragma unroll
-  for (int j = 0; j < 32; j++) {
+  for (int j = 0; j < N / 2; j++) {
     const float2 b = a[j];
     float2 t = b;
-    if (j == 16) {
+    if (j == N / 4) {
       t = make_float2(b.y, -b.x);
     } else if (j > 0) {
       const float2 w = tw[j];

@@ -25,6 +25,12 @@
 // spectra can be bulk-prefetched into L2 while row m is processed (off by
 // default: with one wave of CTAs each holding a row, the prefetched rows
 // exceed what L2 keeps and the extra traffic costs more than it hides).
+//
+// The kernel is bound by the latency of its loads at 24 warps per SM: the
+// spectra and tables of four bins are loaded together, which needs the
+// filter's switches at compile time (fix_switches), and the synthesis window
+// is read in plane order. 10-bit bt=4 with sharpen: 84 -> 57 us at 1080p, 255
+// -> 179 us at 4K (half the loads of a block were window reads of 32 lines).
 #include "f3d_batch_plan.hpp"
 #include "f3d_fast.cuh"
 
@@ -54,13 +60,20 @@ struct SCfg {
   static constexpr size_t SMEM = sizeof(float2) * C::SMEM_F2 * SLOTS + sizeof(float) * TJ * CH * CW;
 };
 
-// Samples x..x+3 (x even) of row y of a block's windowed inverse, stored in
-// its tile as pairs: (x, x+1) at Q[(x/2)*SB + yperm(y)].
+// Samples x..x+3 (x even) of row y of a block's inverse, stored in its tile
+// as pairs: (x, x+1) at Q[(x/2)*SB + yperm(y)].
 template <int SB, int BH>
 __device__ __forceinline__ float4 qload(const float2* Q, int y, int x) {
   const int yp = yperm<BH>(y);
   const float2 lo = Q[(x / 2) * SB + yp], hi = Q[(x / 2 + 1) * SB + yp];
   return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+
+// The same times the block's synthesis window, rounded before it is added up.
+template <int SB, int BW, int BH>
+__device__ __forceinline__ float4 qwin(const float2* Q, const float* win, int y, int x) {
+  const float4 q = qload<SB, BH>(Q, y, x), w = *reinterpret_cast<const float4*>(win + y * BW + x);
+  return make_float4(__fmul_rn(q.x, w.x), __fmul_rn(q.y, w.y), __fmul_rn(q.z, w.z), __fmul_rn(q.w, w.w));
 }
 
 __device__ __forceinline__ float4 add4(float4 a, float4 b) {
@@ -78,13 +91,15 @@ __device__ __forceinline__ void store4(const SweepArgs& sa, int y, int x, float4
 }
 
 // CTA `cta` (strip, segment) of plane sa's sweep.
-template <int BW, int BH, int BM>
+template <int BW, int BH, int BM, int SW>
 __device__ __forceinline__ void sweep_fast_cta(const SweepArgs& sa, int cta) {
   using S_ = SCfg<BW, BH>;
   using C = FCfg<BW, BH>;
   constexpr int TPB = S_::TPB, TJ = S_::TJ, CW = S_::CW, CH = S_::CH, QK = S_::QK;
   constexpr int NWIN = BM >= 2 ? BM : 1;
   const InvArgs& a = sa.inv;
+  FilterArgs fa = a;
+  fix_switches<SW>(fa);
   extern __shared__ float4 smem4[];
   float2* slots = reinterpret_cast<float2*>(smem4);
   float4* P = reinterpret_cast<float4*>(slots + S_::SLOTS * C::SMEM_F2);  // [TJ][CH][QK]
@@ -110,15 +125,14 @@ __device__ __forceinline__ void sweep_fast_cta(const SweepArgs& sa, int cta) {
     const int b = m * a.g.ncols + n;
     const bool pf_next = t == 0 && col_ok && m + 1 < M1;
     if (sa.prefetch == 1 && pf_next) prefetch_block(b + a.g.ncols);
-    // Windowed rows go back into the tile as sample pairs: (x, x+1) of row y
-    // at S[(x/2)*SB + yperm(y)] (see inverse_block).
-    const float* win = (n & 1) ? a.win_b : a.win_a;
-    inverse_block_sq<BW, BM>(a, b, t, col_ok, S, [&](int y, const float2(&xy)[BW / 2]) {
+    // Rows go back into the tile as sample pairs: (x, x+1) of row y at
+    // S[(x/2)*SB + yperm(y)] (see inverse_block). The synthesis window is
+    // applied below, where neighbouring lanes read neighbouring samples of it:
+    // here each lane would read its own row, 32 lines per request.
+    inverse_block_sq<BW, BM, SW == kSwAny ? 2 : 4>(a, fa, b, t, col_ok, S, [&](int y, const float2(&xy)[BW / 2]) {
 #pragma unroll
-      for (int k = 0; k < BW / 2; k++) {
-        const float2 wv = *reinterpret_cast<const float2*>(win + y * BW + 2 * k);
-        S[k * C::SB + yperm<BH>(y)] = make_float2(xy[k].x * inv_n * wv.x, xy[k].y * inv_n * wv.y);
-      }
+      for (int k = 0; k < BW / 2; k++)
+        S[k * C::SB + yperm<BH>(y)] = make_float2(xy[k].x * inv_n, xy[k].y * inv_n);
     }, [&] {
       // Row m's spectra are read by now: fetch row m+1 while the transforms
       // and the cell sums of row m run.
@@ -135,8 +149,10 @@ __device__ __forceinline__ void sweep_fast_cta(const SweepArgs& sa, int cta) {
       if (jj >= ncell) continue;
       const float2* Qa = slots + jj * C::SMEM_F2;
       const float2* Qb = slots + (jj + 1) * C::SMEM_F2;
-      const float4 q10 = qload<C::SB, BH>(Qa, yy, CW + 4 * k);  // block (m, j) top right
-      const float4 q11 = qload<C::SB, BH>(Qb, yy, 4 * k);       // block (m, j+1) top left
+      const float* wa = ((J0 + jj) & 1) ? a.win_b : a.win_a;     // windows of blocks (m, j), (m, j+1)
+      const float* wb = ((J0 + jj) & 1) ? a.win_a : a.win_b;
+      const float4 q10 = qwin<C::SB, BW, BH>(Qa, wa, yy, CW + 4 * k);  // block (m, j) top right
+      const float4 q11 = qwin<C::SB, BW, BH>(Qb, wb, yy, 4 * k);       // block (m, j+1) top left
       float4& p = P[(jj * CH + yy) * QK + k];
       const int x = (J0 + jj) * CW + 4 * k;
       if (emit) {
@@ -147,7 +163,8 @@ __device__ __forceinline__ void sweep_fast_cta(const SweepArgs& sa, int cta) {
         *reinterpret_cast<float4*>(t0) = q10;
         *reinterpret_cast<float4*>(t1) = q11;
       }
-      p = add4(qload<C::SB, BH>(Qa, CH + yy, CW + 4 * k), qload<C::SB, BH>(Qb, CH + yy, 4 * k));  // row m bottom halves
+      p = add4(qwin<C::SB, BW, BH>(Qa, wa, CH + yy, CW + 4 * k),
+               qwin<C::SB, BW, BH>(Qb, wb, CH + yy, 4 * k));  // row m bottom halves
       if (seam_bot) *reinterpret_cast<float4*>(sa.seam_b + ((size_t)seg * CH + yy) * sa.seam_w + x) = p;
     }
     __syncthreads();
@@ -156,71 +173,48 @@ __device__ __forceinline__ void sweep_fast_cta(const SweepArgs& sa, int cta) {
   finish_seams<CH, CW>(sa, strip, seg, J0, ncell, reinterpret_cast<int*>(slots));
 }
 
-template <int BW, int BH, int BM>
-__global__ void __launch_bounds__(kSweepThreads, F3D_SWEEP_MINB) k_sweep_fast(const __grid_constant__ SweepArgs sa) {
-  sweep_fast_cta<BW, BH, BM>(sa, blockIdx.x);
-}
-
 // The sweeps of a batch of planes in one launch: the CTAs of a run of
 // planes of one geometry (consecutive outputs of a plane) are interleaved,
 // so that the window spectra they share are read from L2 the second time.
-template <int BW, int BH, int BM>
-__global__ void __launch_bounds__(kSweepThreads, F3D_SWEEP_MINB)
-    k_sweep_fast_batch(const __grid_constant__ SweepBatch B) {
+template <int BW, int BH, int BM, int SW>
+__global__ void __launch_bounds__(kSweepThreads, F3D_SWEEP_MINB) k_sweep_fast(const __grid_constant__ SweepBatch B) {
   int p = 0;
   while (p + 1 < B.n && (int)blockIdx.x >= B.cta0[p + 1]) p++;
   const int r0 = B.run[p], rl = B.rlen[r0];
   const int local = (int)blockIdx.x - B.cta0[r0];
-  sweep_fast_cta<BW, BH, BM>(B.p[r0 + local % rl], local / rl);
+  sweep_fast_cta<BW, BH, BM, SW>(B.p[r0 + local % rl], local / rl);
 }
 
-template <int BW, int BH, int BM>
-cudaError_t launch_bm(const SweepArgs& a, cudaStream_t st, cudaEvent_t mark) {
+template <int BW, int BH, int BM, int SW>
+cudaError_t launch_sw(const SweepBatch& Bs, cudaStream_t st) {
   using S_ = SCfg<BW, BH>;
-  auto k = k_sweep_fast<BW, BH, BM>;
   static_assert(S_::SMEM * F3D_SWEEP_MINB <= 227 * 1024, "CTAs per SM");
+  auto k = k_sweep_fast<BW, BH, BM, SW>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S_::SMEM);
   if (e != cudaSuccess) return e;
-  k<<<a.strips * a.segs, kSweepThreads, S_::SMEM, st>>>(a);
-  count_launch();
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  if (mark) cudaEventRecord(mark, st);
-  return cudaSuccess;
-}
-
-template <int BW, int BH, int BM>
-cudaError_t launch_batch_bm(const SweepBatch& Bs, int n, cudaStream_t st) {
-  using S_ = SCfg<BW, BH>;
-  auto k = k_sweep_fast_batch<BW, BH, BM>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S_::SMEM);
-  if (e != cudaSuccess) return e;
-  if (Bs.cta0[n] == 0) return cudaSuccess;
-  k<<<Bs.cta0[n], kSweepThreads, S_::SMEM, st>>>(Bs);
+  if (Bs.cta0[Bs.n] == 0) return cudaSuccess;
+  k<<<Bs.cta0[Bs.n], kSweepThreads, S_::SMEM, st>>>(Bs);
   count_launch();
   return cudaGetLastError();
 }
 
-template <int BW, int BH>
-cudaError_t launch_batch_size(const SweepBatch& Bs, int n, cudaStream_t st) {
-  switch (Bs.p[0].inv.bm) {
-  case -1: return launch_batch_bm<BW, BH, -1>(Bs, n, st);
-  case 1: return launch_batch_bm<BW, BH, 1>(Bs, n, st);
-  case 2: return launch_batch_bm<BW, BH, 2>(Bs, n, st);
-  case 3: return launch_batch_bm<BW, BH, 3>(Bs, n, st);
-  case 4: return launch_batch_bm<BW, BH, 4>(Bs, n, st);
-  default: return cudaErrorNotSupported;
+template <int BW, int BH, int BM>
+cudaError_t launch_bm(const SweepBatch& Bs, cudaStream_t st) {
+  switch (filter_switches(Bs)) {
+  case kSwPlain: return launch_sw<BW, BH, BM, kSwPlain>(Bs, st);
+  case kSwSharpen: return launch_sw<BW, BH, BM, kSwSharpen>(Bs, st);
+  default: return launch_sw<BW, BH, BM, kSwAny>(Bs, st);
   }
 }
 
 template <int BW, int BH>
-cudaError_t launch_size(const SweepArgs& a, cudaStream_t st, cudaEvent_t mark) {
-  switch (a.inv.bm) {
-  case -1: return launch_bm<BW, BH, -1>(a, st, mark);
-  case 1: return launch_bm<BW, BH, 1>(a, st, mark);
-  case 2: return launch_bm<BW, BH, 2>(a, st, mark);
-  case 3: return launch_bm<BW, BH, 3>(a, st, mark);
-  case 4: return launch_bm<BW, BH, 4>(a, st, mark);
+cudaError_t launch_size(const SweepBatch& Bs, cudaStream_t st) {
+  switch (Bs.p[0].inv.bm) {
+  case -1: return launch_bm<BW, BH, -1>(Bs, st);
+  case 1: return launch_bm<BW, BH, 1>(Bs, st);
+  case 2: return launch_bm<BW, BH, 2>(Bs, st);
+  case 3: return launch_bm<BW, BH, 3>(Bs, st);
+  case 4: return launch_bm<BW, BH, 4>(Bs, st);
   default: return cudaErrorNotSupported;
   }
 }
@@ -236,9 +230,9 @@ cudaError_t launch_sweep_fast_batch(const SweepArgs* planes, int n, cudaStream_t
   if (!sweep_batches(p, n, Bf, Bs, Bm, false)) return cudaErrorNotSupported;
   cudaError_t e;
   switch (planes[0].inv.g.bw) {
-  case 8: e = launch_batch_size<8, 8>(Bs, n, st); break;
-  case 16: e = launch_batch_size<16, 16>(Bs, n, st); break;
-  case 32: e = launch_batch_size<32, 32>(Bs, n, st); break;
+  case 8: e = launch_size<8, 8>(Bs, st); break;
+  case 16: e = launch_size<16, 16>(Bs, st); break;
+  case 32: e = launch_size<32, 32>(Bs, st); break;
   default: return cudaErrorNotSupported;
   }
   if (e != cudaSuccess) return e;
@@ -278,12 +272,7 @@ size_t sweep_seam_floats(const Geo& g, int strips, int segs) {
 cudaError_t launch_sweep(int form, const SweepArgs& a, cudaStream_t st, cudaEvent_t mark) {
   if (!sweep_supported(form, a.inv.g, a.inv.bm)) return cudaErrorNotSupported;
   if (form == F3D_FORM_TC) return launch_sweep_tc(a, st, mark);
-  switch (a.inv.g.bw) {
-  case 8: return launch_size<8, 8>(a, st, mark);
-  case 16: return launch_size<16, 16>(a, st, mark);
-  case 32: return launch_size<32, 32>(a, st, mark);
-  default: return cudaErrorNotSupported;
-  }
+  return launch_sweep_fast_batch(&a, 1, st, mark);
 }
 
 }  // namespace f3d

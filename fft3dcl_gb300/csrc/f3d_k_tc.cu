@@ -616,20 +616,6 @@ struct FltCfg {
   static constexpr uint32_t BYTES = DC + C::G * 4;
 };
 
-// The switches of the temporal filter as the kernel is built for them: the
-// two usual sets fixed at compile time, or read per bin (about ten
-// instructions of branches per bin). Products that are added later are
-// rounded by themselves (prod), so the three give the same bits.
-enum FilterSwitches { kSwPlain = 0, kSwSharpen = 1, kSwAny = 2 };  // degrid; degrid + sharpen; any
-template <int SW>
-__device__ __forceinline__ void fix_switches(FilterArgs& f) {
-  if constexpr (SW != kSwAny) {
-    f.dg = 1;
-    f.pat = 0;
-    f.shp = SW == kSwSharpen;
-  }
-}
-
 // One bin's result into the image at img (offset `at` of its hi part), or,
 // of columns 0 and n/2, into side.
 template <int N>
@@ -1210,17 +1196,6 @@ const void* filter_kernel_n(int sw, int bm, bool half) {
 template <int N>
 const void* filter_kernel(int minb, int sw, int bm, bool half) {
   return minb >= 5 ? filter_kernel_n<N, 5>(sw, bm, half) : filter_kernel_n<N, 4>(sw, bm, half);
-}
-
-// The switches all planes of a batch share.
-int filter_switches(const SweepBatch& S) {
-  int sw = -1;
-  for (int i = 0; i < S.n; i++) {
-    const FilterArgs& f = S.p[i].inv;
-    const int s = !f.dg || f.pat ? kSwAny : (f.shp ? kSwSharpen : kSwPlain);
-    sw = sw < 0 || sw == s ? s : kSwAny;
-  }
-  return sw;
 }
 
 // The filter launch of a batch (one CTA per group of blocks).

@@ -62,6 +62,12 @@ struct FilterArgs {
   float sigma_x, sigma_y, beta_x, beta, ssmin, ssmax, kalman_cn, kr2;
 };
 
+// The switches of the temporal filter as a kernel is built for them: the two
+// usual sets (degrid; degrid + sharpen) fixed at compile time, or any, read
+// per bin.
+enum FilterSwitches { kSwPlain = 0, kSwSharpen = 1, kSwAny = 2 };
+inline int filter_switches(const FilterArgs& f) { return !f.dg || f.pat ? kSwAny : (f.shp ? kSwSharpen : kSwPlain); }
+
 // Filter and inverse of one output.
 struct InvArgs : FilterArgs {
   Geo g;
