@@ -823,7 +823,7 @@ struct f3d_batch {
     cudaGraphExec_t x = nullptr;
     int kernels = 0;
   };
-  std::map<uint64_t, Graph> graphs;  // by the planes with a forward (bits 0-15), an output (16-31), overlap (32)
+  std::map<uint64_t, Graph> graphs;  // by the planes with a forward (bits 0-15), an output (16-31), overlap (32), unaligned rows (33)
   std::string err;
   // Side stream of the forward when it does not feed this step's outputs.
   cudaStream_t side = nullptr;
@@ -1028,6 +1028,7 @@ int f3d_batch_step(f3d_batch* b, const int* fns, const void* const* dev_src, con
           for (int k = 0; k < nwin[j]; k++)
             if (windows[j][k] == fns[i]) overlap = false;
   if (overlap) mask |= 1ull << 32;
+  if (!b->fast && nf > 0 && !tc_rows_aligned(fa, nf)) mask |= 1ull << 33;
   // Filter and inverse; timed by events unless being captured.
   auto sweep = [&](const TcTune& t, cudaEvent_t after_filter) -> cudaError_t {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;

@@ -105,7 +105,17 @@ constexpr uint64_t kWaitNs = 1000000000ull;  // one second
 template <int N, bool SPLIT>
 struct FwdSmem {
   using C = TcCfg<N>;
-  static constexpr uint32_t A1_TILE = (SPLIT ? 2 : 1) * C::A1_BYTES;  // hi[, lo] of one step-1 tile
+  // Step-1 operand: core matrices of 8 rows x 16 bytes, those of 8 columns of
+  // all rows together (SBO 128), LBO apart. LBO is 32 or 64 bytes over a
+  // multiple of 128: the chunks of a row that neighbouring lanes deposit then
+  // fall in different banks (in the same four before: 512 of the 1214
+  // shared-memory wavefronts of a 10-bit group).
+  static constexpr uint32_t A1_LBO = 128 * 16 + (N == 32 ? 32 : 64), A1_SBO = 128;
+  static constexpr uint32_t A1_PART = C::K1 / 8 * A1_LBO;
+  static constexpr uint32_t A1_TILE = (SPLIT ? 2 : 1) * A1_PART;      // hi[, lo] of one step-1 tile
+  static constexpr uint32_t a1_off(int row, int k) {
+    return (k >> 3) * A1_LBO + (row >> 3) * A1_SBO + (row & 7) * 16 + (k & 7) * 2;
+  }
   static constexpr uint32_t STAGE_BYTES = C::G * C::PS * 8;           // float2 [G][N][FBW]
   static constexpr uint32_t B2 = 0;                       // hi, lo
   static constexpr uint32_t B1 = B2 + 2 * C::B2_BYTES;    // hi, lo
@@ -117,64 +127,158 @@ struct FwdSmem {
   static constexpr uint32_t BYTES = TSLOT + 16 + 1024;    // + alignment slack
   static_assert(STAGE % 16 == 0 && A1 % 128 == 0 && BAR % 16 == 0, "bulk-copy and operand alignment");
 };
-// CTAs per SM of the forward kernel: the launch bound, and what fits.
+// CTAs per SM of the forward kernel: three fit in shared memory without the
+// split, two with it; the words of unaligned rows do not fit in the registers
+// of three (spilled registers cost more than the third CTA: 4K 10-bit 52 -> 60
+// us with 30 bytes of them).
 constexpr int kFwdMaxCtasPerSm = 3;
+constexpr int fwd_ctas(bool split, bool aligned, int bps) { return split || (!aligned && bps == 2) ? 2 : kFwdMaxCtasPerSm; }
 
-// Gather of a group's samples: task q covers 16 source bytes (16/BPS samples)
-// of row y of block bl. The raw bytes are fetched into registers one group
+// Gather of a group's samples: a task covers 16 source bytes (16/BPS samples)
+// of a row of a block. The raw bytes are fetched into registers one group
 // ahead, so that their loads are in flight while the tensor cores work on the
-// current group, and deposited into the step-1 operand as fp16.
+// current group, and deposited into the step-1 operand as fp16. A thread's
+// tasks are one chunk of one row of every BSTEP-th block; neighbouring lanes
+// take the chunks of a row. (Eight rows of a chunk for neighbouring lanes would
+// store without bank conflicts in any layout, but touch 8 lines in every
+// quarter of a load: 4K 10-bit 52 -> 57 us.)
 template <int N, int BPS>
 struct Gather {
   static constexpr int S = 16 / BPS;                   // samples per task
   static constexpr int TPR = N / S;                    // tasks per block row
   static constexpr int TASKS = TcCfg<N>::G * N * TPR;
   static constexpr int TPT = TASKS / kTcThreads;       // tasks per thread
+  static constexpr int BSTEP = kTcThreads / TPR / N;
   static_assert(TASKS % kTcThreads == 0 && S >= 4, "task split");
+  static_assert(BSTEP * TPR * N == kTcThreads, "a thread keeps its row");
+  static __device__ __forceinline__ int chunk() { return threadIdx.x % TPR; }
+  static __device__ __forceinline__ int row() { return threadIdx.x / TPR % N; }
+  static __device__ __forceinline__ int block() { return threadIdx.x / TPR / N; }
 };
 
-template <int N, int BPS>
-__device__ __forceinline__ void fetch(const TcFwdArgs& a, int b0, int nvalid, uint4 (&r)[Gather<N, BPS>::TPT]) {
+// mirror_i; within one plane width of the plane one reflection does it,
+// without the division.
+__device__ __forceinline__ int mirror_near(int x, int w) {
+  if (x >= -w && x < 2 * w) return x < 0 ? -1 - x : (x < w ? x : 2 * w - 1 - x);
+  return mirror_i(x, w);
+}
+
+// 16 bytes at p: one load where they are aligned, else the words that hold
+// them. (A word read here holds at least one of the 16 bytes.)
+__device__ __forceinline__ uint4 load16(const uint8_t* p) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+  if ((at & 15) == 0) return __ldg(reinterpret_cast<const uint4*>(p));
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(at & ~static_cast<uintptr_t>(3));
+  const uint32_t sh = (at & 3) * 8;
+  uint4 r = make_uint4(__ldg(w), __ldg(w + 1), __ldg(w + 2), __ldg(w + 3));
+  if (sh) {
+    const uint32_t e = __ldg(w + 4);
+    r = make_uint4(__funnelshift_r(r.x, r.y, sh), __funnelshift_r(r.y, r.z, sh), __funnelshift_r(r.z, r.w, sh),
+                   __funnelshift_r(r.w, e, sh));
+  }
+  return r;
+}
+// r = the 16 bytes (word) at p where `on`, else unchanged.
+__device__ __forceinline__ void load16_if(bool on, const uint8_t* p, uint4& r) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t@q ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%5];\n\t}"
+      : "+r"(r.x), "+r"(r.y), "+r"(r.z), "+r"(r.w)
+      : "r"((int)on), "l"(p));
+}
+__device__ __forceinline__ void load4_if(bool on, const uint8_t* p, uint32_t& r) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q ld.global.nc.u32 %0, [%2];\n\t}"
+               : "+r"(r)
+               : "r"((int)on), "l"(p));
+}
+
+// Raw bytes of a thread's tasks, one group ahead. ALIGNED: rows whose blocks
+// start on 16 bytes (of every plane of the launch); else the words that hold
+// the 16 bytes, shifted into place when they are used. plain: the group lies in
+// one block row, inside the plane, and its loads have been issued; other groups
+// (mirrored blocks, the ends of block rows) are read when they are used. The
+// loads are predicated: behind a branch they were waited for where the paths
+// join, one group early (4K 10-bit 50 -> 59 us).
+template <int N, int BPS, bool ALIGNED>
+struct RawGroup {
   using Gt = Gather<N, BPS>;
-  // The group's blocks are consecutive in the mode-1 grid (the only mode of
-  // this form): one division for the first, a carry into the next block row
-  // for the others.
-  const int m0 = b0 / a.g.ncols, n0 = b0 - m0 * a.g.ncols;
+  static constexpr bool EXTRA = !ALIGNED && BPS < 4;  // a fifth word where rows start inside words
+  uint4 r[Gt::TPT];
+  uint32_t e[EXTRA ? Gt::TPT : 1];
+  uint32_t sh;
+  bool plain;
+
+  __device__ __forceinline__ void fetch(const TcFwdArgs& a, int b0, int nvalid) {
+    const int m0 = b0 / a.g.ncols, n0 = b0 - m0 * a.g.ncols;
+    const int bx0 = a.g.xoff + n0 * a.g.xstep, by0 = a.g.yoff + m0 * a.g.ystep;
+    plain = nvalid == TcCfg<N>::G && n0 + TcCfg<N>::G <= a.g.ncols && by0 >= 0 && by0 + N <= a.g.H && bx0 >= 0 &&
+            bx0 + (TcCfg<N>::G - 1) * a.g.xstep + N <= a.g.W;
+    const uint8_t* p = a.src + (long long)(by0 + Gt::row()) * a.pitch + (bx0 + Gt::block() * a.g.xstep) * BPS + 16 * Gt::chunk();
+    const int step = Gt::BSTEP * a.g.xstep * BPS;  // a multiple of 4
+    sh = ALIGNED ? 0u : (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3) * 8;
+    if constexpr (!ALIGNED) p -= sh / 8;
 #pragma unroll
-  for (int i = 0; i < Gt::TPT; i++) {
-    const int q = threadIdx.x + i * kTcThreads;
-    const int c = q % Gt::TPR, ry = q / Gt::TPR;
-    const int bl = ry / N, y = ry - bl * N;
-    r[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (bl >= nvalid) continue;
-    int n = n0 + bl, m = m0;
-    while (n >= a.g.ncols) {
-      n -= a.g.ncols;
-      m++;
-    }
-    const int bx = a.g.xoff + n * a.g.xstep, by = a.g.yoff + m * a.g.ystep;
-    if (bx >= 0 && by >= 0 && bx + N <= a.g.W && by + N <= a.g.H) {
-      const uint8_t* p = a.src + (long long)(by + y) * a.pitch + (long long)bx * BPS + 16 * c;
-      if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-        r[i] = __ldg(reinterpret_cast<const uint4*>(p));
-        continue;
+    for (int i = 0; i < Gt::TPT; i++) {
+      r[i] = make_uint4(0u, 0u, 0u, 0u);
+      if constexpr (ALIGNED) {
+        load16_if(plain, p + i * step, r[i]);
+      } else {
+        load4_if(plain, p + i * step, r[i].x);
+        load4_if(plain, p + i * step + 4, r[i].y);
+        load4_if(plain, p + i * step + 8, r[i].z);
+        load4_if(plain, p + i * step + 12, r[i].w);
+        if constexpr (EXTRA) {
+          e[i] = 0u;
+          load4_if(plain && sh, p + i * step + 16, e[i]);
+        }
       }
     }
-    // Mirrored or unaligned: one sample at a time (src/cpu/reference.cpp:10-17).
-    const uint8_t* row = a.src + (long long)mirror_i(by + y, a.g.H) * a.pitch;
-    uint32_t w[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-    for (int k = 0; k < Gt::S; k++) {
-      const int x = mirror_i(bx + c * Gt::S + k, a.g.W);
-      uint32_t v;
-      if (BPS == 1) v = row[x];
-      else if (BPS == 2) v = reinterpret_cast<const uint16_t*>(row)[x];
-      else v = reinterpret_cast<const uint32_t*>(row)[x];
-      w[(k * BPS) / 4] |= v << (8 * ((k * BPS) % 4));
-    }
-    r[i] = make_uint4(w[0], w[1], w[2], w[3]);
   }
-}
+
+  // The bytes of the group that fetch() was called for, in r.
+  __device__ __forceinline__ void finish(const TcFwdArgs& a, int b0, int nvalid) {
+    if (plain) {
+      if constexpr (EXTRA) {
+#pragma unroll
+        for (int i = 0; i < Gt::TPT; i++)
+          r[i] = make_uint4(__funnelshift_r(r[i].x, r[i].y, sh), __funnelshift_r(r[i].y, r[i].z, sh),
+                            __funnelshift_r(r[i].z, r[i].w, sh), __funnelshift_r(r[i].w, e[i], sh));
+      }
+      return;
+    }
+    // The group's blocks are consecutive in the mode-1 grid (the only mode of
+    // this form): one division for the first, a carry into the next block row
+    // for the others.
+    const int m0 = b0 / a.g.ncols, n0 = b0 - m0 * a.g.ncols;
+#pragma unroll
+    for (int i = 0; i < Gt::TPT; i++) {
+      const int bl = Gt::block() + i * Gt::BSTEP, y = Gt::row(), c = Gt::chunk();
+      if (bl >= nvalid) continue;
+      int n = n0 + bl, m = m0;
+      while (n >= a.g.ncols) {
+        n -= a.g.ncols;
+        m++;
+      }
+      const int bx = a.g.xoff + n * a.g.xstep, by = a.g.yoff + m * a.g.ystep;
+      if (bx >= 0 && by >= 0 && bx + N <= a.g.W && by + N <= a.g.H) {
+        r[i] = load16(a.src + (long long)(by + y) * a.pitch + (long long)bx * BPS + 16 * c);
+        continue;
+      }
+      // Mirrored: one sample at a time (src/cpu/reference.cpp:10-17).
+      const uint8_t* line = a.src + (long long)mirror_near(by + y, a.g.H) * a.pitch;
+      uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+      for (int k = 0; k < Gt::S; k++) {
+        const int x = mirror_near(bx + c * Gt::S + k, a.g.W);
+        uint32_t v;
+        if (BPS == 1) v = line[x];
+        else if (BPS == 2) v = reinterpret_cast<const uint16_t*>(line)[x];
+        else v = reinterpret_cast<const uint32_t*>(line)[x];
+        w[(k * BPS) / 4] |= v << (8 * ((k * BPS) % 4));
+      }
+      r[i] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+};
 
 // Raw bytes -> fp16 (hi, and lo on the split path) in A1[tile][part]: rows
 // (block % BPT1, y), K = x.
@@ -182,6 +286,7 @@ template <int N, int BPS, bool SPLIT>
 __device__ __forceinline__ void deposit(const TcFwdArgs& a, uint8_t* a1, const uint4 (&r)[Gather<N, BPS>::TPT]) {
   using Gt = Gather<N, BPS>;
   using C = TcCfg<N>;
+  using L = FwdSmem<N, SPLIT>;
   const bool split = SPLIT && a.split;
   // Integer samples below 1024 become fp16 exactly by exponent bias: 0x6400
   // is 1024.0, and its ten mantissa bits hold the sample, so (0x6400 | v) -
@@ -197,9 +302,7 @@ __device__ __forceinline__ void deposit(const TcFwdArgs& a, uint8_t* a1, const u
   const __half2 k1024 = __halves2half2(__ushort_as_half(0x6400), __ushort_as_half(0x6400));
 #pragma unroll
   for (int i = 0; i < Gt::TPT; i++) {
-    const int q = threadIdx.x + i * kTcThreads;
-    const int c = q % Gt::TPR, ry = q / Gt::TPR;
-    const int bl = ry / N, y = ry - bl * N;
+    const int c = Gt::chunk(), bl = Gt::block() + i * Gt::BSTEP, y = Gt::row();
     const int tile = bl / C::BPT1, row = (bl % C::BPT1) * N + y;
     const uint32_t w[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
     uint32_t h[Gt::S / 2], l[Gt::S / 2];
@@ -224,20 +327,20 @@ __device__ __forceinline__ void deposit(const TcFwdArgs& a, uint8_t* a1, const u
 #pragma unroll
       for (int k = 0; k < Gt::S / 2; k++) tc::split_pair(v[2 * k], v[2 * k + 1], h[k], l[k]);
     }
-    uint8_t* t0 = a1 + tile * FwdSmem<N, SPLIT>::A1_TILE;
+    uint8_t* t0 = a1 + tile * L::A1_TILE;
     const int x0 = c * Gt::S;
     if (Gt::S >= 8) {
 #pragma unroll
       for (int j = 0; j < Gt::S / 8; j++) {
-        const uint32_t o = tc::off_il(row, x0 + 8 * j, C::K1);
+        const uint32_t o = L::a1_off(row, x0 + 8 * j);
         *reinterpret_cast<uint4*>(t0 + o) = make_uint4(h[4 * j], h[4 * j + 1], h[4 * j + 2], h[4 * j + 3]);
         if (split)
-          *reinterpret_cast<uint4*>(t0 + C::A1_BYTES + o) = make_uint4(l[4 * j], l[4 * j + 1], l[4 * j + 2], l[4 * j + 3]);
+          *reinterpret_cast<uint4*>(t0 + L::A1_PART + o) = make_uint4(l[4 * j], l[4 * j + 1], l[4 * j + 2], l[4 * j + 3]);
       }
     } else {
-      const uint32_t o = tc::off_il(row, x0, C::K1);
+      const uint32_t o = L::a1_off(row, x0);
       *reinterpret_cast<uint2*>(t0 + o) = make_uint2(h[0], h[1]);
-      if (split) *reinterpret_cast<uint2*>(t0 + C::A1_BYTES + o) = make_uint2(l[0], l[1]);
+      if (split) *reinterpret_cast<uint2*>(t0 + L::A1_PART + o) = make_uint2(l[0], l[1]);
     }
   }
 }
@@ -250,8 +353,15 @@ __device__ __forceinline__ int plane_of(const Batch& b, const int (&prefix)[kMax
   return p;
 }
 
-template <int N, int BPS, bool SPLIT>
-__global__ void __launch_bounds__(kTcThreads, kFwdMaxCtasPerSm) k_forward_tc(const __grid_constant__ TcFwdBatch B) {
+// Forward kernel: bound by the latency of a group's barrier-separated phases
+// (tensor memory -> registers -> shared memory -> tensor cores), which three
+// CTAs per SM overlap, and by shared-memory wavefronts. Without the address
+// work and the bank conflicts of the gather (829 -> 590 instructions per block)
+// ten 4K 10-bit outputs' step takes 1422 -> 1387 us; one 4K frame stays at 49
+// us (cold), 1919x1079 float with 16x16 blocks goes 38 -> 30 us with word
+// loads for its unaligned rows.
+template <int N, int BPS, bool SPLIT, bool ALIGNED>
+__global__ void __launch_bounds__(kTcThreads, fwd_ctas(SPLIT, ALIGNED, BPS)) k_forward_tc(const __grid_constant__ TcFwdBatch B) {
   using C = TcCfg<N>;
   using L = FwdSmem<N, SPLIT>;
   using T = TcTab<N>;
@@ -262,6 +372,26 @@ __global__ void __launch_bounds__(kTcThreads, kFwdMaxCtasPerSm) k_forward_tc(con
   uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + L::TSLOT);
   float2* stage = reinterpret_cast<float2*>(sm + L::STAGE);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  const int ngroups = B.grp0[B.n];
+  uint32_t phase = 0;
+  RawGroup<N, BPS, ALIGNED> raw;
+  // The CTA's groups ascend, and so do their planes: pl is that of the group
+  // whose spectra leave next, at or before any later group's.
+  int pl = 0;
+  auto plane_from = [&](int g) {
+    int p = pl;
+    while (g >= B.grp0[p + 1]) p++;
+    return p;
+  };
+  // Raw samples of batch group g (the block group g - grp0[p] of plane p).
+  auto fetch_group = [&](int g) {
+    const int p = plane_from(g);
+    const TcFwdArgs& ap = B.p[p];
+    const int b = (g - B.grp0[p]) * C::G;
+    raw.fetch(ap, b, min(C::G, ap.g.nb - b));
+  };
+  if ((int)blockIdx.x < ngroups) fetch_group(blockIdx.x);  // on its way while the CTA is set up
 
   // Constant operands (the same for every plane of a batch): B2 (hi, lo) and
   // B1 (hi, lo) are contiguous in the table.
@@ -286,23 +416,16 @@ __global__ void __launch_bounds__(kTcThreads, kFwdMaxCtasPerSm) k_forward_tc(con
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = *tslot;
-  const int ngroups = B.grp0[B.n];
-  uint32_t phase = 0;
-  uint4 raw[Gather<N, BPS>::TPT];
-  // Raw samples of batch group g (the block group g - grp0[p] of plane p).
-  auto fetch_group = [&](int g) {
-    const int p = plane_of(B, B.grp0, g);
-    const TcFwdArgs& ap = B.p[p];
-    const int b = (g - B.grp0[p]) * C::G;
-    fetch<N, BPS>(ap, b, min(C::G, ap.g.nb - b), raw);
-  };
   // Group g (its samples in raw) into A1, the loads of the CTA's group after
   // it started, then step 1 on the tensor cores: D1[tile] = A1 * B1^T, two or
   // three passes, committed to bar[0]. A1 and D1 must be free: no step 1 in
   // flight, D1 read out.
   auto begin_group = [&](int g) {
-    const TcFwdArgs& ap = B.p[plane_of(B, B.grp0, g)];
-    deposit<N, BPS, SPLIT>(ap, sm + L::A1, raw);
+    const int p = plane_from(g);
+    const TcFwdArgs& ap = B.p[p];
+    const int b = (g - B.grp0[p]) * C::G;
+    raw.finish(ap, b, min(C::G, ap.g.nb - b));
+    deposit<N, BPS, SPLIT>(ap, sm + L::A1, raw.r);
     if (g + (int)gridDim.x < ngroups) fetch_group(g + gridDim.x);
     tc::fence_async_smem();
     tc::fence_before_sync();
@@ -312,32 +435,29 @@ __global__ void __launch_bounds__(kTcThreads, kFwdMaxCtasPerSm) k_forward_tc(con
       constexpr uint32_t id1 = tc::idesc_f16(128, C::N1);
       const uint32_t sbo = (C::K1 / 8) * 128;
       for (int t = 0; t < C::T1; t++) {
-        const uint32_t a_hi = sbase + L::A1 + t * L::A1_TILE, a_lo = a_hi + C::A1_BYTES;
+        const uint32_t a_hi = sbase + L::A1 + t * L::A1_TILE, a_lo = a_hi + L::A1_PART;
         const uint32_t d = tmem + C::D1_COL + t * C::N1;
         for (int ks = 0; ks < C::K1 / 16; ks++) {
-          const uint64_t ah = tc::sdesc(a_hi + ks * 256, 128, sbo, tc::LAYOUT_INTERLEAVE);
+          const uint64_t ah = tc::sdesc(a_hi + ks * 2 * L::A1_LBO, L::A1_LBO, L::A1_SBO, tc::LAYOUT_INTERLEAVE);
           const uint64_t bh = tc::sdesc(sbase + L::B1 + ks * 256, 128, sbo, tc::LAYOUT_INTERLEAVE);
           const uint64_t bl = tc::sdesc(sbase + L::B1 + C::B1_BYTES + ks * 256, 128, sbo, tc::LAYOUT_INTERLEAVE);
           tc::mma_f16(d, ah, bh, id1, ks > 0);
           tc::mma_f16(d, ah, bl, id1, 1);
           if (SPLIT && ap.split)
-            tc::mma_f16(d, tc::sdesc(a_lo + ks * 256, 128, sbo, tc::LAYOUT_INTERLEAVE), bh, id1, 1);
+            tc::mma_f16(d, tc::sdesc(a_lo + ks * 2 * L::A1_LBO, L::A1_LBO, L::A1_SBO, tc::LAYOUT_INTERLEAVE), bh, id1, 1);
         }
       }
       tc::mma_commit(&bar[0]);
     }
   };
-  if ((int)blockIdx.x < ngroups) {
-    fetch_group(blockIdx.x);
-    begin_group(blockIdx.x);
-  }
+  if ((int)blockIdx.x < ngroups) begin_group(blockIdx.x);
 
   // Per group: step 1 was issued one iteration earlier; step 2 runs while
   // the next group's samples are deposited and its step 1 issued; the
   // spectra are staged and leave by one bulk copy, which drains while the
   // next group goes through steps 1 to 5.
   for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
-    const int pl = plane_of(B, B.grp0, grp);
+    pl = plane_from(grp);
     const TcFwdArgs& a = B.p[pl];
     const int b0 = (grp - B.grp0[pl]) * C::G;
     const int nvalid = min(C::G, a.g.nb - b0);
@@ -356,15 +476,19 @@ __global__ void __launch_bounds__(kTcThreads, kFwdMaxCtasPerSm) k_forward_tc(con
       const int t = warp >> 2, s = warp & 3;
       const int r1 = 32 * s + lane;
       const int bl = t * C::BPT1 + r1 / N, y = r1 % N;
-      float v[C::N1];
-      tc::tmem_ld<C::N1>(tmem + ((uint32_t)(32 * s) << 16) + C::D1_COL + t * C::N1, v);
+      // 16 columns at a time: the next group's samples are in registers too.
 #pragma unroll
-      for (int kp = 0; kp < C::NY; kp++) {
-        uint32_t hi, lo;
-        tc::split_pair(v[2 * kp], v[2 * kp + 1], hi, lo);
-        const uint32_t o = a2_off<N>(bl * C::NY + kp, 2 * y);
-        *reinterpret_cast<uint32_t*>(sm + L::A2 + o) = hi;
-        *reinterpret_cast<uint32_t*>(sm + L::A2 + C::A2_BYTES + o) = lo;
+      for (int k0 = 0; k0 < C::NY; k0 += 8) {
+        float v[16];
+        tc::tmem_ld<16>(tmem + ((uint32_t)(32 * s) << 16) + C::D1_COL + t * C::N1 + 2 * k0, v);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          uint32_t hi, lo;
+          tc::split_pair(v[2 * k], v[2 * k + 1], hi, lo);
+          const uint32_t o = a2_off<N>(bl * C::NY + k0 + k, 2 * y);
+          *reinterpret_cast<uint32_t*>(sm + L::A2 + o) = hi;
+          *reinterpret_cast<uint32_t*>(sm + L::A2 + C::A2_BYTES + o) = lo;
+        }
       }
     }
     tc::fence_async_smem();
@@ -461,7 +585,7 @@ __global__ void __launch_bounds__(kTcThreads, kFwdMaxCtasPerSm) k_forward_tc(con
       tc::bulk_commit();
     }
   }
-  if (tid == 0) tc::bulk_wait();
+  if (tid == 0) tc::bulk_wait_read();  // the shared memory outlives the copies out of it
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -742,7 +866,7 @@ __global__ void __launch_bounds__(kTcThreads, MINB) k_filter_tc(const __grid_con
   if (tid == 0) {
     tc::bulk_store(P.img + (size_t)b0 * K::IMG, smem_f, nvb * K::IMG);
     tc::bulk_commit();
-    tc::bulk_wait();
+    tc::bulk_wait_read();
   }
 }
 
@@ -928,9 +1052,9 @@ __device__ __forceinline__ bool inverse_row(const SweepArgs& sa, InvState& st, i
 }
 
 // Constant operands of the inverse (C2 hi, lo, then C1 A hi, lo, B hi, lo)
-// into shared memory, tensor memory and the barriers.
+// into shared memory, and tensor memory.
 template <int N>
-__device__ __forceinline__ void inverse_setup(const SweepArgs& sa, uint8_t* sm, uint64_t* bar, uint32_t* tslot) {
+__device__ __forceinline__ void inverse_setup(const SweepArgs& sa, uint8_t* sm, uint32_t* tslot) {
   using C = TcCfg<N>;
   using S = SwpCfg<N>;
   using T = TcTab<N>;
@@ -944,10 +1068,6 @@ __device__ __forceinline__ void inverse_setup(const SweepArgs& sa, uint8_t* sm, 
   if ((tid >> 5) == 0) {
     tc::tmem_alloc(tslot, C::TMEM_COLS);
     tc::tmem_relinquish();
-  }
-  if (tid == 0) {
-    for (int i = 0; i < 3; i++) tc::mbar_init(&bar[i], 1);
-    tc::fence_mbar_init();
   }
 }
 
@@ -976,8 +1096,9 @@ __global__ void __launch_bounds__(kTcThreads, kTcSweepCtasPerSm) k_sweep_tc(cons
   auto tile_of = [&](int m) { return sa.img + ((size_t)m * sa.inv.g.ncols + J0) * BlkImg<N>::BYTES; };
   const uint32_t tile_bytes = (ncell + 1) * BlkImg<N>::BYTES;
 
-  inverse_setup<N>(sa, sm, bar, tslot);
-  if (tid == 0) {
+  if (tid == 0) {  // the first tile is on its way while the CTA is set up
+    for (int i = 0; i < 3; i++) tc::mbar_init(&bar[i], 1);
+    tc::fence_mbar_init();
     tc::fence_async_smem();
     if (M0 < M1) {
       tc::mbar_expect_tx(&bar[0], tile_bytes);
@@ -986,6 +1107,8 @@ __global__ void __launch_bounds__(kTcThreads, kTcSweepCtasPerSm) k_sweep_tc(cons
       if (!(sa.test_skip && cta == 0)) tc::bulk_load(sm + S::A2, tile_of(M0), tile_bytes, &bar[0]);
     }
   }
+  inverse_setup<N>(sa, sm, tslot);
+  tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -1134,38 +1257,68 @@ std::vector<uint8_t> tc_tables(int n, const std::vector<double>& wx, const std::
 
 namespace {
 
+template <int N, bool ALIGNED>
+void (*forward_kernel(int fmt, bool split))(TcFwdBatch) {
+  return fmt == FMT_U8 ? k_forward_tc<N, 1, false, ALIGNED>
+         : fmt == FMT_U16 ? (split ? k_forward_tc<N, 2, true, ALIGNED> : k_forward_tc<N, 2, false, ALIGNED>)
+                          : k_forward_tc<N, 4, true, ALIGNED>;
+}
+// Whether the blocks of a plane start on 16 bytes in every row.
+bool rows_aligned(const TcFwdArgs& a, int bps) {
+  return ((reinterpret_cast<uintptr_t>(a.src) | (uintptr_t)a.pitch | (uintptr_t)(a.g.xoff * bps) |
+           (uintptr_t)(a.g.xstep * bps)) & 15) == 0;
+}
+
+// The forward launch of a batch of planes of one sample format: the split
+// kernel (hi + lo step-1 operand) where any plane needs it; it takes the others
+// too. Null where there is none.
+struct FwdLaunch {
+  void (*kernel)(TcFwdBatch) = nullptr;
+  size_t smem = 0;
+  int ctas = 0;  // per SM
+};
 template <int N>
-cudaError_t launch_forward_n(const TcFwdBatch& B, const TcFwdArgs* planes, int n, const TcTune& t,
-                             cudaStream_t st) {
-  // The split kernel (hi + lo step-1 operand) also takes planes that need no
-  // split; it fits two CTAs per SM, the other three.
+FwdLaunch forward_launch_n(const TcFwdArgs* planes, int n) {
+  FwdLaunch l;
+  const int fmt = planes[0].fmt;
+  const bool aligned = tc_rows_aligned(planes, n);
   bool split = false;
   for (int i = 0; i < n; i++) split = split || planes[i].split;
-  const int fmt = planes[0].fmt;
-  if (fmt == FMT_U8 && split) return cudaErrorNotSupported;
-  auto k = fmt == FMT_U8 ? k_forward_tc<N, 1, false>
-           : fmt == FMT_U16 ? (split ? k_forward_tc<N, 2, true> : k_forward_tc<N, 2, false>)
-                            : k_forward_tc<N, 4, true>;
-  const size_t smem = split ? FwdSmem<N, true>::BYTES : FwdSmem<N, false>::BYTES;
-  cudaError_t attr = prepare(k, smem);
-  if (attr != cudaSuccess) return attr;
-  const int ngroups = B.grp0[n];
-  if (ngroups == 0) return cudaSuccess;
-  const int per_sm = std::max(1, std::min(t.fwd_ctas_per_sm, split ? 2 : kFwdMaxCtasPerSm));
-  static_assert(kFwdMaxCtasPerSm * (FwdSmem<N, false>::BYTES + 1024) <= 228 * 1024, "CTAs per SM");
-  static_assert(2 * (FwdSmem<N, true>::BYTES + 1024) <= 228 * 1024, "CTAs per SM");
-  const int grid = std::min(ngroups, per_sm * sm_count());
-  k<<<grid, kTcThreads, smem, st>>>(B);
-  count_launch();
-  return cudaGetLastError();
+  if (fmt == FMT_U8 && split) return l;
+  l.kernel = aligned ? forward_kernel<N, true>(fmt, split) : forward_kernel<N, false>(fmt, split);
+  l.smem = split ? FwdSmem<N, true>::BYTES : FwdSmem<N, false>::BYTES;
+  l.ctas = fwd_ctas(split, aligned, fmt == FMT_U16 ? 2 : 1);
+  return l;
+}
+FwdLaunch forward_launch(const TcFwdArgs* planes, int n) {
+  return planes[0].g.bw == 16 ? forward_launch_n<16>(planes, n) : forward_launch_n<32>(planes, n);
 }
 
 }  // namespace
 
+bool tc_rows_aligned(const TcFwdArgs* planes, int n) {
+  const int bps = planes[0].fmt == FMT_U8 ? 1 : (planes[0].fmt == FMT_U16 ? 2 : 4);
+  for (int i = 0; i < n; i++)
+    if (!rows_aligned(planes[i], bps)) return false;
+  return true;
+}
+
 cudaError_t launch_forward_tc_batch(const TcFwdArgs* planes, int n, const TcTune& t, cudaStream_t st) {
   TcFwdBatch B;
   if (!forward_batch(planes, n, B)) return n < 1 || n > kMaxBatch ? cudaErrorInvalidValue : cudaErrorNotSupported;
-  return planes[0].g.bw == 16 ? launch_forward_n<16>(B, planes, n, t, st) : launch_forward_n<32>(B, planes, n, t, st);
+  const FwdLaunch l = forward_launch(planes, n);
+  if (!l.kernel) return cudaErrorNotSupported;
+  const cudaError_t attr = prepare(l.kernel, l.smem);
+  if (attr != cudaSuccess) return attr;
+  const int ngroups = B.grp0[n];
+  if (ngroups == 0) return cudaSuccess;
+  static_assert(kFwdMaxCtasPerSm * (FwdSmem<32, false>::BYTES + 1024) <= 228 * 1024, "CTAs per SM");
+  static_assert(2 * (FwdSmem<32, true>::BYTES + 1024) <= 228 * 1024, "CTAs per SM");
+  const int per_sm = std::max(1, std::min(t.fwd_ctas_per_sm, l.ctas));
+  const int grid = std::min(ngroups, per_sm * sm_count());
+  l.kernel<<<grid, kTcThreads, l.smem, st>>>(B);
+  count_launch();
+  return cudaGetLastError();
 }
 
 cudaError_t launch_forward_tc(const TcFwdArgs& a, cudaStream_t st) { return launch_forward_tc_batch(&a, 1, TcTune{}, st); }
@@ -1274,14 +1427,6 @@ cudaError_t launch_sweep_tc(const SweepArgs& a, cudaStream_t st, cudaEvent_t mar
   return launch_sweep_tc_batch(&a, 1, TcTune{}, st, mark);
 }
 
-namespace {
-template <int N>
-bool is_forward(const void* f) {
-  return f == (const void*)k_forward_tc<N, 1, false> || f == (const void*)k_forward_tc<N, 2, false> ||
-         f == (const void*)k_forward_tc<N, 2, true> || f == (const void*)k_forward_tc<N, 4, true>;
-}
-}  // namespace
-
 cudaError_t tc_graph_update(cudaGraphExec_t exec, cudaGraph_t graph, const TcFwdArgs* fwd, int nf,
                             const SweepArgs* sw, int ns) {
   TcFwdBatch Bw{};
@@ -1289,7 +1434,12 @@ cudaError_t tc_graph_update(cudaGraphExec_t exec, cudaGraph_t graph, const TcFwd
   FilterBatch F;
   FilterLaunch fl[2];
   cudaError_t e = cudaSuccess;
-  if (nf > 0 && !forward_batch(fwd, nf, Bw)) return cudaErrorNotSupported;
+  FwdLaunch wl;
+  if (nf > 0) {
+    if (!forward_batch(fwd, nf, Bw)) return cudaErrorNotSupported;
+    wl = forward_launch(fwd, nf);
+    if (!wl.kernel) return cudaErrorNotSupported;
+  }
   if (ns > 0) {
     if ((e = tc_sweep_batch(sw, ns, Bs)) != cudaSuccess) return e;
     for (int v = 0; v < 2; v++) fl[v] = filter_launch(Bs, 4 + v, F);
@@ -1307,7 +1457,7 @@ cudaError_t tc_graph_update(cudaGraphExec_t exec, cudaGraph_t graph, const TcFwd
     if ((e = cudaGraphKernelNodeGetParams(node, &kp)) != cudaSuccess) return e;
     void* args[1] = {nullptr};
     const void* f = kp.func;
-    if (is_forward<32>(f) || is_forward<16>(f)) {
+    if (nf > 0 && f == (const void*)wl.kernel) {
       args[0] = &Bw;
     } else if (ns > 0 && (f == fl[0].kernel || f == fl[1].kernel)) {
       args[0] = &F;

@@ -245,9 +245,12 @@ cudaError_t launch_forward_tc_batch(const TcFwdArgs* planes, int n, const TcTune
 // filter and the inverse kernels.
 cudaError_t launch_sweep_tc_batch(const SweepArgs* planes, int n, const TcTune& t, cudaStream_t st,
                                   cudaEvent_t mark, cudaEvent_t after_filter = nullptr);
+// Whether the blocks of every plane start on 16 bytes in every row: the
+// forward has a kernel for such planes and one for any.
+bool tc_rows_aligned(const TcFwdArgs* planes, int n);
 // Re-points the kernel nodes of a graph captured from launch_forward_tc_batch
 // (nf planes, 0: none) + launch_sweep_tc_batch (ns planes) at new plane
-// arguments of the same shapes.
+// arguments of the same shapes (and the same answer of tc_rows_aligned).
 cudaError_t tc_graph_update(cudaGraphExec_t exec, cudaGraph_t graph, const TcFwdArgs* fwd, int nf,
                             const SweepArgs* sw, int ns);
 // Tensor-core sweep: cells per strip, CTAs per SM, and the launches (filter,

@@ -35,3 +35,38 @@ def test_spectra_do_not_depend_on_placement(form, bw, bits):
                 e.prune(1 << 20, 1 << 20)
                 ref = got if ref is None else ref
                 np.testing.assert_array_equal(got.view(np.uint32), ref.view(np.uint32), err_msg=f"{pitch} {start}")
+
+
+@pytest.mark.parametrize("bits", [8, 10])
+def test_graph_steps_with_other_placements(bits):
+    # A batch replays its graph for planes placed alike; a frame at another
+    # alignment is another graph. Outputs equal the engine's own.
+    w, h, nfr = 192, 96, 9
+    dtype = np.uint8 if bits == 8 else np.uint16
+    peak = (1 << bits) - 1.0
+    frames = synth.moving_rects(w, h, nfr, 5, lo=peak * 0.1, hi=peak * 0.9, noise=2.0, dtype=dtype, maxval=peak)
+    ref = F.FFT3DCL(frames, bits=bits, form="tc", bt=3)
+    bps = frames[0].itemsize
+    pitch = w * bps + 16
+    bufs, ptrs = [], []
+    for i, f in enumerate(frames):
+        start = [0, bps, 16, 3 * bps][i % 4]
+        buf = torch.zeros(h * pitch + 64, dtype=torch.uint8, device="cuda")
+        buf[start:start + h * pitch].view(h, pitch)[:, :w * bps] = torch.from_numpy(f.view(np.uint8).reshape(h, -1).copy()).cuda()
+        bufs.append(buf)
+        ptrs.append(buf.data_ptr() + start)
+    st = torch.cuda.Stream()
+    out = torch.empty((nfr, h, w * bps), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    with F.Engine(w, h, bits, form="tc", bt=3, stream=st.cuda_stream) as e:
+        e.forward_device(0, ptrs[0], pitch)
+        with F.Batch([e], graph=True, autotune=False) as b:
+            for n in range(nfr):
+                win = [max(n - 1, 0), n, min(n + 1, nfr - 1)]
+                fn = n + 1 if n + 1 < nfr else -1
+                b.step([fn], [ptrs[fn] if fn >= 0 else 0], [pitch], [win], [out[n].data_ptr()], [w * bps])
+                e.prune(n, n + 2)
+            torch.cuda.synchronize()
+    got = out.cpu().numpy()
+    for n in range(nfr):
+        np.testing.assert_array_equal(got[n].view(dtype), ref[n])
