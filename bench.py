@@ -756,7 +756,7 @@ def run_gpu(args, rank, world, local_rank):
     ab = algorithmic_bytes(info.nblocks, info.fbw, ip.bh, bt)
     peak, peak_kind = load_peaks()
     inv_ms = float(kt[1])
-    # The dominant kernel, timed between the engine's events: the tensor-core
+    # The dominant kernel, timed by itself on the GPU: the tensor-core
     # filter (window spectra in; its operand tiles are an intermediate), the
     # fused fast-form sweep (window spectra in, packed plane out) or, unfused,
     # the filter+inverse kernel (window spectra in).

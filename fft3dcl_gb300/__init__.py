@@ -669,7 +669,7 @@ class Batch:
         return {"tuned": bool(tuned), "fwd_ctas_per_sm": a.value, "filter_minb": b.value}
 
     def last_kernel_ms(self) -> list[float]:
-        """[filter, inverse + overlap-add + seam merge] device ms of the last
+        """[filter, inverse + overlap-add] device ms of the last
         step with outputs that ran outside a CUDA graph."""
         ms = (C.c_float * 2)()
         if lib().f3d_batch_last_kernel_ms(self._h, ms) != F3D_OK:

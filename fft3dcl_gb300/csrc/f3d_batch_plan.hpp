@@ -125,6 +125,7 @@ inline void plan_segments(SweepArgs* planes, int n, int slots) {
 inline int filter_batch(const SweepBatch& S, int group, FilterBatch& F) {
   F.n = S.n;
   F.shifted = S.shifted;
+  F.clk = S.p[0].clk;
   F.cta0[0] = 0;
   for (int i = 0; i < S.n; i++) {
     const SweepArgs& a = S.p[i];

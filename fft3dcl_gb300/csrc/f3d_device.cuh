@@ -31,6 +31,21 @@ __host__ __device__ constexpr int bit_reverse(int i, int bits) {
   return r;
 }
 
+// A kernel's times, taken by its own threads (thread 0 of the first CTA, then
+// of every CTA): events around the kernels would keep each from starting until
+// the one before has ended and its time is written, about 2 us an event.
+__device__ __forceinline__ KernelClock device_ns() {
+  KernelClock t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+__device__ __forceinline__ void stamp_start(KernelClock* clk) {
+  if (clk && (blockIdx.x | blockIdx.y | threadIdx.x) == 0) clk[0] = device_ns();
+}
+__device__ __forceinline__ void stamp_end(KernelClock* clk) {
+  if (clk && threadIdx.x == 0) atomicMax(clk + 1, device_ns());
+}
+
 // D3D9 MIRROR addressing, src/cpu/reference.cpp:10-17.
 __device__ __forceinline__ int mirror_i(int x, int w) {
   int p = x % (2 * w);

@@ -102,9 +102,9 @@ struct f3d_engine {
   size_t img_bytes = 0;
 
   size_t bytes = 0;
-  // Kernel timing on the engine stream: forward [0,1], filter+inverse [2,4],
-  // overlap-add [4,3].
-  cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+  // Kernel times (start, end) of the last forward, filter + inverse (or filter)
+  // and overlap-add (or tensor-core inverse).
+  KernelClock* d_clk = nullptr;
   bool fwd_timed = false, proc_timed = false;
 
   int fail(int code, const std::string& msg) {
@@ -235,16 +235,16 @@ FwdArgs forward_args(const f3d_engine* e, const uint8_t* dsrc, long long pitch, 
 int run_forward(f3d_engine* e, int fn, const uint8_t* dsrc, long long pitch, int fmt) {
   float2* spec = spectra_slot(e, fn, true);
   if (!spec) return e->fail(F3D_E_NOMEM, "FFT3DCL: GPU spectra alloc failed");
-  const FwdArgs a = forward_args(e, dsrc, pitch, fmt, spec);
-  cudaEventRecord(e->ev[0], e->stream);
   cudaError_t ce;
   if (e->form == F3D_FORM_TC) {
-    const TcFwdArgs t = tc_forward_args(e, dsrc, pitch, fmt, spec);
+    TcFwdArgs t = tc_forward_args(e, dsrc, pitch, fmt, spec);
+    t.clk = e->d_clk;
     ce = launch_forward_tc_batch(&t, 1, e->tune, e->stream);
   } else {
+    FwdArgs a = forward_args(e, dsrc, pitch, fmt, spec);
+    a.clk = e->d_clk;
     ce = launch_forward(e->form, a, e->stream);
   }
-  cudaEventRecord(e->ev[1], e->stream);
   e->fwd_timed = true;
   if (ce != cudaSuccess) {
     e->cache.erase(fn);
@@ -329,19 +329,18 @@ int run_process(f3d_engine* e, const int* window, int n, uint8_t* ddst, long lon
   if (rc != F3D_OK) return rc;
   if (e->fused) {
     // The fused launch (tensor-core form: filter, then inverse) writes the packed plane.
-    const SweepArgs sa = sweep_args(e, a, ddst, pitch, fmt);
+    SweepArgs sa = sweep_args(e, a, ddst, pitch, fmt);
+    sa.clk = e->d_clk + 2;
+    sa.clk2 = e->d_clk + 4;
     e->test_skip = false;
-    cudaEventRecord(e->ev[2], e->stream);
-    cudaError_t ce = e->inv_form == F3D_FORM_TC ? launch_sweep_tc_batch(&sa, 1, e->tune, e->stream, e->ev[4])
-                                                : launch_sweep(e->inv_form, sa, e->stream, e->ev[4]);
-    cudaEventRecord(e->ev[3], e->stream);
+    cudaError_t ce = e->inv_form == F3D_FORM_TC ? launch_sweep_tc_batch(&sa, 1, e->tune, e->stream)
+                                                : launch_sweep(e->inv_form, sa, e->stream);
     e->proc_timed = true;
     if (ce != cudaSuccess) return e->cuda_fail(ce, "the fused filter/inverse/overlap-add launch");
     return F3D_OK;
   }
-  cudaEventRecord(e->ev[2], e->stream);
+  a.clk = e->d_clk + 2;
   cudaError_t ce = launch_filter_inverse(e->inv_form, a, e->stream);
-  cudaEventRecord(e->ev[4], e->stream);
   if (ce != cudaSuccess) return e->cuda_fail(ce, "the filter/inverse launch");
   if (a.kalman_init) e->kalman_first = false;
   OlaArgs o{};
@@ -353,11 +352,36 @@ int run_process(f3d_engine* e, const int* window, int n, uint8_t* ddst, long lon
   o.chroma_norm = e->cnorm;
   o.inv_norm = e->inv_norm;
   o.max_pix = e->max_pix;
+  o.clk = e->d_clk + 4;
   ce = launch_ola(o, e->stream);
-  cudaEventRecord(e->ev[3], e->stream);
   e->proc_timed = true;
   if (ce != cudaSuccess) return e->cuda_fail(ce, "the overlap-add launch");
   return F3D_OK;
+}
+
+constexpr int kClocks = 3;
+constexpr size_t kClockBytes = 2 * kClocks * sizeof(KernelClock);
+// Bytes of an engine's input plane and its clocks.
+size_t in_bytes(const f3d_plane_geom& g) { return ((size_t)g.width * g.height * 4 + 15) / 16 * 16 + kClockBytes; }
+
+// Milliseconds of n kernels from their clocks, read once the work queued on st
+// is done (wait: waited for; else false when it is not). -1 where a kernel has
+// not run.
+bool read_clocks(const KernelClock* d, int n, cudaStream_t st, bool wait, float* ms) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone ||
+      (wait ? cudaStreamSynchronize(st) : cudaStreamQuery(st)) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  KernelClock t[2 * kClocks];
+  if (cudaMemcpyAsync(t, d, 2 * n * sizeof(KernelClock), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+      cudaStreamSynchronize(st) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  for (int i = 0; i < n; i++) ms[i] = t[2 * i] && t[2 * i + 1] >= t[2 * i] ? (t[2 * i + 1] - t[2 * i]) * 1e-6f : -1.0f;
+  return true;
 }
 
 struct Lock {
@@ -498,10 +522,6 @@ int f3d_engine_create(const f3d_script_params* sp, const f3d_plane_geom* geom,
     if (ce != cudaSuccess) return finish_fail(e->cuda_fail(ce, "stream creation"));
     e->own_stream = true;
   }
-  for (auto& ev : e->ev) {
-    ce = cudaEventCreate(&ev);
-    if (ce != cudaSuccess) return finish_fail(e->cuda_fail(ce, "event creation"));
-  }
   const size_t bwbh = (size_t)ip.bw * ip.bh;
   const size_t plane_bytes = (size_t)g.width * g.height * 4;
   auto up = [&](float** d, const std::vector<float>& h) -> cudaError_t {
@@ -526,8 +546,11 @@ int f3d_engine_create(const f3d_script_params* sp, const f3d_plane_geom* geom,
         (ce = e->alloc(&e->d_err, sizeof(int))) != cudaSuccess || (ce = cudaMemset(e->d_err, 0, sizeof(int))) != cudaSuccess)
       return finish_fail(e->cuda_fail(ce, "tensor-core table upload"));
   }
-  if ((ce = e->alloc(&e->d_in, plane_bytes)) != cudaSuccess ||
-      (ce = e->alloc(&e->d_out, plane_bytes)) != cudaSuccess)
+  // The clocks stand behind the input plane.
+  if ((ce = e->alloc(&e->d_in, in_bytes(g))) != cudaSuccess || (ce = e->alloc(&e->d_out, plane_bytes)) != cudaSuccess)
+    return finish_fail(e->cuda_fail(ce, "buffer allocation"));
+  e->d_clk = reinterpret_cast<KernelClock*>(e->d_in + in_bytes(g) - kClockBytes);
+  if ((ce = cudaMemsetAsync(e->d_clk, 0, kClockBytes, e->stream)) != cudaSuccess)
     return finish_fail(e->cuda_fail(ce, "buffer allocation"));
   if (ip.bm == 0) {
     const size_t nbin = (size_t)e->grid.nb * e->ps;
@@ -593,7 +616,7 @@ void f3d_engine_destroy(f3d_engine* e) {
     e->release(e->d_sharpen, e->sharpen.size() * sizeof(float));
     e->release(e->d_gs, e->gs.size() * sizeof(float));
     const size_t plane_bytes = (size_t)e->geom.width * e->geom.height * 4;
-    e->release(e->d_in, plane_bytes);
+    e->release(e->d_in, in_bytes(e->geom));
     e->release(e->d_out, plane_bytes);
     e->release(e->d_blocks, sizeof(float) * (size_t)e->ip.bw * e->ip.bh * e->grid.nb);
     e->release(e->d_twr, e->tw_row.size() * sizeof(float));
@@ -604,8 +627,6 @@ void f3d_engine_destroy(f3d_engine* e) {
     e->release(e->d_kcov, sizeof(float) * nbin);
     e->release(e->d_kproc, sizeof(float) * nbin);
     e->release(e->d_seam, sizeof(float) * e->seam_floats);
-    for (auto& ev : e->ev)
-      if (ev) cudaEventDestroy(ev);
     if (e->own_stream && e->stream) cudaStreamDestroy(e->stream);
   }
   --g_live;
@@ -795,12 +816,15 @@ int f3d_last_kernel_ms(f3d_engine* e, float* ms) {
   if (!e || !ms) return fail_thread(F3D_E_PARAM, "FFT3DCL: null argument");
   Lock l(e);
   ms[0] = ms[1] = ms[2] = -1.0f;
-  if (e->fwd_timed) cudaEventElapsedTime(&ms[0], e->ev[0], e->ev[1]);
+  if (!e->fwd_timed && !e->proc_timed) return F3D_OK;
+  float t[kClocks];
+  if (!read_clocks(e->d_clk, kClocks, e->stream, false, t)) return F3D_OK;  // not finished yet
+  if (e->fwd_timed) ms[0] = t[0];
   if (e->proc_timed) {
-    cudaEventElapsedTime(&ms[1], e->ev[2], e->ev[4]);
-    cudaEventElapsedTime(&ms[2], e->ev[4], e->ev[3]);
+    ms[1] = t[1];
+    // The fused fast form has one kernel.
+    ms[2] = e->fused && e->inv_form != F3D_FORM_TC ? 0.0f : t[2];
   }
-  cudaGetLastError();
   return F3D_OK;
 }
 
@@ -828,9 +852,9 @@ struct f3d_batch {
   // Side stream of the forward when it does not feed this step's outputs.
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
-  // Kernel timing of the last step run outside a graph: before the filter,
-  // after it, after the inverse kernels.
-  cudaEvent_t kev[3] = {nullptr, nullptr, nullptr};
+  // Kernel times of the last step run outside a graph: filter (fast form: the
+  // fused sweep) and inverse.
+  KernelClock* clk = nullptr;
   bool ktimed = false;
   // Entries whose engine appeared earlier in the batch (one more output of
   // that plane per step) have operand tiles and seam rows of their own.
@@ -924,8 +948,7 @@ int f3d_batch_create(f3d_engine* const* engines, int n, int flags, f3d_batch** o
   if (cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreate(&b->kev[0]) != cudaSuccess || cudaEventCreate(&b->kev[1]) != cudaSuccess ||
-      cudaEventCreate(&b->kev[2]) != cudaSuccess) {
+      cudaMalloc(&b->clk, kClockBytes) != cudaSuccess || cudaMemset(b->clk, 0, kClockBytes) != cudaSuccess) {
     cudaGetLastError();
     f3d_batch_destroy(b);
     return fail_thread(F3D_E_CUDA, "FFT3DCL: batch stream creation failed");
@@ -953,8 +976,7 @@ void f3d_batch_destroy(f3d_batch* b) {
   }
   if (b->fork) cudaEventDestroy(b->fork);
   if (b->join) cudaEventDestroy(b->join);
-  for (cudaEvent_t ev : b->kev)
-    if (ev) cudaEventDestroy(ev);
+  if (b->clk) cudaFree(b->clk);
   if (b->side) cudaStreamDestroy(b->side);
   for (uint8_t* p : b->img)
     if (p) cudaFree(p);
@@ -1029,18 +1051,16 @@ int f3d_batch_step(f3d_batch* b, const int* fns, const void* const* dev_src, con
             if (windows[j][k] == fns[i]) overlap = false;
   if (overlap) mask |= 1ull << 32;
   if (!b->fast && nf > 0 && !tc_rows_aligned(fa, nf)) mask |= 1ull << 33;
-  // Filter and inverse; timed by events unless being captured.
+  // Filter and inverse; timed unless being captured.
   auto sweep = [&](const TcTune& t, cudaEvent_t after_filter) -> cudaError_t {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(b->stream, &cs);
     const bool timed = cs == cudaStreamCaptureStatusNone;
-    if (timed) cudaEventRecord(b->kev[0], b->stream);
-    cudaError_t ce = b->fast ? launch_sweep_fast_batch(sa, ns, b->stream, timed ? b->kev[1] : nullptr)
-                             : launch_sweep_tc_batch(sa, ns, t, b->stream, timed ? b->kev[1] : nullptr, after_filter);
-    if (timed && ce == cudaSuccess) {
-      cudaEventRecord(b->kev[2], b->stream);
-      b->ktimed = true;
-    }
+    sa[0].clk = timed ? b->clk : nullptr;
+    sa[0].clk2 = timed ? b->clk + 2 : nullptr;
+    const cudaError_t ce = b->fast ? launch_sweep_fast_batch(sa, ns, b->stream)
+                                   : launch_sweep_tc_batch(sa, ns, t, b->stream, after_filter);
+    if (timed && ce == cudaSuccess) b->ktimed = true;
     return ce;
   };
   auto forwards = [&](const TcTune& t, cudaStream_t st) -> cudaError_t {
@@ -1162,11 +1182,10 @@ int f3d_batch_last_kernel_ms(f3d_batch* b, float* ms) {
   if (!b || !ms) return fail_thread(F3D_E_PARAM, "FFT3DCL: null argument");
   if (!b->ktimed) return batch_fail(b, F3D_E_STATE, "FFT3DCL: no batch step with outputs ran outside a CUDA graph");
   cudaSetDevice(b->eng[0]->device);
-  cudaError_t ce = cudaEventSynchronize(b->kev[2]);
-  if (ce == cudaSuccess) ce = cudaEventElapsedTime(&ms[0], b->kev[0], b->kev[1]);
-  if (ce == cudaSuccess) ce = cudaEventElapsedTime(&ms[1], b->kev[1], b->kev[2]);
-  if (ce != cudaSuccess)
-    return batch_fail(b, F3D_E_CUDA, std::string("FFT3DCL: batch kernel timing: ") + cudaGetErrorString(ce));
+  float t[2];
+  if (!read_clocks(b->clk, 2, b->stream, true, t)) return batch_fail(b, F3D_E_CUDA, "FFT3DCL: batch kernel timing failed");
+  ms[0] = t[0];
+  ms[1] = b->fast ? 0.0f : t[1];  // the fused fast form has one kernel
   return F3D_OK;
 }
 
@@ -1256,7 +1275,7 @@ int engines_step(f3d_engine* const* eng, int n, const int* fns, const void* cons
   }
   cudaSetDevice(eng[0]->device);
   cudaError_t ce = nf ? launch_forward_tc_batch(fa, nf, TcTune{}, st) : cudaSuccess;
-  if (ce == cudaSuccess && ns) ce = launch_sweep_tc_batch(sa, ns, TcTune{}, st, nullptr);
+  if (ce == cudaSuccess && ns) ce = launch_sweep_tc_batch(sa, ns, TcTune{}, st);
   if (ce != cudaSuccess) return bad(F3D_E_CUDA, std::string("FFT3DCL: shared step launch: ") + cudaGetErrorString(ce));
   return F3D_OK;
 }

@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(kBigThreads) k_forward_big(const __grid_consta
   float2* buf = sm_big + w * kBigMax;
   float2* twr = sm_big + kBigWarps * kBigMax;
   float2* twc = twr + kBigMax / 2;
+  stamp_start(a.clk);
   load_twiddles(a.twr, a.twc, bw, bh, twr, twc);
   const int b = blockIdx.x;
   int bx, by, par;
@@ -114,6 +115,7 @@ __global__ void __launch_bounds__(kBigThreads) k_forward_big(const __grid_consta
     for (int r = lane; r < bh; r += 32) out[r * fbw + c] = buf[r];
     __syncwarp();
   }
+  stamp_end(a.clk);
 }
 
 // One block: temporal filter + sharpen per bin into the block's work area
@@ -128,6 +130,7 @@ __global__ void __launch_bounds__(kBigThreads) k_inverse_big(const __grid_consta
   float2* buf = sm_big + w * kBigMax;
   float2* twr = sm_big + kBigWarps * kBigMax;
   float2* twc = twr + kBigMax / 2;
+  stamp_start(a.clk);
   load_twiddles(a.twr, a.twc, bw, bh, twr, twc);
   const int b = blockIdx.x;
   float2* F = a.work + (size_t)b * bh * bw;
@@ -169,6 +172,7 @@ __global__ void __launch_bounds__(kBigThreads) k_inverse_big(const __grid_consta
     for (int x = lane; x < bw; x += 32) out[r * bw + x] = buf[x].x * win[r * bw + x];
     __syncwarp();
   }
+  stamp_end(a.clk);
 }
 
 constexpr size_t kBigSmem = sizeof(float2) * (kBigWarps * kBigMax + kBigMax);

@@ -48,7 +48,8 @@ __global__ void __launch_bounds__(256) k_ola(const __grid_constant__ OlaArgs a) 
   const int x = (blockIdx.x * 32 + (threadIdx.x & 31)) * V;
   const int y = blockIdx.y * 8 + (threadIdx.x >> 5);
   const Geo& g = a.g;
-  if (x >= g.W || y >= g.H) return;
+  stamp_start(a.clk);
+  if (x >= g.W || y >= g.H) return;  // not thread 0
   const int bsz = g.bw * g.bh;
   float sum[V];
 #pragma unroll
@@ -98,6 +99,7 @@ __global__ void __launch_bounds__(256) k_ola(const __grid_constant__ OlaArgs a) 
     for (int k = 0; k < V; k++) sum[k] += a.chroma_norm;
   if constexpr (V == 4) store_quad(a.dst + (long long)y * a.pitch, x, g.W, sum, a.fmt, a.inv_norm, a.max_pix);
   else store_sample(a.dst + (long long)y * a.pitch, x, sum[0], a.fmt, a.inv_norm, a.max_pix);
+  stamp_end(a.clk);
 }
 
 }  // namespace

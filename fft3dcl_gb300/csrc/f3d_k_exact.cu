@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(Cfg<BW, BH>::THREADS, Cfg<BW, BH>::FWD_CTAS)
   float2* rows = reinterpret_cast<float2*>(tile);
   float2* out = a.spec + (size_t)b * C::PS;
 
+  stamp_start(a.clk);
   if (valid) gather_block<BW, BH, C::TPB, C::GB, C::TS>(a, b, t, tile);
   block_sync<C::TPB>();
   static_assert(C::TPB >= BH && C::TPB >= C::FBW, "one row, one column per thread");
@@ -143,6 +144,7 @@ __global__ void __launch_bounds__(Cfg<BW, BH>::THREADS, Cfg<BW, BH>::FWD_CTAS)
 #pragma unroll
     for (int r = 0; r < BH; r++) out[r * C::FBW + t] = v[r];
   }
+  stamp_end(a.clk);
 }
 
 // The filtered half spectrum of block b (temporal filter + sharpen per bin,
@@ -240,6 +242,7 @@ __global__ void __launch_bounds__(Cfg<BW, BH>::THREADS, Cfg<BW, BH>::INV_CTAS - 
   float2* F = reinterpret_cast<float2*>(smem + slot * C::INV_FLOATS);
   float2* G = F;
 
+  stamp_start(a.clk);
   if (!KALMAN && valid && t == 0) prefetch_window<C::PS>(a, b);
   if (valid) filter_block_any<KALMAN, BW == BH, C::PS, C::TPB, C::KB>(a, b, t, F);
   block_sync<C::TPB>();
@@ -273,6 +276,7 @@ __global__ void __launch_bounds__(Cfg<BW, BH>::THREADS, Cfg<BW, BH>::INV_CTAS - 
   }
   block_sync<C::TPB>();
   if (valid) store_block<BW, BH, C::TPB, C::TS>(a, b, t, G, [](int j) { return j; });
+  stamp_end(a.clk);
 }
 
 // ---- 64 x 64 blocks: each 64-point transform on a lane pair ----------------
@@ -353,6 +357,7 @@ __global__ void __launch_bounds__(kPairThreads, 6) k_forward_exact64(const __gri
   const int t = threadIdx.x, p = t >> 1;
   const bool odd = t & 1;
   const int b = blockIdx.x;
+  stamp_start(a.clk);
   gather_block<64, 64, kPairThreads, 16, kPairTS>(a, b, t, tile);
   __syncthreads();
   float2 r[32];
@@ -376,6 +381,7 @@ __global__ void __launch_bounds__(kPairThreads, 6) k_forward_exact64(const __gri
       float2* out = a.spec + (size_t)b * 64 * FBW + c;
 #pragma unroll
       for (int q = 0; q < 32; q++) out[(32 * odd + q) * FBW] = r[q];
+      stamp_end(a.clk);  // in here: behind the branches it made the registers spill
     }
   }
 }
@@ -393,6 +399,7 @@ __global__ void __launch_bounds__(kPairThreads, 5) k_inverse_exact64(const __gri
   const int t = threadIdx.x, p = t >> 1;
   const bool odd = t & 1;
   const int b = blockIdx.x;
+  stamp_start(a.clk);
   if (!KALMAN && t == 0) prefetch_window<PS>(a, b);
   filter_block_any<KALMAN, true, PS, kPairThreads, 6>(a, b, t, F);
   __syncthreads();
@@ -426,6 +433,7 @@ __global__ void __launch_bounds__(kPairThreads, 5) k_inverse_exact64(const __gri
   for (int q = 0; q < 16; q++) G[p * kPairTS + kOddAt * odd + q] = make_float2(r[2 * q].x, r[2 * q + 1].x);
   __syncthreads();
   store_block<64, 64, kPairThreads, kPairTS>(a, b, t, G, [](int j) { return j < 16 ? j : j + (kOddAt - 16); });
+  stamp_end(a.clk);
 }
 
 cudaError_t launch_fwd64(const FwdArgs& a, cudaStream_t st) {

@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(128) k_forward_fast(const __grid_constant__ Fw
   float2* S = reinterpret_cast<float2*>(smem4) + slot * C::SMEM_F2;
   float* tile = reinterpret_cast<float*>(S);  // input tile [BH][TS], aliased with S
 
+  stamp_start(a.clk);
   if (valid) gather_block<BW, BH, C::TPB, C::TS>(a, b, t, tile);
   __syncwarp();
   float2 z[BW];
@@ -164,6 +165,7 @@ __global__ void __launch_bounds__(128) k_forward_fast(const __grid_constant__ Fw
       for (int r = 0; r < BH; r++) out[r * C::FBW + t] = y[r];
     }
   }
+  stamp_end(a.clk);
 }
 
 template <int BW, int BH, int BM>
@@ -180,6 +182,7 @@ __global__ void __launch_bounds__(128) k_inverse_fast(const __grid_constant__ In
   const float* win = par ? a.win_b : a.win_a;
   float* out = a.blocks + (size_t)b * BW * BH;
   constexpr float inv_n = 1.0f / (BW * BH);
+  stamp_start(a.clk);
   inverse_block<BW, BH, BM>(a, b, t, valid, S, [&](int y, const float2(&xy)[BW / 2]) {
 #pragma unroll
     for (int n = 0; n < BW / 2; n += 2) {
@@ -189,6 +192,7 @@ __global__ void __launch_bounds__(128) k_inverse_fast(const __grid_constant__ In
                       xy[n + 1].y * inv_n * wv.w);
     }
   }, [] {});
+  stamp_end(a.clk);
 }
 
 // ---- square blocks ---------------------------------------------------------
@@ -219,6 +223,7 @@ __global__ void __launch_bounds__(kPairThreads, kPairFwdCtas<N>) k_forward_fast_
   const bool valid = b < a.g.nb;
   float2* S = reinterpret_cast<float2*>(smem4) + slot * C::SMEM_F2;
   float* tile = reinterpret_cast<float*>(S);  // input tile [N][TS], aliased with S
+  stamp_start(a.clk);
   if (valid) gather_block<N, N, N, C::TS>(a, b, t, tile);
   pair_sync<N>();
   float2 z[H];
@@ -267,6 +272,7 @@ __global__ void __launch_bounds__(kPairThreads, kPairFwdCtas<N>) k_forward_fast_
 #pragma unroll
     for (int i = 0; i < H; i++) out[i * FBW + p] = z[i];
   }
+  stamp_end(a.clk);
 }
 
 template <int N>
@@ -300,6 +306,7 @@ __global__ void __launch_bounds__(kPairThreads, 12) k_inverse_fast64(const __gri
   float2* S = reinterpret_cast<float2*>(smem4);
   const int t = threadIdx.x, c = t >> 1, h = t & 1, b = blockIdx.x;
   const size_t base = (size_t)b * C::PS;
+  stamp_start(a.clk);
   {
     constexpr int NF = BM >= 2 ? BM : 1;
     if (t < NF) prefetch_l2(a.s[t] + base, C::PS * sizeof(float2));
@@ -380,6 +387,7 @@ __global__ void __launch_bounds__(kPairThreads, 12) k_inverse_fast64(const __gri
     const float2 v = S[(i % H) * SB + yperm<64>(i / H)], w = win[i];
     out[i] = make_float2(v.x * inv_n * w.x, v.y * inv_n * w.y);
   }
+  stamp_end(a.clk);
 }
 
 template <int BM>
@@ -403,11 +411,12 @@ __global__ void __launch_bounds__(kThreads) k_inverse_fast_sq(const __grid_const
   const int b = blockIdx.x * BPC + slot;
   const bool valid = b < a.g.nb;
   float2* S = reinterpret_cast<float2*>(smem4) + slot * C::SMEM_F2;
+  stamp_start(a.clk);
   inverse_block_sq<N, BM, 4>(a, a, b, t, valid, S, [&](int y, const float2(&xy)[N / 2]) {
 #pragma unroll
     for (int k = 0; k < N / 2; k++) S[k * SB + yperm<N>(y)] = xy[k];
   }, [] {});
-  if (!valid) return;
+  if (!valid) return;  // not thread 0
   int bx, by, par;
   block_origin(a.g, b, bx, by, par);
   const float2* win = reinterpret_cast<const float2*>(par ? a.win_b : a.win_a);
@@ -418,6 +427,7 @@ __global__ void __launch_bounds__(kThreads) k_inverse_fast_sq(const __grid_const
     const float2 v = S[(i % (N / 2)) * SB + yperm<N>(i / (N / 2))], w = win[i];
     out[i] = make_float2(v.x * inv_n * w.x, v.y * inv_n * w.y);
   }
+  stamp_end(a.clk);
 }
 
 template <int N, int BM>

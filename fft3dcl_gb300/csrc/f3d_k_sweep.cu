@@ -182,7 +182,9 @@ __global__ void __launch_bounds__(kSweepThreads, F3D_SWEEP_MINB) k_sweep_fast(co
   while (p + 1 < B.n && (int)blockIdx.x >= B.cta0[p + 1]) p++;
   const int r0 = B.run[p], rl = B.rlen[r0];
   const int local = (int)blockIdx.x - B.cta0[r0];
+  stamp_start(B.p[0].clk);
   sweep_fast_cta<BW, BH, BM, SW>(B.p[r0 + local % rl], local / rl);
+  stamp_end(B.p[0].clk);
 }
 
 template <int BW, int BH, int BM, int SW>
@@ -221,7 +223,7 @@ cudaError_t launch_size(const SweepBatch& Bs, cudaStream_t st) {
 
 }  // namespace
 
-cudaError_t launch_sweep_fast_batch(const SweepArgs* planes, int n, cudaStream_t st, cudaEvent_t mark) {
+cudaError_t launch_sweep_fast_batch(const SweepArgs* planes, int n, cudaStream_t st) {
   if (n < 1 || n > kMaxBatch) return cudaErrorInvalidValue;
   SweepArgs p[kMaxBatch];
   std::copy(planes, planes + n, p);
@@ -235,9 +237,7 @@ cudaError_t launch_sweep_fast_batch(const SweepArgs* planes, int n, cudaStream_t
   case 32: e = launch_size<32, 32>(Bs, st); break;
   default: return cudaErrorNotSupported;
   }
-  if (e != cudaSuccess) return e;
-  if (mark) cudaEventRecord(mark, st);
-  return cudaSuccess;
+  return e;
 }
 
 bool sweep_supported(int form, const Geo& g, int bm) {
@@ -269,10 +269,10 @@ size_t sweep_seam_floats(const Geo& g, int strips, int segs) {
   return (size_t)(segs > 1 ? segs - 1 : 0) * (3 * (g.bh / 2) * (size_t)cells_x * (g.bw / 2) + strips);
 }
 
-cudaError_t launch_sweep(int form, const SweepArgs& a, cudaStream_t st, cudaEvent_t mark) {
+cudaError_t launch_sweep(int form, const SweepArgs& a, cudaStream_t st) {
   if (!sweep_supported(form, a.inv.g, a.inv.bm)) return cudaErrorNotSupported;
-  if (form == F3D_FORM_TC) return launch_sweep_tc(a, st, mark);
-  return launch_sweep_fast_batch(&a, 1, st, mark);
+  if (form == F3D_FORM_TC) return launch_sweep_tc(a, st);
+  return launch_sweep_fast_batch(&a, 1, st);
 }
 
 }  // namespace f3d

@@ -373,6 +373,7 @@ __global__ void __launch_bounds__(kTcThreads, fwd_ctas(SPLIT, ALIGNED, BPS)) k_f
   float2* stage = reinterpret_cast<float2*>(sm + L::STAGE);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
+  stamp_start(B.p[0].clk);
   const int ngroups = B.grp0[B.n];
   uint32_t phase = 0;
   RawGroup<N, BPS, ALIGNED> raw;
@@ -586,6 +587,7 @@ __global__ void __launch_bounds__(kTcThreads, fwd_ctas(SPLIT, ALIGNED, BPS)) k_f
     }
   }
   if (tid == 0) tc::bulk_wait_read();  // the shared memory outlives the copies out of it
+  stamp_end(B.p[0].clk);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -835,6 +837,7 @@ __global__ void __launch_bounds__(kTcThreads, MINB) k_filter_tc(const __grid_con
   const int local = (int)blockIdx.x - B.cta0[r0];
   const int pl = r0 + local % rl;
   const FilterPlane& P = B.p[pl];
+  stamp_start(B.clk);
   FilterArgs a = P.f;
   fix_switches<SW>(a);
   extern __shared__ __align__(128) uint8_t smem_f[];
@@ -868,6 +871,7 @@ __global__ void __launch_bounds__(kTcThreads, MINB) k_filter_tc(const __grid_con
     tc::bulk_commit();
     tc::bulk_wait_read();
   }
+  stamp_end(B.clk);
 }
 
 // Shared-memory and barrier state of the inverse phases of one CTA.
@@ -1082,6 +1086,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcSweepCtasPerSm) k_sweep_tc(cons
   uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + S::TSLOT);
   const int tid = threadIdx.x, warp = tid >> 5;
 
+  stamp_start(B.p[0].clk2);
   const int pl = plane_of(B, B.cta0, blockIdx.x);
   const SweepArgs& sa = B.p[pl];
   const int cta = blockIdx.x - B.cta0[pl];
@@ -1138,6 +1143,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcSweepCtasPerSm) k_sweep_tc(cons
   if (warp == 0) tc::tmem_dealloc(st.tmem, C::TMEM_COLS);
   // The partial sums are done with: two ints of them for the seams.
   finish_seams<S::CH, S::CW>(sa, strip, seg, J0, ncell, reinterpret_cast<int*>(sm + S::P));
+  stamp_end(B.p[0].clk2);
 }
 
 template <class K>
@@ -1373,8 +1379,7 @@ FilterLaunch filter_launch(const SweepBatch& S, int minb, FilterBatch& F) {
 namespace {
 
 template <int N>
-cudaError_t launch_sweep_n(const SweepBatch& B, int n, const TcTune& t, cudaStream_t st, cudaEvent_t mark,
-                           cudaEvent_t after_filter) {
+cudaError_t launch_sweep_n(const SweepBatch& B, int n, const TcTune& t, cudaStream_t st, cudaEvent_t after_filter) {
   using S = SwpCfg<N>;
   constexpr size_t smem = S::BYTES;
   static_assert(kTcSweepCtasPerSm * (S::BYTES + 1024) <= 228 * 1024, "CTAs per SM");
@@ -1390,7 +1395,6 @@ cudaError_t launch_sweep_n(const SweepBatch& B, int n, const TcTune& t, cudaStre
     if (e != cudaSuccess) return e;
     count_launch();
   }
-  if (mark) cudaEventRecord(mark, st);
   if (after_filter && (e = cudaEventRecord(after_filter, st)) != cudaSuccess) return e;
   // Inverse + overlap-add: one CTA per (strip, segment) of every plane.
   e = prepare(k_sweep_tc<N>, smem);
@@ -1414,17 +1418,17 @@ cudaError_t tc_sweep_batch(const SweepArgs* planes, int n, SweepBatch& B) {
 }  // namespace
 
 cudaError_t launch_sweep_tc_batch(const SweepArgs* planes, int n, const TcTune& t, cudaStream_t st,
-                                  cudaEvent_t mark, cudaEvent_t after_filter) {
+                                  cudaEvent_t after_filter) {
   SweepBatch B;
   const cudaError_t e = tc_sweep_batch(planes, n, B);
   if (e != cudaSuccess) return e;
   static_assert(SwpCfg<32>::TJ == 7 && SwpCfg<16>::TJ == 15, "cells per strip");
-  return planes[0].inv.g.bw == 16 ? launch_sweep_n<16>(B, n, t, st, mark, after_filter)
-                                  : launch_sweep_n<32>(B, n, t, st, mark, after_filter);
+  return planes[0].inv.g.bw == 16 ? launch_sweep_n<16>(B, n, t, st, after_filter)
+                                  : launch_sweep_n<32>(B, n, t, st, after_filter);
 }
 
-cudaError_t launch_sweep_tc(const SweepArgs& a, cudaStream_t st, cudaEvent_t mark) {
-  return launch_sweep_tc_batch(&a, 1, TcTune{}, st, mark);
+cudaError_t launch_sweep_tc(const SweepArgs& a, cudaStream_t st) {
+  return launch_sweep_tc_batch(&a, 1, TcTune{}, st);
 }
 
 cudaError_t tc_graph_update(cudaGraphExec_t exec, cudaGraph_t graph, const TcFwdArgs* fwd, int nf,

@@ -20,6 +20,10 @@ struct Geo {
   int xoff, xstep, yoff, ystep;
 };
 
+// Device times of a kernel: [0] when its first CTA started, [1] when its last
+// one ended, in nanoseconds of the GPU's global timer. Null: not timed.
+using KernelClock = unsigned long long;
+
 // Sample formats of the raw planes.
 enum Fmt : int { FMT_F32 = 0, FMT_U8 = 8, FMT_U16 = 16 };
 
@@ -43,6 +47,7 @@ struct FwdArgs {
   float2* spec;        // out: nb x bh x fbw half spectra
   const float2* twr;   // blocks above 64: device twiddles, bw/2 and bh/2 entries
   const float2* twc;
+  KernelClock* clk;
 };
 
 // The temporal filter of one output.
@@ -78,6 +83,7 @@ struct InvArgs : FilterArgs {
   const float2* twr;   // blocks above 64: device twiddles, bw/2 and bh/2 entries,
   const float2* twc;   //   and nb x bh x bw complex work space
   float2* work;
+  KernelClock* clk;    // of the inverse kernel
 };
 
 struct OlaArgs {
@@ -87,6 +93,7 @@ struct OlaArgs {
   long long pitch;
   int fmt;
   float chroma_norm, inv_norm, max_pix;
+  KernelClock* clk;
 };
 
 // Fused filter + inverse + overlap-add + packing for mode 1 with half
@@ -114,6 +121,8 @@ struct SweepArgs {
   int* err;              // tensor-core form: bits set when a wait gives up (kErrWait*)
   uint8_t* img;          // tensor-core form: filtered column-inverse operands, one image per block
   int test_skip;         // tests only: the plane's first CTA skips its first operand-tile copy
+  KernelClock* clk;      // of the fast form's sweep or the tensor-core filter (of a batch: the first plane's)
+  KernelClock* clk2;     // of the tensor-core inverse
 };
 
 // Bits of the tensor-core kernels' error word: which wait gave up.
@@ -137,9 +146,7 @@ inline void set_seams(SweepArgs& sa, float* scratch, int max_segs) {
   sa.seam_t = scratch ? scratch + rows : nullptr;
   sa.seam_cnt = scratch ? reinterpret_cast<int*>(scratch + 3 * rows) : nullptr;
 }
-// `mark` (optional) is recorded after the first kernel: the fast-form sweep,
-// or the tensor-core filter kernel.
-cudaError_t launch_sweep(int form, const SweepArgs& a, cudaStream_t st, cudaEvent_t mark = nullptr);
+cudaError_t launch_sweep(int form, const SweepArgs& a, cudaStream_t st);
 
 // Kernel launches; each returns the launch error. `form` is F3D_FORM_*.
 cudaError_t launch_forward(int form, const FwdArgs& a, cudaStream_t st);
@@ -185,6 +192,7 @@ struct TcFwdArgs {
   float2* spec;        // out: nb x bh x fbw half spectra (__half2 pairs when half)
   int half;            // store the spectra as fp16 pairs
   int* err;            // kErrWaitForward set when a tensor-core wait gives up
+  KernelClock* clk;    // of a batch: the first plane's
 };
 bool tc_supported(int mode, int bw, int bh, int bm);
 // DFT matrices (fp16 hi/lo, in the kernels' shared-memory operand layout)
@@ -233,6 +241,7 @@ struct FilterBatch {
   int cta0[kMaxBatch + 1];
   int run[kMaxBatch], rlen[kMaxBatch];
   int shifted;
+  KernelClock* clk;
   FilterPlane p[kMaxBatch];
 };
 // Launch shape of the tensor-core kernels, picked by the autotuner.
@@ -241,10 +250,10 @@ struct TcTune {
   int filter_minb = 5;      // filter kernel variant: 5, 4 or 3 CTAs per SM (spectra loads of 1, 2, 2 blocks in flight)
 };
 cudaError_t launch_forward_tc_batch(const TcFwdArgs* planes, int n, const TcTune& t, cudaStream_t st);
-// mark and after_filter (either may be null) are recorded on st between the
-// filter and the inverse kernels.
+// after_filter (may be null) is recorded on st between the filter and the
+// inverse kernels.
 cudaError_t launch_sweep_tc_batch(const SweepArgs* planes, int n, const TcTune& t, cudaStream_t st,
-                                  cudaEvent_t mark, cudaEvent_t after_filter = nullptr);
+                                  cudaEvent_t after_filter = nullptr);
 // Whether the blocks of every plane start on 16 bytes in every row: the
 // forward has a kernel for such planes and one for any.
 bool tc_rows_aligned(const TcFwdArgs* planes, int n);
@@ -257,10 +266,10 @@ cudaError_t tc_graph_update(cudaGraphExec_t exec, cudaGraph_t graph, const TcFwd
 // inverse + overlap-add).
 int tc_sweep_cells(int n);  // 7 for 32 x 32 blocks, 15 for 16 x 16
 constexpr int kTcSweepCtasPerSm = 3;
-cudaError_t launch_sweep_tc(const SweepArgs& a, cudaStream_t st, cudaEvent_t mark);
+cudaError_t launch_sweep_tc(const SweepArgs& a, cudaStream_t st);
 // The fast form's fused sweeps of n planes (8x8 to 32x32 blocks, one
-// temporal mode) in one launch; `mark` is recorded after it.
-cudaError_t launch_sweep_fast_batch(const SweepArgs* planes, int n, cudaStream_t st, cudaEvent_t mark);
+// temporal mode) in one launch.
+cudaError_t launch_sweep_fast_batch(const SweepArgs* planes, int n, cudaStream_t st);
 // Bytes of SweepArgs::img for this geometry.
 size_t tc_image_bytes(const Geo& g);
 

@@ -240,7 +240,7 @@ const VSFrame* VS_CC get_frame(int n, int reason, void* data, void**, VSFrameCon
       return nullptr;
     }
     if (time_on()) {
-      // The readback has completed, so the engine's events are: the last
+      // The readback has completed, and with it the engine's kernels: the last
       // forward (this frame's, when one ran) and this output's kernels.
       float ms[3];
       if (f3d_last_kernel_ms(e, ms) == F3D_OK) {

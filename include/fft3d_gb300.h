@@ -208,13 +208,14 @@ int f3d_prune(f3d_engine* e, int lo, int hi);
  * kernel's bounded wait gave up since the last call (the message names the
  * wait; the outputs queued since are invalid); the report clears it. */
 int f3d_synchronize(f3d_engine* e);
-/* Device time of the kernels of the last forward / process calls in ms
- * (CUDA events on the engine stream; valid after f3d_synchronize):
+/* Device time of the kernels of the last forward / process calls in ms,
+ * taken by the kernels on the GPU's global timer (valid after f3d_synchronize;
+ * -1 while the engine's stream has work queued):
  * ms[0] forward transform;
  * ms[1] filter + inverse (separate kernels), the whole sweep (fused fast
  *       form) or the filter kernel (tensor-core form);
- * ms[2] overlap-add + pack (separate kernels), the seam merge (fused fast
- *       form) or inverse + overlap-add + seam merge (tensor-core form). */
+ * ms[2] overlap-add + pack (separate kernels), 0 (fused fast form, one
+ *       kernel) or inverse + overlap-add (tensor-core form). */
 int f3d_last_kernel_ms(f3d_engine* e, float* ms);
 
 /* GpuRef::liveInstances / liveBytes (src/cl/gpu.cpp:44-57). */
@@ -300,8 +301,8 @@ int f3d_batch_tune(f3d_batch* b, int* fwd_ctas_per_sm, int* filter_minb);
 int f3d_batch_set_tune(f3d_batch* b, int fwd_ctas_per_sm, int filter_minb);
 /* Device times (ms) of the last step with outputs that ran outside a CUDA
  * graph (steps replayed as a graph are not timed): ms[0] the filter kernel,
- * ms[1] the inverse + overlap-add kernel and the seam merge (fast form:
- * ms[0] the fused sweep, ms[1] the seam merge). Waits for that step.
+ * ms[1] the inverse + overlap-add kernel (fast form: ms[0] the fused sweep,
+ * ms[1] 0). Waits for that step.
  * F3D_E_STATE when no such step ran. */
 int f3d_batch_last_kernel_ms(f3d_batch* b, float* ms);
 
