@@ -31,6 +31,13 @@ __host__ __device__ constexpr int bit_reverse(int i, int bits) {
   return r;
 }
 
+// Every kernel: grid_wait before the first access to memory that another
+// kernel writes or reads (launch_kernel), grid_go as early as its CTAs hold
+// what they need to finish; in the kernels with tensor memory after its
+// allocation, which a successor's waiting CTA could otherwise take first.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // A kernel's times, taken by its own threads (thread 0 of the first CTA, then
 // of every CTA): events around the kernels would keep each from starting until
 // the one before has ended and its time is written, about 2 us an event.
@@ -39,7 +46,7 @@ __device__ __forceinline__ KernelClock device_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-__device__ __forceinline__ void stamp_start(KernelClock* clk) {
+__device__ __forceinline__ void stamp_start(KernelClock* clk) {  // after grid_wait
   if (clk && (blockIdx.x | blockIdx.y | threadIdx.x) == 0) clk[0] = device_ns();
 }
 __device__ __forceinline__ void stamp_end(KernelClock* clk) {

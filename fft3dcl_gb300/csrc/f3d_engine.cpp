@@ -1102,7 +1102,11 @@ int f3d_batch_step(f3d_batch* b, const int* fns, const void* const* dev_src, con
   // 1-3 % slower in steady state at eight and ten outputs.
   const uint64_t all = (1ull << n) - 1;
   if (!b->fast && (b->flags & F3D_BATCH_AUTOTUNE) && !b->tuned && (mask & 0xFFFFFFFFull) == (all | (all << 16))) {
-    const TcTune cands[] = {{3, 5}, {2, 5}, {1, 5}, {3, 4}, {2, 4}, {1, 4}};
+    // Both filter variants, with the forward kernel on as many CTAs as fit: on
+    // two or one per SM a step was never faster, only picked by that noise (three
+    // 1080p planes {3,5} 111.7, {3,4} 111.5, {2,5} 115, {1,5} 133 us; ten 10-bit
+    // 4K outputs 1390, 1437, 1558, 1974 us).
+    const TcTune cands[] = {{3, 5}, {3, 4}};
     constexpr int kCands = sizeof(cands) / sizeof(cands[0]);
     cudaEvent_t t0, t1;
     cudaEventCreate(&t0);

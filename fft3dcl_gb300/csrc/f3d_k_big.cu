@@ -85,6 +85,8 @@ __global__ void __launch_bounds__(kBigThreads) k_forward_big(const __grid_consta
   float2* buf = sm_big + w * kBigMax;
   float2* twr = sm_big + kBigWarps * kBigMax;
   float2* twc = twr + kBigMax / 2;
+  grid_go();
+  grid_wait();
   stamp_start(a.clk);
   load_twiddles(a.twr, a.twc, bw, bh, twr, twc);
   const int b = blockIdx.x;
@@ -130,6 +132,8 @@ __global__ void __launch_bounds__(kBigThreads) k_inverse_big(const __grid_consta
   float2* buf = sm_big + w * kBigMax;
   float2* twr = sm_big + kBigWarps * kBigMax;
   float2* twc = twr + kBigMax / 2;
+  grid_go();
+  grid_wait();
   stamp_start(a.clk);
   load_twiddles(a.twr, a.twc, bw, bh, twr, twc);
   const int b = blockIdx.x;
@@ -184,17 +188,13 @@ bool big_block(int bw, int bh) { return bw > 64 || bh > 64; }
 cudaError_t launch_forward_big(const FwdArgs& a, cudaStream_t st) {
   if (a.g.bw > kBigMax || a.g.bh > kBigMax || !a.twr || !a.twc) return cudaErrorInvalidValue;
   if (a.g.nb == 0) return cudaSuccess;
-  k_forward_big<<<a.g.nb, kBigThreads, kBigSmem, st>>>(a);
-  count_launch();
-  return cudaGetLastError();
+  return launch_kernel(k_forward_big, a.g.nb, kBigThreads, kBigSmem, st, a);
 }
 
 cudaError_t launch_inverse_big(const InvArgs& a, cudaStream_t st) {
   if (a.g.bw > kBigMax || a.g.bh > kBigMax || !a.twr || !a.twc || !a.work) return cudaErrorInvalidValue;
   if (a.g.nb == 0) return cudaSuccess;
-  k_inverse_big<<<a.g.nb, kBigThreads, kBigSmem, st>>>(a);
-  count_launch();
-  return cudaGetLastError();
+  return launch_kernel(k_inverse_big, a.g.nb, kBigThreads, kBigSmem, st, a);
 }
 
 }  // namespace f3d

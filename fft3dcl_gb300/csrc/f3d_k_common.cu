@@ -48,6 +48,8 @@ __global__ void __launch_bounds__(256) k_ola(const __grid_constant__ OlaArgs a) 
   const int x = (blockIdx.x * 32 + (threadIdx.x & 31)) * V;
   const int y = blockIdx.y * 8 + (threadIdx.x >> 5);
   const Geo& g = a.g;
+  grid_go();
+  grid_wait();
   stamp_start(a.clk);
   if (x >= g.W || y >= g.H) return;  // not thread 0
   const int bsz = g.bw * g.bh;
@@ -109,10 +111,7 @@ cudaError_t launch_ola(const OlaArgs& a, cudaStream_t st) {
   const bool quads = a.g.mode == 1 && a.g.bw % 4 == 0 && a.g.xoff % 4 == 0 && a.g.xstep % 4 == 0;
   const int v = quads ? 4 : 1;
   dim3 grid((a.g.W + 32 * v - 1) / (32 * v), (a.g.H + 7) / 8);
-  if (quads) k_ola<4><<<grid, 256, 0, st>>>(a);
-  else k_ola<1><<<grid, 256, 0, st>>>(a);
-  count_launch();
-  return cudaGetLastError();
+  return launch_kernel(quads ? k_ola<4> : k_ola<1>, grid, 256, 0, st, a);
 }
 
 static bool pow2_in(int v, int lo, int hi) { return v >= lo && v <= hi && (v & (v - 1)) == 0; }

@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(Cfg<BW, BH>::THREADS, Cfg<BW, BH>::FWD_CTAS)
   float2* rows = reinterpret_cast<float2*>(tile);
   float2* out = a.spec + (size_t)b * C::PS;
 
+  grid_go();
+  grid_wait();
   stamp_start(a.clk);
   if (valid) gather_block<BW, BH, C::TPB, C::GB, C::TS>(a, b, t, tile);
   block_sync<C::TPB>();
@@ -242,6 +244,8 @@ __global__ void __launch_bounds__(Cfg<BW, BH>::THREADS, Cfg<BW, BH>::INV_CTAS - 
   float2* F = reinterpret_cast<float2*>(smem + slot * C::INV_FLOATS);
   float2* G = F;
 
+  grid_go();
+  grid_wait();
   stamp_start(a.clk);
   if (!KALMAN && valid && t == 0) prefetch_window<C::PS>(a, b);
   if (valid) filter_block_any<KALMAN, BW == BH, C::PS, C::TPB, C::KB>(a, b, t, F);
@@ -357,6 +361,8 @@ __global__ void __launch_bounds__(kPairThreads, 6) k_forward_exact64(const __gri
   const int t = threadIdx.x, p = t >> 1;
   const bool odd = t & 1;
   const int b = blockIdx.x;
+  grid_go();
+  grid_wait();
   stamp_start(a.clk);
   gather_block<64, 64, kPairThreads, 16, kPairTS>(a, b, t, tile);
   __syncthreads();
@@ -399,6 +405,8 @@ __global__ void __launch_bounds__(kPairThreads, 5) k_inverse_exact64(const __gri
   const int t = threadIdx.x, p = t >> 1;
   const bool odd = t & 1;
   const int b = blockIdx.x;
+  grid_go();
+  grid_wait();
   stamp_start(a.clk);
   if (!KALMAN && t == 0) prefetch_window<PS>(a, b);
   filter_block_any<KALMAN, true, PS, kPairThreads, 6>(a, b, t, F);
@@ -440,9 +448,7 @@ cudaError_t launch_fwd64(const FwdArgs& a, cudaStream_t st) {
   const size_t smem = sizeof(float2) * 64 * 33 > sizeof(float) * 64 * kPairTS ? sizeof(float2) * 64 * 33
                                                                                : sizeof(float) * 64 * kPairTS;
   if (a.g.nb == 0) return cudaSuccess;
-  k_forward_exact64<<<a.g.nb, kPairThreads, smem, st>>>(a);
-  count_launch();
-  return cudaGetLastError();
+  return launch_kernel(k_forward_exact64, a.g.nb, kPairThreads, smem, st, a);
 }
 
 cudaError_t launch_inv64(const InvArgs& a, cudaStream_t st) {
@@ -453,9 +459,7 @@ cudaError_t launch_inv64(const InvArgs& a, cudaStream_t st) {
     if (e != cudaSuccess) return e;
   }
   if (a.g.nb == 0) return cudaSuccess;
-  k<<<a.g.nb, kPairThreads, smem, st>>>(a);
-  count_launch();
-  return cudaGetLastError();
+  return launch_kernel(k, a.g.nb, kPairThreads, smem, st, a);
 }
 
 template <int BW, int BH>
@@ -472,9 +476,7 @@ cudaError_t launch_fwd(const FwdArgs& a, cudaStream_t st) {
     }
     const int grid = (a.g.nb + C::BPC - 1) / C::BPC;
     if (grid == 0) return cudaSuccess;
-    k<<<grid, C::THREADS, smem, st>>>(a);
-    count_launch();
-    return cudaGetLastError();
+    return launch_kernel(k, grid, C::THREADS, smem, st, a);
   }
 }
 
@@ -492,9 +494,7 @@ cudaError_t launch_inv(const InvArgs& a, cudaStream_t st) {
     }
     const int grid = (a.g.nb + C::BPC - 1) / C::BPC;
     if (grid == 0) return cudaSuccess;
-    k<<<grid, C::THREADS, smem, st>>>(a);
-    count_launch();
-    return cudaGetLastError();
+    return launch_kernel(k, grid, C::THREADS, smem, st, a);
   }
 }
 

