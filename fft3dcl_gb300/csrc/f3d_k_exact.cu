@@ -184,7 +184,12 @@ __device__ __forceinline__ void filter_block(const InvArgs& a, int b, int t, flo
 // filter for each mode, of which a launch runs one) or read per bin.
 template <bool KALMAN, bool BY_MODE, int PS, int TPB, int KB>
 __device__ __forceinline__ void filter_block_any(const InvArgs& a, int b, int t, float2* F) {
-  constexpr int KN = 4;  // bins in flight, temporal modes
+  // Bins in flight, temporal modes (the block's spectra are on their way into
+  // L2): with more, the code outgrows the instruction cache (1080p 10-bit, pass
+  // with 1, 2, 3, 4 in flight: 32x32 bt=4 97.4, 97.6, 97.6, 104 us, bt=1 78, 76,
+  // 75, 76; bt=3 64x64 129.5, 129.6, 132, 137, 16x16 79, 81, 84, 86, 8x8 85, 86,
+  // 89, 95).
+  constexpr int KN = TPB == 64 ? 3 : 1;
   if constexpr (KALMAN) {
     filter_block<0, PS, TPB, KB>(a, b, t, F);
   } else if constexpr (BY_MODE) {
@@ -283,23 +288,29 @@ __global__ void __launch_bounds__(Cfg<BW, BH>::THREADS, Cfg<BW, BH>::INV_CTAS - 
   stamp_end(a.clk);
 }
 
-// ---- 64 x 64 blocks: each 64-point transform on a lane pair ----------------
+// ---- 64 x 64 blocks, inverse of 32 x 32: each transform on a lane pair -----
 //
 // One thread per 64-point transform holds 128 registers of data and leaves
 // 504 CTAs of two 720p blocks in two waves; a lane pair (lanes 2i, 2i+1)
 // halves both. The bit-reversed array is split in halves: the even lane
-// holds positions 0..31, the odd lane 32..63. Stages len = 2..32 stay inside
-// a half (twiddles tw[j * 64 / len], as in the whole transform); the last
-// stage pairs position j with j + 32: the odd lane forms t = w_j * a[j + 32],
+// holds positions 0..N/2-1, the odd lane the others. Stages len = 2..N/2 stay
+// inside a half (twiddles tw[j * N / len], as in the whole transform); the last
+// stage pairs position j with j + N/2: the odd lane forms t = w_j * a[j + N/2],
 // the lanes swap t and u = a[j] by one shuffle, and each forms its output,
 // u + t or u - t. Every value is computed by the same operations as in
-// fft_r2<64> (src/cpu/fft.cpp:28-58), so the bits are the same.
+// fft_r2<N> (src/cpu/fft.cpp:28-58), so the bits are the same.
+//
+// The inverse of 32 x 32 blocks, 64 threads a block of 64 registers each, runs
+// 32 warps an SM (k_inverse_exact: 24 of twice the work, half of their issue
+// slots idle on loads, divides and instruction fetch): pass of 1080p 10-bit
+// bt=4 124 -> 98 us, bt=1 90 -> 75, Kalman 89 -> 74, 360p bt=3 38 -> 28. The
+// forward lost by it (98 -> 103 us): 17 columns take a second warp.
 
-template <int LEN, bool INV>
-__device__ __forceinline__ void half_stage64(float2 (&a)[32], const float2* tw) {
-  constexpr int half = LEN / 2, step = 64 / LEN;
+template <int N, int LEN, bool INV>
+__device__ __forceinline__ void half_stage(float2 (&a)[N / 2], const float2* tw) {
+  constexpr int half = LEN / 2, step = N / LEN;
 #pragma unroll
-  for (int i = 0; i < 32; i += LEN) {
+  for (int i = 0; i < N / 2; i += LEN) {
 #pragma unroll
     for (int j = 0; j < half; j++) {
       const float2 b = a[i + j + half];
@@ -317,16 +328,16 @@ __device__ __forceinline__ void half_stage64(float2 (&a)[32], const float2* tw) 
       a[i + j + half] = make_float2(u.x - t.x, u.y - t.y);
     }
   }
-  if constexpr (LEN < 32) half_stage64<LEN * 2, INV>(a, tw);
+  if constexpr (LEN < N / 2) half_stage<N, LEN * 2, INV>(a, tw);
 }
 
-// a: positions 32 * odd + p (p < 32) of the bit-reversed input; out: the
-// transform's values 32 * odd + p. Every lane of the warp takes part.
-template <bool INV>
-__device__ __forceinline__ void fft64_pair(float2 (&a)[32], const float2* tw, bool odd) {
-  half_stage64<2, INV>(a, tw);
+// a: positions N/2 * odd + p (p < N/2) of the bit-reversed input; out: the
+// transform's values N/2 * odd + p. Every lane of the warp takes part.
+template <int N, bool INV>
+__device__ __forceinline__ void fft_pair(float2 (&a)[N / 2], const float2* tw, bool odd) {
+  half_stage<N, 2, INV>(a, tw);
 #pragma unroll
-  for (int j = 0; j < 32; j++) {
+  for (int j = 0; j < N / 2; j++) {
     const float2 x = a[j];
     float2 t = x;
     if (j > 0) {
@@ -340,9 +351,9 @@ __device__ __forceinline__ void fft64_pair(float2 (&a)[32], const float2* tw, bo
     a[j] = odd ? make_float2(rx - t.x, ry - t.y) : make_float2(x.x + rx, x.y + ry);
   }
   if (INV) {
-    const float invn = 1.0f / 64;
+    const float invn = 1.0f / N;
 #pragma unroll
-    for (int i = 0; i < 32; i++) a[i] = make_float2(a[i].x * invn, a[i].y * invn);
+    for (int i = 0; i < N / 2; i++) a[i] = make_float2(a[i].x * invn, a[i].y * invn);
   }
 }
 
@@ -370,7 +381,7 @@ __global__ void __launch_bounds__(kPairThreads, 6) k_forward_exact64(const __gri
 #pragma unroll
   for (int q = 0; q < 32; q++) r[q] = make_float2(tile[p * kPairTS + bit_reverse(q, 6) + odd], 0.0f);
   __syncthreads();  // the tile is read: the row spectra may overwrite it
-  fft64_pair<false>(r, a.tw.row, odd);
+  fft_pair<64, false>(r, a.tw.row, odd);
   if (!odd) {
 #pragma unroll
     for (int c = 0; c < 32; c++) rows[p * FBW + c] = r[c];
@@ -382,7 +393,7 @@ __global__ void __launch_bounds__(kPairThreads, 6) k_forward_exact64(const __gri
     const int c = p < FBW ? p : 0;
 #pragma unroll
     for (int q = 0; q < 32; q++) r[q] = rows[(bit_reverse(q, 6) + odd) * FBW + c];
-    fft64_pair<false>(r, a.tw.col, odd);
+    fft_pair<64, false>(r, a.tw.col, odd);
     if (p < FBW) {
       float2* out = a.spec + (size_t)b * 64 * FBW + c;
 #pragma unroll
@@ -392,16 +403,16 @@ __global__ void __launch_bounds__(kPairThreads, 6) k_forward_exact64(const __gri
   }
 }
 
-// Filter + inverse of one 64 x 64 block per CTA: the filtered half spectrum
-// F, column transforms (pair p = column p, Hermitian completion on the fly)
-// into G, which shares F's space once every column is in registers, then
-// row transforms (pair p = row p) and the windowed rows in plane order.
-template <bool KALMAN>
-__global__ void __launch_bounds__(kPairThreads, 5) k_inverse_exact64(const __grid_constant__ InvArgs a) {
-  constexpr int FBW = 33, PS = 64 * FBW;
+// Filter + inverse of one N x N block per CTA: the filtered half spectrum F,
+// column transforms (pair p = column p, Hermitian completion on the fly) into
+// G, which shares F's space once every column is in registers, then row
+// transforms (pair p = row p) and the windowed rows in plane order.
+template <int N, bool KALMAN>
+__global__ void __launch_bounds__(2 * N, N == 64 ? 5 : 16) k_inverse_pair(const __grid_constant__ InvArgs a) {
+  constexpr int FBW = N / 2 + 1, PS = N * FBW, H = N / 2, TS = N + 1, L = Log2<N>::v;
   extern __shared__ float4 smem4[];
-  float2* F = reinterpret_cast<float2*>(smem4);  // [64][FBW]
-  float2* G = F;                                 // [64][kPairTS], after the column reads
+  float2* F = reinterpret_cast<float2*>(smem4);  // [N][FBW]
+  float2* G = F;                                 // [N][TS], after the column reads
   const int t = threadIdx.x, p = t >> 1;
   const bool odd = t & 1;
   const int b = blockIdx.x;
@@ -409,38 +420,39 @@ __global__ void __launch_bounds__(kPairThreads, 5) k_inverse_exact64(const __gri
   grid_wait();
   stamp_start(a.clk);
   if (!KALMAN && t == 0) prefetch_window<PS>(a, b);
-  filter_block_any<KALMAN, true, PS, kPairThreads, 6>(a, b, t, F);
+  filter_block_any<KALMAN, true, PS, 2 * N, N == 64 ? 6 : 3>(a, b, t, F);
   __syncthreads();
-  // A row's odd lane puts its 16 sample pairs 24 entries along: in other
-  // banks than its even lane's.
-  constexpr int kOddAt = 24;
-  float2 r[32];
+  // A row's odd lane puts its N/4 sample pairs 8 entries (of 16 that the banks
+  // hold) beside its even lane's.
+  constexpr int kOddAt = N == 64 ? 24 : 8;
+  static_assert(kOddAt >= N / 4 && kOddAt % 16 == 8 && kOddAt + N / 4 <= TS, "row of sample pairs");
+  float2 r[H];
   {
     const int c = p;
 #pragma unroll
-    for (int q = 0; q < 32; q++) {
-      const int row = bit_reverse(q, 6) + odd;
+    for (int q = 0; q < H; q++) {
+      const int row = bit_reverse(q, L) + odd;
       if (c < FBW) {
         r[q] = F[row * FBW + c];
       } else {
-        const float2 m = F[((64 - row) & 63) * FBW + (64 - c)];
+        const float2 m = F[((N - row) & (N - 1)) * FBW + (N - c)];
         r[q] = make_float2(m.x, -m.y);
       }
     }
   }
   __syncthreads();  // F is read: G may overwrite it
-  fft64_pair<true>(r, a.tw.col, odd);
+  fft_pair<N, true>(r, a.tw.col, odd);
 #pragma unroll
-  for (int q = 0; q < 32; q++) G[(32 * odd + q) * kPairTS + p] = r[q];
+  for (int q = 0; q < H; q++) G[(H * odd + q) * TS + p] = r[q];
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < 32; q++) r[q] = G[p * kPairTS + bit_reverse(q, 6) + odd];
-  fft64_pair<true>(r, a.tw.row, odd);
+  for (int q = 0; q < H; q++) r[q] = G[p * TS + bit_reverse(q, L) + odd];
+  fft_pair<N, true>(r, a.tw.row, odd);
   __syncwarp();  // the pair has read its row
 #pragma unroll
-  for (int q = 0; q < 16; q++) G[p * kPairTS + kOddAt * odd + q] = make_float2(r[2 * q].x, r[2 * q + 1].x);
+  for (int q = 0; q < N / 4; q++) G[p * TS + kOddAt * odd + q] = make_float2(r[2 * q].x, r[2 * q + 1].x);
   __syncthreads();
-  store_block<64, 64, kPairThreads, kPairTS>(a, b, t, G, [](int j) { return j < 16 ? j : j + (kOddAt - 16); });
+  store_block<N, N, 2 * N, TS>(a, b, t, G, [](int j) { return j < N / 4 ? j : j + (kOddAt - N / 4); });
   stamp_end(a.clk);
 }
 
@@ -451,15 +463,12 @@ cudaError_t launch_fwd64(const FwdArgs& a, cudaStream_t st) {
   return launch_kernel(k_forward_exact64, a.g.nb, kPairThreads, smem, st, a);
 }
 
-cudaError_t launch_inv64(const InvArgs& a, cudaStream_t st) {
-  const size_t smem = sizeof(float2) * 64 * kPairTS;  // G, which covers F
-  auto k = a.bm == 0 ? k_inverse_exact64<true> : k_inverse_exact64<false>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+template <int N>
+cudaError_t launch_inv_pair(const InvArgs& a, cudaStream_t st) {
+  const size_t smem = sizeof(float2) * N * (N + 1);  // G, which covers F
+  static_assert(sizeof(float2) * N * (N + 1) <= 48 * 1024, "shared memory without opting in");
   if (a.g.nb == 0) return cudaSuccess;
-  return launch_kernel(k, a.g.nb, kPairThreads, smem, st, a);
+  return launch_kernel(a.bm == 0 ? k_inverse_pair<N, true> : k_inverse_pair<N, false>, a.g.nb, 2 * N, smem, st, a);
 }
 
 template <int BW, int BH>
@@ -482,8 +491,8 @@ cudaError_t launch_fwd(const FwdArgs& a, cudaStream_t st) {
 
 template <int BW, int BH>
 cudaError_t launch_inv(const InvArgs& a, cudaStream_t st) {
-  if constexpr (BW == 64 && BH == 64) {
-    return launch_inv64(a, st);
+  if constexpr (BW == BH && BW >= 32) {
+    return launch_inv_pair<BW>(a, st);
   } else {
     using C = Cfg<BW, BH>;
     const size_t smem = sizeof(float) * C::INV_FLOATS * C::BPC;
