@@ -187,7 +187,7 @@ __device__ __forceinline__ void filter_block_any(const InvArgs& a, int b, int t,
   // Bins in flight, temporal modes (the block's spectra are on their way into
   // L2): with more, the code outgrows the instruction cache (1080p 10-bit, pass
   // with 1, 2, 3, 4 in flight: 32x32 bt=4 97.4, 97.6, 97.6, 104 us, bt=1 78, 76,
-  // 75, 76; bt=3 64x64 129.5, 129.6, 132, 137, 16x16 79, 81, 84, 86, 8x8 85, 86,
+  // 75, 76; bt=3 64x64 on pairs 129.5, 129.6, 132, 137, 16x16 79, 81, 84, 86, 8x8 85, 86,
   // 89, 95).
   constexpr int KN = TPB == 64 ? 3 : 1;
   if constexpr (KALMAN) {
@@ -220,7 +220,7 @@ __device__ __forceinline__ void prefetch_window(const InvArgs& a, int b) {
 // each thread walks its own row: 16 to 32 lines per request, and the loads
 // and stores of the block took half of the kernel (inverse, 1080p 10-bit bt=4
 // with 32x32 blocks: 180 -> 99 us; 720p Kalman with 64x64 blocks: 60 -> 35 us).
-template <int BW, int BH, int TPB, int TS, class At>
+template <int BW, int BH, int TPB, class At>
 __device__ __forceinline__ void store_block(const InvArgs& a, int b, int t, const float2* S, At&& at) {
   int bx, by, par;
   block_origin(a.g, b, bx, by, par);
@@ -228,7 +228,7 @@ __device__ __forceinline__ void store_block(const InvArgs& a, int b, int t, cons
   float2* out = reinterpret_cast<float2*>(a.blocks + (size_t)b * BW * BH);
 #pragma unroll 8
   for (int i = t; i < BW * BH / 2; i += TPB) {
-    const float2 v = S[(i / (BW / 2)) * TS + at(i % (BW / 2))], w = win[i];
+    const float2 v = S[at(i / (BW / 2), i % (BW / 2))], w = win[i];
     out[i] = make_float2(v.x * w.x, v.y * w.y);
   }
 }
@@ -284,11 +284,11 @@ __global__ void __launch_bounds__(Cfg<BW, BH>::THREADS, Cfg<BW, BH>::INV_CTAS - 
     for (int c = 0; c < BW / 2; c++) G[t * C::TS + c] = make_float2(v[2 * c].x, v[2 * c + 1].x);
   }
   block_sync<C::TPB>();
-  if (valid) store_block<BW, BH, C::TPB, C::TS>(a, b, t, G, [](int j) { return j; });
+  if (valid) store_block<BW, BH, C::TPB>(a, b, t, G, [](int r, int j) { return r * C::TS + j; });
   stamp_end(a.clk);
 }
 
-// ---- 64 x 64 blocks, inverse of 32 x 32: each transform on a lane pair -----
+// ---- 64 x 64 blocks, inverse of 32 x 32: each transform on 2 or 4 lanes -----
 //
 // One thread per 64-point transform holds 128 registers of data and leaves
 // 504 CTAs of two 720p blocks in two waves; a lane pair (lanes 2i, 2i+1)
@@ -297,20 +297,25 @@ __global__ void __launch_bounds__(Cfg<BW, BH>::THREADS, Cfg<BW, BH>::INV_CTAS - 
 // inside a half (twiddles tw[j * N / len], as in the whole transform); the last
 // stage pairs position j with j + N/2: the odd lane forms t = w_j * a[j + N/2],
 // the lanes swap t and u = a[j] by one shuffle, and each forms its output,
-// u + t or u - t. Every value is computed by the same operations as in
-// fft_r2<N> (src/cpu/fft.cpp:28-58), so the bits are the same.
+// u + t or u - t. On four lanes the last two stages are formed so. Every value
+// is computed by the same operations as in fft_r2<N> (src/cpu/fft.cpp:28-58),
+// so the bits are the same.
 //
-// The inverse of 32 x 32 blocks, 64 threads a block of 64 registers each, runs
-// 32 warps an SM (k_inverse_exact: 24 of twice the work, half of their issue
-// slots idle on loads, divides and instruction fetch): pass of 1080p 10-bit
-// bt=4 124 -> 98 us, bt=1 90 -> 75, Kalman 89 -> 74, 360p bt=3 38 -> 28. The
-// forward lost by it (98 -> 103 us): 17 columns take a second warp.
+// The inverse takes 16 values of a transform per lane: 64 registers a thread
+// and 32 warps an SM. 32 x 32 blocks, pairs (k_inverse_exact: 24 warps of twice
+// the work, half of their issue slots idle on loads, divides and instruction
+// fetch): pass of 1080p 10-bit bt=4 124 -> 98 us, bt=1 90 -> 75, Kalman
+// 89 -> 74, 360p bt=3 38 -> 27. 64 x 64 blocks, four lanes (pairs: 20 warps, and
+// the latency of one block counted twice where 720p has 1,008 of them for 760
+// places): 720p Kalman 56 -> 51, bt=3 72 -> 59, 1080p bt=3 130 -> 116.
+// The forward of 32 x 32 blocks lost by pairs (98 -> 103 us): 17 columns take
+// a second warp.
 
-template <int N, int LEN, bool INV>
-__device__ __forceinline__ void half_stage(float2 (&a)[N / 2], const float2* tw) {
+template <int N, int LEN, bool INV, int M>
+__device__ __forceinline__ void half_stage(float2 (&a)[M], const float2* tw) {
   constexpr int half = LEN / 2, step = N / LEN;
 #pragma unroll
-  for (int i = 0; i < N / 2; i += LEN) {
+  for (int i = 0; i < M; i += LEN) {
 #pragma unroll
     for (int j = 0; j < half; j++) {
       const float2 b = a[i + j + half];
@@ -328,14 +333,14 @@ __device__ __forceinline__ void half_stage(float2 (&a)[N / 2], const float2* tw)
       a[i + j + half] = make_float2(u.x - t.x, u.y - t.y);
     }
   }
-  if constexpr (LEN < N / 2) half_stage<N, LEN * 2, INV>(a, tw);
+  if constexpr (LEN < M) half_stage<N, LEN * 2, INV, M>(a, tw);
 }
 
 // a: positions N/2 * odd + p (p < N/2) of the bit-reversed input; out: the
 // transform's values N/2 * odd + p. Every lane of the warp takes part.
 template <int N, bool INV>
 __device__ __forceinline__ void fft_pair(float2 (&a)[N / 2], const float2* tw, bool odd) {
-  half_stage<N, 2, INV>(a, tw);
+  half_stage<N, 2, INV, N / 2>(a, tw);
 #pragma unroll
   for (int j = 0; j < N / 2; j++) {
     const float2 x = a[j];
@@ -403,56 +408,105 @@ __global__ void __launch_bounds__(kPairThreads, 6) k_forward_exact64(const __gri
   }
 }
 
-// Filter + inverse of one N x N block per CTA: the filtered half spectrum F,
-// column transforms (pair p = column p, Hermitian completion on the fly) into
-// G, which shares F's space once every column is in registers, then row
-// transforms (pair p = row p) and the windowed rows in plane order.
+// One stage between lanes: u + t on the lane with the lower half (hi false),
+// u - t on the other, t = w_j * its value; w_0 = 1 (first: of a[0]) takes no
+// product, which would change zeros' signs and infinities.
+template <bool INV, int M, class W>
+__device__ __forceinline__ void lane_stage(float2 (&a)[M], int lane_mask, bool hi, bool first, W&& tw) {
+#pragma unroll
+  for (int j = 0; j < M; j++) {
+    const float2 x = a[j], w = tw(j);
+    const float wy = INV ? -w.y : w.y;
+    float2 t = make_float2(w.x * x.x - wy * x.y, w.x * x.y + wy * x.x);
+    if (j == 0 && first) t = x;
+    const float2 send = hi ? t : x;
+    const float rx = __shfl_xor_sync(0xffffffffu, send.x, lane_mask), ry = __shfl_xor_sync(0xffffffffu, send.y, lane_mask);
+    a[j] = hi ? make_float2(rx - t.x, ry - t.y) : make_float2(x.x + rx, x.y + ry);
+  }
+}
+
+// The inverse transform of N values on a group of G lanes, lane l holding
+// positions N/G * l + q of the bit-reversed input, then of the output.
+template <int N, int G>
+__device__ __forceinline__ void ifft_group(float2 (&a)[N / G], const float2* tw, int l) {
+  if constexpr (G == 2) {
+    fft_pair<N, true>(a, tw, l);
+  } else {
+    constexpr int M = N / 4;
+    static_assert(G == 4, "two or four lanes");
+    half_stage<N, 2, true, M>(a, tw);
+    lane_stage<true>(a, 1, l & 1, true, [&](int j) { return tw[2 * j]; });
+    lane_stage<true>(a, 2, l & 2, !(l & 1), [&](int j) {
+      const float2 w0 = tw[j], w1 = tw[j + M];
+      return l & 1 ? w1 : w0;
+    });
+    const float invn = 1.0f / N;
+#pragma unroll
+    for (int i = 0; i < M; i++) a[i] = make_float2(a[i].x * invn, a[i].y * invn);
+  }
+}
+
+template <int N>
+struct InvLanes {
+  static constexpr int LN = N == 64 ? 4 : 2;
+  static constexpr int THREADS = LN * N, M = N / LN;
+  // Row stride of G, and how far each further M rows are moved along: a
+  // half-warp's columns, or rows, lie in different banks.
+  static constexpr int TS = LN == 4 ? N + 4 : N + 1, SKEW = LN == 4 ? 4 : 0;
+  static __device__ __forceinline__ int at(int row, int col) { return row * TS + row / M * SKEW + col; }
+  // A row's lanes put their M/2 sample pairs kAt entries apart (banks again).
+  static constexpr int kAt = LN == 4 ? 12 : 8;
+  static constexpr size_t SMEM = sizeof(float2) * (N * TS + LN * SKEW);
+};
+
+// Filter + inverse of one N x N block per CTA, each transform on LN lanes: the
+// filtered half spectrum F, column transforms (group p = column p, Hermitian
+// completion on the fly) into G, which shares F's space once every column is in
+// registers, then row transforms (group p = row p) and the windowed rows in
+// plane order.
 template <int N, bool KALMAN>
-__global__ void __launch_bounds__(2 * N, N == 64 ? 5 : 16) k_inverse_pair(const __grid_constant__ InvArgs a) {
-  constexpr int FBW = N / 2 + 1, PS = N * FBW, H = N / 2, TS = N + 1, L = Log2<N>::v;
+__global__ void __launch_bounds__(InvLanes<N>::THREADS, 1024 / InvLanes<N>::THREADS)
+    k_inverse_lanes(const __grid_constant__ InvArgs a) {
+  using C = InvLanes<N>;
+  constexpr int FBW = N / 2 + 1, PS = N * FBW, LN = C::LN, M = C::M, L = Log2<N>::v;
   extern __shared__ float4 smem4[];
   float2* F = reinterpret_cast<float2*>(smem4);  // [N][FBW]
   float2* G = F;                                 // [N][TS], after the column reads
-  const int t = threadIdx.x, p = t >> 1;
-  const bool odd = t & 1;
+  const int t = threadIdx.x, p = t / LN, l = t % LN;
+  const int rl = LN == 4 ? bit_reverse(l, 2) : l;
   const int b = blockIdx.x;
   grid_go();
   grid_wait();
   stamp_start(a.clk);
   if (!KALMAN && t == 0) prefetch_window<PS>(a, b);
-  filter_block_any<KALMAN, true, PS, 2 * N, N == 64 ? 6 : 3>(a, b, t, F);
+  filter_block_any<KALMAN, true, PS, C::THREADS, 3>(a, b, t, F);
   __syncthreads();
-  // A row's odd lane puts its N/4 sample pairs 8 entries (of 16 that the banks
-  // hold) beside its even lane's.
-  constexpr int kOddAt = N == 64 ? 24 : 8;
-  static_assert(kOddAt >= N / 4 && kOddAt % 16 == 8 && kOddAt + N / 4 <= TS, "row of sample pairs");
-  float2 r[H];
-  {
-    const int c = p;
+  float2 r[M];
 #pragma unroll
-    for (int q = 0; q < H; q++) {
-      const int row = bit_reverse(q, L) + odd;
-      if (c < FBW) {
-        r[q] = F[row * FBW + c];
-      } else {
-        const float2 m = F[((N - row) & (N - 1)) * FBW + (N - c)];
-        r[q] = make_float2(m.x, -m.y);
-      }
+  for (int q = 0; q < M; q++) {
+    const int row = bit_reverse(q, L) + rl;  // bit_reverse(M * l + q)
+    if (p < FBW) {
+      r[q] = F[row * FBW + p];
+    } else {
+      const float2 m = F[((N - row) & (N - 1)) * FBW + (N - p)];
+      r[q] = make_float2(m.x, -m.y);
     }
   }
   __syncthreads();  // F is read: G may overwrite it
-  fft_pair<N, true>(r, a.tw.col, odd);
+  ifft_group<N, LN>(r, a.tw.col, l);
 #pragma unroll
-  for (int q = 0; q < H; q++) G[(H * odd + q) * TS + p] = r[q];
+  for (int q = 0; q < M; q++) G[C::at(M * l + q, p)] = r[q];
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < H; q++) r[q] = G[p * TS + bit_reverse(q, L) + odd];
-  fft_pair<N, true>(r, a.tw.row, odd);
-  __syncwarp();  // the pair has read its row
+  for (int q = 0; q < M; q++) r[q] = G[C::at(p, bit_reverse(q, L) + rl)];
+  ifft_group<N, LN>(r, a.tw.row, l);
+  __syncwarp();  // the group has read its row
 #pragma unroll
-  for (int q = 0; q < N / 4; q++) G[p * TS + kOddAt * odd + q] = make_float2(r[2 * q].x, r[2 * q + 1].x);
+  for (int q = 0; q < M / 2; q++) G[C::at(p, C::kAt * l + q)] = make_float2(r[2 * q].x, r[2 * q + 1].x);
   __syncthreads();
-  store_block<N, N, 2 * N, TS>(a, b, t, G, [](int j) { return j < N / 4 ? j : j + (kOddAt - N / 4); });
+  store_block<N, N, C::THREADS>(a, b, t, G, [](int row, int j) {
+    return C::at(row, j / (M / 2) * C::kAt + j % (M / 2));
+  });
   stamp_end(a.clk);
 }
 
@@ -463,12 +517,13 @@ cudaError_t launch_fwd64(const FwdArgs& a, cudaStream_t st) {
   return launch_kernel(k_forward_exact64, a.g.nb, kPairThreads, smem, st, a);
 }
 
-template <int N>
-cudaError_t launch_inv_pair(const InvArgs& a, cudaStream_t st) {
-  const size_t smem = sizeof(float2) * N * (N + 1);  // G, which covers F
-  static_assert(sizeof(float2) * N * (N + 1) <= 48 * 1024, "shared memory without opting in");
+template <int N, bool KALMAN>
+cudaError_t launch_inv_lanes(const InvArgs& a, cudaStream_t st) {
+  using C = InvLanes<N>;
+  static_assert(C::SMEM <= 48 * 1024, "shared memory without opting in");
+  static_assert(C::SMEM >= sizeof(float2) * N * (N / 2 + 1), "G covers F");
   if (a.g.nb == 0) return cudaSuccess;
-  return launch_kernel(a.bm == 0 ? k_inverse_pair<N, true> : k_inverse_pair<N, false>, a.g.nb, 2 * N, smem, st, a);
+  return launch_kernel(k_inverse_lanes<N, KALMAN>, a.g.nb, C::THREADS, C::SMEM, st, a);
 }
 
 template <int BW, int BH>
@@ -492,7 +547,7 @@ cudaError_t launch_fwd(const FwdArgs& a, cudaStream_t st) {
 template <int BW, int BH>
 cudaError_t launch_inv(const InvArgs& a, cudaStream_t st) {
   if constexpr (BW == BH && BW >= 32) {
-    return launch_inv_pair<BW>(a, st);
+    return a.bm == 0 ? launch_inv_lanes<BW, true>(a, st) : launch_inv_lanes<BW, false>(a, st);
   } else {
     using C = Cfg<BW, BH>;
     const size_t smem = sizeof(float) * C::INV_FLOATS * C::BPC;
