@@ -50,9 +50,9 @@ NCU_TRAFFIC = {"tc": 571806464 + 130638592}
 # 1920x1080 --steps 1 --warmup 3 --no-cpu --serve-streams 0 --no-yuv
 # --compare tc --outputs-per-step k`, mean of the k-output launches; k=4:
 # 260.2 MB read + 124.4 MB written, k=8: 410.5 + 286.0 MB, k=10 (with the
-# filter's current column mapping): 490.3 + 366.7 MB) and scaled to
+# filter's block images): 495.5 + 305.5 MB) and scaled to
 # 3840x2160 by the block count (32912 / 8540).
-NCU_TRAFFIC_BATCH = {4: 1002927925 + 479516689, 8: 1581975962 + 1102231724, 10: 1889588860 + 1413116250}
+NCU_TRAFFIC_BATCH = {4: 1002927925 + 479516689, 8: 1581975962 + 1102231724, 10: 1909589696 + 1177355504}
 # Consecutive outputs per batch step of the tensor-core headline (4K sweeps:
 # ten beat eight and twelve); its traffic must be in NCU_TRAFFIC_BATCH.
 DEFAULT_OUTPUTS_PER_STEP = 10
@@ -757,7 +757,7 @@ def run_gpu(args, rank, world, local_rank):
     peak, peak_kind = load_peaks()
     inv_ms = float(kt[1])
     # The dominant kernel, timed by itself on the GPU: the tensor-core
-    # filter (window spectra in; its operand tiles are an intermediate), the
+    # filter (window spectra in; its block images are an intermediate), the
     # fused fast-form sweep (window spectra in, packed plane out) or, unfused,
     # the filter+inverse kernel (window spectra in).
     if info.form == 2 and info.fused:
@@ -778,9 +778,9 @@ def run_gpu(args, rank, world, local_rank):
     roof = roof_single
     bkt = forms_extra.get("batch_kernel_ms")
     if bkt and kframes > 1 and info.form == 2 and info.fused:
-        # The headline step's own filter launch: kframes consecutive outputs,
-        # each reading its bt window spectra (shared ones from L2).
-        bbytes = kframes * kbytes
+        # The headline step's own filter launch: kframes consecutive outputs
+        # whose windows share spectra, each distinct one counted once.
+        bbytes = kbytes // bt * (kframes + bt - 1)
         bach = bbytes / (bkt[0] / 1000.0) / 1e9
         roof = {"kernel": f"k_filter_tc, {kframes} consecutive outputs per launch (the headline batch step)",
                 "bound": "hbm", "achieved": round(bach, 1), "peak": peak, "unit": "GB/s",

@@ -1,7 +1,7 @@
 // f3d_batch_plan.hpp -- host-side planning of the batched tensor-core
-// launches: the by-value batch parameters of the forward and of the filter,
-// inverse and seam-merge kernels, with each kernel's per-plane prefix of CTA
-// (or block-group) counts, the filter's runs of one geometry and its
+// launches: the by-value batch parameters of the forward and of the filter
+// and inverse kernels, with each kernel's per-plane prefix of CTA (or
+// block-group) counts, the filter's runs of one geometry and its
 // shifted-window bits. Plain host code, also compiled by the CPU tests.
 #pragma once
 
@@ -31,11 +31,11 @@ inline bool forward_batch(const TcFwdArgs* planes, int n, TcFwdBatch& B) {
   return true;
 }
 
-// The three sweep-side batch parameters (filter, inverse, seam merge) of
-// `planes`: the same planes, with the prefix of each kernel's CTA counts.
-// tc: the tensor-core sweep (16x16 or 32x32 blocks, tables, operand tiles);
-// otherwise the fast form's fused sweep (8x8 to 32x32 blocks; only Bs and Bm
-// are used).
+// The sweep-side batch parameters (by (row, strip) group, by CTA of the sweep,
+// by seam row) of `planes`: the same planes, with the prefix of each one's
+// counts. tc: the tensor-core sweep (16x16 or 32x32 blocks, tables, block
+// images); otherwise the fast form's fused sweep (8x8 to 32x32 blocks; only Bs
+// is used).
 inline bool sweep_batches(const SweepArgs* planes, int n, SweepBatch& Bf, SweepBatch& Bs, SweepBatch& Bm,
                           bool tc = true) {
   if (n < 1 || n > kMaxBatch) return false;

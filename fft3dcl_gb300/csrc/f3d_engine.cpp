@@ -98,7 +98,7 @@ struct f3d_engine {
   int sweep_strips = 0, sweep_segs = 0, sweep_prefetch = 0;
   float* d_seam = nullptr;
   size_t seam_floats = 0;
-  uint8_t* d_img = nullptr;  // tensor-core sweep: filtered operand tiles
+  uint8_t* d_img = nullptr;  // tensor-core sweep: filtered block images
   size_t img_bytes = 0;
 
   size_t bytes = 0;
@@ -857,7 +857,7 @@ struct f3d_batch {
   KernelClock* clk = nullptr;
   bool ktimed = false;
   // Entries whose engine appeared earlier in the batch (one more output of
-  // that plane per step) have operand tiles and seam rows of their own.
+  // that plane per step) have block images and seam rows of their own.
   std::vector<uint8_t*> img;   // per entry, null: the engine's own
   std::vector<float*> seam;
   std::vector<size_t> img_bytes, seam_bytes;
@@ -935,7 +935,7 @@ int f3d_batch_create(f3d_engine* const* engines, int n, int flags, f3d_batch** o
     if (!repeat) continue;
     b->repeat[i] = true;
     const f3d_engine* e = engines[i];
-    b->img_bytes[i] = b->fast ? 0 : e->img_bytes;  // the fast sweep has no operand tiles
+    b->img_bytes[i] = b->fast ? 0 : e->img_bytes;  // the fast sweep has no block images
     b->seam_bytes[i] = sizeof(float) * e->seam_floats;
     if ((b->img_bytes[i] && cudaMalloc(&b->img[i], b->img_bytes[i]) != cudaSuccess) ||
         (b->seam_bytes[i] && (cudaMalloc(&b->seam[i], b->seam_bytes[i]) != cudaSuccess ||
@@ -1102,7 +1102,7 @@ int f3d_batch_step(f3d_batch* b, const int* fns, const void* const* dev_src, con
   // 1-3 % slower in steady state at eight and ten outputs.
   const uint64_t all = (1ull << n) - 1;
   if (!b->fast && (b->flags & F3D_BATCH_AUTOTUNE) && !b->tuned && (mask & 0xFFFFFFFFull) == (all | (all << 16))) {
-    // Both filter variants, with the forward kernel on as many CTAs as fit: on
+    // The filter's two load batches, with the forward kernel on as many CTAs as fit: on
     // two or one per SM a step was never faster, only picked by that noise (three
     // 1080p planes {3,5} 111.7, {3,4} 111.5, {2,5} 115, {1,5} 133 us; ten 10-bit
     // 4K outputs 1390, 1437, 1558, 1974 us).

@@ -24,7 +24,7 @@ uint64_t plane_batch_key(const f3d_internal_params& p, const f3d_plane_geom& g);
 // One temporal step of n (1..16) distinct batchable engines whose stream is
 // st, one launch per kernel for all of them: engine i forwards frame fns[i]
 // from src[i] (skipped when fns[i] < 0 or cached), then, when nwin[i] > 0,
-// filters its window win[i] into dst[i] with its own operand tiles and seam
+// filters its window win[i] into dst[i] with its own block images and seam
 // rows. Queued on st. On failure *err has the message.
 int engines_step(f3d_engine* const* e, int n, const int* fns, const void* const* src, const size_t* src_pitch,
                  const int* const* win, const int* nwin, void* const* dst, const size_t* dst_pitch, cudaStream_t st,

@@ -214,7 +214,7 @@ __device__ __forceinline__ void prefetch_window(const InvArgs& a, int b) {
 }
 
 // Rows of a block's windowed inverse: sample pair j of row r (its two values
-// before the window) at S[r * TS + at(j)], written by the threads of the row
+// before the window) at S[at(r, j)], written by the threads of the row
 // transforms, read back here in plane order, so that the window is read and
 // the block written in whole lines. Stored straight from the row transforms
 // each thread walks its own row: 16 to 32 lines per request, and the loads

@@ -247,7 +247,7 @@ struct FilterBatch {
 // Launch shape of the tensor-core kernels, picked by the autotuner.
 struct TcTune {
   int fwd_ctas_per_sm = 3;  // persistent forward grid: CTAs per SM (1 to 3; 2 at most with the split)
-  int filter_minb = 5;      // filter kernel variant: 5, 4 or 3 CTAs per SM (spectra loads of 1, 2, 2 blocks in flight)
+  int filter_minb = 5;      // filter kernel variant: spectra loads of one block in flight, or (4, 3) of two
 };
 cudaError_t launch_forward_tc_batch(const TcFwdArgs* planes, int n, const TcTune& t, cudaStream_t st);
 // after_filter (may be null) is recorded on st between the filter and the

@@ -14,7 +14,7 @@
 // FFT3DCL_TIME names a file to which every released instance appends the
 // process-wide time per stage of the frame path (src/timing.h:1-31 of the
 // reference): wall-clock spans of getFrame, and the device time of the
-// engine's kernels from its CUDA events.
+// engine's kernels from their own clock stamps.
 #include "VSHelper4.h"
 #include "VapourSynth4.h"
 #include "fft3d_gb300.h"
