@@ -1,4 +1,4 @@
-"""The exact form's inverse on lane pairs (32x32 and 64x64 blocks) against the
+"""The exact form's inverse on lane groups (32x32 and 64x64 blocks) against the
 oracle, bit for bit: from one row of blocks up, every temporal mode with
 sharpening and degrid on and off, integer and float output."""
 import numpy as np
