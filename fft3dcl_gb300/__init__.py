@@ -652,8 +652,9 @@ class Batch:
         for k in lens:
             starts.append(at)
             at += 4 * k
-        args = (array("i", fns), array("Q", srcs), array("Q", src_pitches), array("Q", starts), array("i", lens),
-                array("Q", dsts), array("Q", dst_pitches))
+        # list(): array takes bytes and bytearrays as raw memory, not as whole numbers.
+        args = (array("i", list(fns)), array("Q", list(srcs)), array("Q", list(src_pitches)), array("Q", starts),
+                array("i", lens), array("Q", list(dsts)), array("Q", list(dst_pitches)))
         return lib().f3d_batch_step(self._h, *[a.buffer_info()[0] for a in args])
 
     def _step_ctypes(self, n, fns, srcs, src_pitches, windows, dsts, dst_pitches):
