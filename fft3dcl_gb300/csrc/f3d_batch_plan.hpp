@@ -86,6 +86,16 @@ inline int filter_switches(const SweepBatch& S) {
   return sw;
 }
 
+// The most segments a plane's strips are cut into: at most one wave of `slots`
+// resident CTAs (a partial second wave would double the time); one block row a
+// segment where they still fit (360p 8-bit bt=3, 72 -> 144 CTAs: 27.6 -> 26.8 us
+// a pass; every row is then read and written once more, in L2).
+inline int most_segments(int slots, int strips, int cells_y) {
+  int s = slots / strips;
+  if (s > cells_y + 1) s = cells_y + 1;
+  return s < 1 ? 1 : s;
+}
+
 // Segments of each plane's strips (written to its segs, at most what it comes
 // with) for one launch of all planes' sweeps, `slots` CTAs of which run at a
 // time. A CTA costs its block rows plus about one and a half for its set-up
@@ -95,6 +105,11 @@ inline int filter_switches(const SweepBatch& S) {
 // CTAs of 2 to 3 rows for 456 slots and 56 seams, here 378 CTAs of 5 rows and
 // 25 seams (its step, with the seams finished in the sweep: 123.5 -> 120.7
 // us; ten 4K outputs 1750 -> 1738 us).
+//
+// rows goes from one change of any plane's segments to the next: every number
+// of rows in turn took most of a long plane's host time (eight outputs of
+// 64x16384 with 8x8 blocks: 160 us a step, 56 before there was a plan; sixteen
+// planned in 282 us on an x86 host, 4 this way).
 inline void plan_segments(SweepArgs* planes, int n, int slots) {
   if (slots < 1) return;
   int most = 1;
@@ -105,13 +120,20 @@ inline void plan_segments(SweepArgs* planes, int n, int slots) {
   };
   int best = 0;
   long long best_cost = 0;
-  for (int rows = 1; rows <= most; rows++) {
+  for (int rows = 1, next; rows <= most; rows = next) {
     long long ctas = 0;
-    int longest = 0;
+    int longest = 0, s = 1;
+    next = most + 1;
     for (int i = 0; i < n; i++) {
-      const int s = segs_of(planes[i], rows), r = (planes[i].cells_y + 1 + s - 1) / s;
-      ctas += (long long)planes[i].strips * s;
-      longest = r > longest ? r : longest;
+      const SweepArgs& a = planes[i];
+      if (i == 0 || a.cells_y != planes[i - 1].cells_y || a.segs != planes[i - 1].segs) {
+        const int all = a.cells_y + 1;
+        s = segs_of(a, rows);
+        const int r = (all + s - 1) / s, fewer = s > 1 ? (all + s - 2) / (s - 1) : next;  // rows with s - 1 segments
+        longest = r > longest ? r : longest;
+        next = fewer < next ? fewer : next;
+      }
+      ctas += (long long)a.strips * s;
     }
     const long long cost = (ctas + slots - 1) / slots * (2 * longest + 3);
     if (best == 0 || cost <= best_cost) best = rows, best_cost = cost;

@@ -256,13 +256,7 @@ void sweep_plan(int form, const Geo& g, int sms, int* strips, int* segs) {
   const int cells_x = (g.W + g.bw / 2 - 1) / (g.bw / 2);
   const int cells_y = (g.H + g.bh / 2 - 1) / (g.bh / 2);
   *strips = (cells_x + tj - 1) / tj;
-  // At most one wave of resident CTAs (a partial second wave would double the
-  // time); one block row a segment where they still fit
-  // (360p 8-bit bt=3, 72 -> 144 CTAs: 27.6 -> 26.8 us a pass; every row is then
-  // read and written once more, in L2).
-  int s = per_sm * sms / *strips;
-  if (s > cells_y + 1) s = cells_y + 1;
-  *segs = s < 1 ? 1 : s;
+  *segs = most_segments(per_sm * sms, *strips, cells_y);
 }
 
 size_t sweep_seam_floats(const Geo& g, int strips, int segs) {
