@@ -41,16 +41,22 @@ __device__ __forceinline__ void grid_go() { asm volatile("griddepcontrol.launch_
 // A kernel's times, taken by its own threads (thread 0 of the first CTA, then
 // of every CTA): events around the kernels would keep each from starting until
 // the one before has ended and its time is written, about 2 us an event.
-__device__ __forceinline__ KernelClock device_ns() {
-  KernelClock t;
+__device__ __forceinline__ unsigned long long device_ns() {
+  unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
 __device__ __forceinline__ void stamp_start(KernelClock* clk) {  // after grid_wait
-  if (clk && (blockIdx.x | blockIdx.y | threadIdx.x) == 0) clk[0] = device_ns();
+  if (clk && (blockIdx.x | blockIdx.y | threadIdx.x) == 0) {
+    clk->start = device_ns();
+    atomicAdd(&clk->runs, (1ull << 32) + gridDim.x * gridDim.y);
+  }
 }
 __device__ __forceinline__ void stamp_end(KernelClock* clk) {
-  if (clk && threadIdx.x == 0) atomicMax(clk + 1, device_ns());
+  if (clk && threadIdx.x == 0) {
+    atomicMax(&clk->end, device_ns());
+    atomicAdd(&clk->runs, ~0ull);
+  }
 }
 
 // D3D9 MIRROR addressing, src/cpu/reference.cpp:10-17.

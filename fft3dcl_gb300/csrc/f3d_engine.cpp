@@ -18,11 +18,13 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cstdio>
 #include <cstring>
 #include <map>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 namespace f3d {
@@ -105,8 +107,9 @@ struct f3d_engine {
   // Kernel times (start, end) of the last forward, filter + inverse (or filter)
   // and overlap-add (or tensor-core inverse).
   KernelClock* d_clk = nullptr;
+  uint64_t clk_runs[3] = {};  // launches of each so far
   bool fwd_timed = false, proc_timed = false;
-  cudaStream_t side = nullptr;  // for work beside the caller's stream (zero_now)
+  cudaStream_t side = nullptr;  // for work beside the caller's stream (zero_now, read_clocks)
 
   int fail(int code, const std::string& msg) {
     err = msg;
@@ -252,6 +255,7 @@ int run_forward(f3d_engine* e, int fn, const uint8_t* dsrc, long long pitch, int
     retire(e, spec);
     return e->cuda_fail(ce, "the forward transform launch");
   }
+  e->clk_runs[0]++;
   return F3D_OK;
 }
 
@@ -331,18 +335,21 @@ int run_process(f3d_engine* e, const int* window, int n, uint8_t* ddst, long lon
   if (e->fused) {
     // The fused launch (tensor-core form: filter, then inverse) writes the packed plane.
     SweepArgs sa = sweep_args(e, a, ddst, pitch, fmt);
-    sa.clk = e->d_clk + 2;
-    sa.clk2 = e->d_clk + 4;
+    sa.clk = e->d_clk + 1;
+    sa.clk2 = e->d_clk + 2;
     e->test_skip = false;
     cudaError_t ce = e->inv_form == F3D_FORM_TC ? launch_sweep_tc_batch(&sa, 1, e->tune, e->stream)
                                                 : launch_sweep(e->inv_form, sa, e->stream);
     e->proc_timed = true;
     if (ce != cudaSuccess) return e->cuda_fail(ce, "the fused filter/inverse/overlap-add launch");
+    e->clk_runs[1]++;
+    if (e->inv_form == F3D_FORM_TC) e->clk_runs[2]++;
     return F3D_OK;
   }
-  a.clk = e->d_clk + 2;
+  a.clk = e->d_clk + 1;
   cudaError_t ce = launch_filter_inverse(e->inv_form, a, e->stream);
   if (ce != cudaSuccess) return e->cuda_fail(ce, "the filter/inverse launch");
+  e->clk_runs[1]++;
   if (a.kalman_init) e->kalman_first = false;
   OlaArgs o{};
   o.g = a.g;
@@ -353,10 +360,11 @@ int run_process(f3d_engine* e, const int* window, int n, uint8_t* ddst, long lon
   o.chroma_norm = e->cnorm;
   o.inv_norm = e->inv_norm;
   o.max_pix = e->max_pix;
-  o.clk = e->d_clk + 4;
+  o.clk = e->d_clk + 2;
   ce = launch_ola(o, e->stream);
   e->proc_timed = true;
   if (ce != cudaSuccess) return e->cuda_fail(ce, "the overlap-add launch");
+  e->clk_runs[2]++;
   return F3D_OK;
 }
 
@@ -369,27 +377,36 @@ cudaError_t zero_now(void* p, size_t n, cudaStream_t side) {
 }
 
 constexpr int kClocks = 3;
-constexpr size_t kClockBytes = 2 * kClocks * sizeof(KernelClock);
+constexpr size_t kClockBytes = kClocks * sizeof(KernelClock);
 // Bytes of an engine's input plane and its clocks.
 size_t in_bytes(const f3d_plane_geom& g) { return ((size_t)g.width * g.height * 4 + 15) / 16 * 16 + kClockBytes; }
 
-// Milliseconds of n kernels from their clocks, read once the work queued on st
-// is done (wait: waited for; else false when it is not). -1 where a kernel has
-// not run.
-bool read_clocks(const KernelClock* d, int n, cudaStream_t st, bool wait, float* ms) {
+// Milliseconds of n kernels from their clocks, runs[i] of whose launches have
+// been queued on st: -1 where one has not run, or where the last has not ended,
+// whatever else is queued on st. The clocks are copied on a stream of their own:
+// twice, because the adds of a CTA to its clock may land in either order.
+// Launches that were captured run as often as their graph does: with st idle
+// runs[i] is what the clock has counted. False: a copy failed. *was_idle
+// (optional): st was idle before the copies.
+bool read_clocks(const KernelClock* d, int n, uint64_t* runs, cudaStream_t st, cudaStream_t side, float* ms,
+                 bool* was_idle = nullptr) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone ||
-      (wait ? cudaStreamSynchronize(st) : cudaStreamQuery(st)) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
+  const bool idle = cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
+                    cudaStreamQuery(st) == cudaSuccess;
+  cudaGetLastError();
+  if (was_idle) *was_idle = idle;
+  KernelClock first[kClocks], t[kClocks];
+  for (KernelClock* to : {first, t})
+    if (cudaMemcpyAsync(to, d, n * sizeof(KernelClock), cudaMemcpyDeviceToHost, side) != cudaSuccess ||
+        cudaStreamSynchronize(side) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+  for (int i = 0; i < n; i++) {
+    if (idle) runs[i] = first[i].runs >> 32;
+    const bool ended = first[i].runs == runs[i] << 32;
+    ms[i] = ended && t[i].start && t[i].end >= t[i].start ? (t[i].end - t[i].start) * 1e-6f : -1.0f;
   }
-  KernelClock t[2 * kClocks];
-  if (cudaMemcpyAsync(t, d, 2 * n * sizeof(KernelClock), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  for (int i = 0; i < n; i++) ms[i] = t[2 * i] && t[2 * i + 1] >= t[2 * i] ? (t[2 * i + 1] - t[2 * i]) * 1e-6f : -1.0f;
   return true;
 }
 
@@ -830,12 +847,12 @@ int f3d_last_kernel_ms(f3d_engine* e, float* ms) {
   ms[0] = ms[1] = ms[2] = -1.0f;
   if (!e->fwd_timed && !e->proc_timed) return F3D_OK;
   float t[kClocks];
-  if (!read_clocks(e->d_clk, kClocks, e->stream, false, t)) return F3D_OK;  // not finished yet
+  if (!read_clocks(e->d_clk, kClocks, e->clk_runs, e->stream, e->side, t)) return F3D_OK;
   if (e->fwd_timed) ms[0] = t[0];
   if (e->proc_timed) {
     ms[1] = t[1];
     // The fused fast form has one kernel.
-    ms[2] = e->fused && e->inv_form != F3D_FORM_TC ? 0.0f : t[2];
+    ms[2] = e->fused && e->inv_form != F3D_FORM_TC ? std::min(t[1], 0.0f) : t[2];
   }
   return F3D_OK;
 }
@@ -867,6 +884,7 @@ struct f3d_batch {
   // Kernel times of the last step run outside a graph: filter (fast form: the
   // fused sweep) and inverse.
   KernelClock* clk = nullptr;
+  uint64_t clk_runs[2] = {};  // launches of each so far
   bool ktimed = false;
   // Entries whose engine appeared earlier in the batch (one more output of
   // that plane per step) have block images and seam rows of their own.
@@ -1069,10 +1087,14 @@ int f3d_batch_step(f3d_batch* b, const int* fns, const void* const* dev_src, con
     cudaStreamIsCapturing(b->stream, &cs);
     const bool timed = cs == cudaStreamCaptureStatusNone;
     sa[0].clk = timed ? b->clk : nullptr;
-    sa[0].clk2 = timed ? b->clk + 2 : nullptr;
+    sa[0].clk2 = timed ? b->clk + 1 : nullptr;
     const cudaError_t ce = b->fast ? launch_sweep_fast_batch(sa, ns, b->stream)
                                    : launch_sweep_tc_batch(sa, ns, t, b->stream, after_filter);
-    if (timed && ce == cudaSuccess) b->ktimed = true;
+    if (timed && ce == cudaSuccess) {
+      b->ktimed = true;
+      b->clk_runs[0]++;
+      b->clk_runs[1] += !b->fast;
+    }
     return ce;
   };
   auto forwards = [&](const TcTune& t, cudaStream_t st) -> cudaError_t {
@@ -1199,7 +1221,13 @@ int f3d_batch_last_kernel_ms(f3d_batch* b, float* ms) {
   if (!b->ktimed) return batch_fail(b, F3D_E_STATE, "FFT3DCL: no batch step with outputs ran outside a CUDA graph");
   cudaSetDevice(b->eng[0]->device);
   float t[2];
-  if (!read_clocks(b->clk, 2, b->stream, true, t)) return batch_fail(b, F3D_E_CUDA, "FFT3DCL: batch kernel timing failed");
+  for (;;) {
+    bool idle;
+    const bool read = read_clocks(b->clk, 2, b->clk_runs, b->stream, b->side, t, &idle);
+    if (read && t[0] >= 0.0f && (b->fast || t[1] >= 0.0f)) break;
+    if (!read || idle) return batch_fail(b, F3D_E_CUDA, "FFT3DCL: batch kernel timing failed");
+    std::this_thread::sleep_for(std::chrono::microseconds(20));
+  }
   ms[0] = t[0];
   ms[1] = b->fast ? 0.0f : t[1];  // the fused fast form has one kernel
   return F3D_OK;

@@ -20,9 +20,14 @@ struct Geo {
   int xoff, xstep, yoff, ystep;
 };
 
-// Device times of a kernel: [0] when its first CTA started, [1] when its last
-// one ended, in nanoseconds of the GPU's global timer. Null: not timed.
-using KernelClock = unsigned long long;
+// Device times of a kernel, in nanoseconds of the GPU's global timer, and how
+// far it is: the launches that have started, in the high 32 bits, plus the CTAs
+// still to end, so that the low bits are 0 when none of it runs. Null: not timed.
+struct KernelClock {
+  unsigned long long start;  // its first CTA past the wait for the kernel ahead
+  unsigned long long end;    // thread 0 of its last CTA done
+  unsigned long long runs;
+};
 
 // Sample formats of the raw planes.
 enum Fmt : int { FMT_F32 = 0, FMT_U8 = 8, FMT_U16 = 16 };

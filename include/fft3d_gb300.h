@@ -209,8 +209,8 @@ int f3d_prune(f3d_engine* e, int lo, int hi);
  * wait; the outputs queued since are invalid); the report clears it. */
 int f3d_synchronize(f3d_engine* e);
 /* Device time of the kernels of the last forward / process calls in ms,
- * taken by the kernels on the GPU's global timer (valid after f3d_synchronize;
- * -1 while the engine's stream has work queued):
+ * taken by the kernels on the GPU's global timer (-1 for a kernel that has not
+ * run or not ended; other work queued on the engine's stream does not matter):
  * ms[0] forward transform;
  * ms[1] filter + inverse (separate kernels), the whole sweep (fused fast
  *       form) or the filter kernel (tensor-core form);
