@@ -31,8 +31,9 @@ __host__ __device__ constexpr int bit_reverse(int i, int bits) {
   return r;
 }
 
-// Every kernel: grid_wait before the first access to memory that another
-// kernel writes or reads (launch_kernel), grid_go as early as its CTAs hold
+// Every kernel that may start before the one ahead has ended (launch_kernel; all
+// but f3d_k_big.cu's): grid_wait before the first access to memory that another
+// kernel writes or reads, grid_go as early as its CTAs hold
 // what they need to finish; in the kernels with tensor memory after its
 // allocation, which a successor's waiting CTA could otherwise take first.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -13,6 +13,16 @@
 // scale by 1/n. The butterflies of one stage are independent, so the result
 // does not depend on which lane computes which; with --fmad=false the bits
 // equal the reference CPU backend's.
+//
+// These kernels start when the one ahead has ended (launch_kernel, overlap
+// false), so they have no grid_wait. Their CTAs are few, long and about one to
+// an SM: started while the one ahead still ran, they took the places that were
+// free just then, several on some SMs and none on others. Queued passes, before
+// the kernels overlapped / overlapped / now: 640x360 128x64 185, 275, 173 us;
+// 854x480 64x256 364, 615, 350 and 512x512 4.39, 5.22, 4.28 ms (24 blocks);
+// 1080p 128x128 620, 755, 593. A plane of 8 blocks gives back 2 % of 10 (154,
+// 138, 141). The bound of kBigCtas keeps k_inverse_big from spilling (24 bytes
+// at the same 40 registers without it; 1080p 64x256 717 -> 690).
 #include "f3d_device.cuh"
 
 namespace f3d {
@@ -21,6 +31,7 @@ namespace {
 constexpr int kBigThreads = 256;
 constexpr int kBigWarps = kBigThreads / 32;
 constexpr int kBigMax = 512;
+constexpr int kBigCtas = 6;  // CTAs per SM: as many as shared memory holds (kBigSmem)
 
 __device__ __forceinline__ int log2_int(int n) {
   int l = 0;
@@ -77,7 +88,7 @@ __device__ __forceinline__ void load_twiddles(const float2* twr, const float2* t
 // centering, analysis window (src/cpu/reference.cpp:140-159); row transforms
 // keeping fbw columns, then the fbw column transforms
 // (src/cpu/fft.cpp:68-86), in place in the block's half spectrum.
-__global__ void __launch_bounds__(kBigThreads) k_forward_big(const __grid_constant__ FwdArgs a) {
+__global__ void __launch_bounds__(kBigThreads, kBigCtas) k_forward_big(const __grid_constant__ FwdArgs a) {
   extern __shared__ float2 sm_big[];
   const int bw = a.g.bw, bh = a.g.bh, fbw = bw / 2 + 1;
   const int lbw = log2_int(bw), lbh = log2_int(bh);
@@ -85,8 +96,6 @@ __global__ void __launch_bounds__(kBigThreads) k_forward_big(const __grid_consta
   float2* buf = sm_big + w * kBigMax;
   float2* twr = sm_big + kBigWarps * kBigMax;
   float2* twc = twr + kBigMax / 2;
-  grid_go();
-  grid_wait();
   stamp_start(a.clk);
   load_twiddles(a.twr, a.twc, bw, bh, twr, twc);
   const int b = blockIdx.x;
@@ -124,7 +133,7 @@ __global__ void __launch_bounds__(kBigThreads) k_forward_big(const __grid_consta
 // (bh x bw complex), Hermitian completion and column inverse transforms,
 // row inverse transforms, real part times the synthesis window
 // (src/cpu/reference.cpp:246-430, src/cpu/fft.cpp:88-119).
-__global__ void __launch_bounds__(kBigThreads) k_inverse_big(const __grid_constant__ InvArgs a) {
+__global__ void __launch_bounds__(kBigThreads, kBigCtas) k_inverse_big(const __grid_constant__ InvArgs a) {
   extern __shared__ float2 sm_big[];
   const int bw = a.g.bw, bh = a.g.bh, fbw = bw / 2 + 1, ps = fbw * bh;
   const int lbw = log2_int(bw), lbh = log2_int(bh);
@@ -132,8 +141,6 @@ __global__ void __launch_bounds__(kBigThreads) k_inverse_big(const __grid_consta
   float2* buf = sm_big + w * kBigMax;
   float2* twr = sm_big + kBigWarps * kBigMax;
   float2* twc = twr + kBigMax / 2;
-  grid_go();
-  grid_wait();
   stamp_start(a.clk);
   load_twiddles(a.twr, a.twc, bw, bh, twr, twc);
   const int b = blockIdx.x;
@@ -180,6 +187,7 @@ __global__ void __launch_bounds__(kBigThreads) k_inverse_big(const __grid_consta
 }
 
 constexpr size_t kBigSmem = sizeof(float2) * (kBigWarps * kBigMax + kBigMax);
+static_assert(kBigCtas * (kBigSmem + 1024) <= 228 * 1024, "CTAs per SM");
 
 }  // namespace
 
@@ -188,13 +196,13 @@ bool big_block(int bw, int bh) { return bw > 64 || bh > 64; }
 cudaError_t launch_forward_big(const FwdArgs& a, cudaStream_t st) {
   if (a.g.bw > kBigMax || a.g.bh > kBigMax || !a.twr || !a.twc) return cudaErrorInvalidValue;
   if (a.g.nb == 0) return cudaSuccess;
-  return launch_kernel(k_forward_big, a.g.nb, kBigThreads, kBigSmem, st, a);
+  return launch_kernel(k_forward_big, a.g.nb, kBigThreads, kBigSmem, st, a, false);
 }
 
 cudaError_t launch_inverse_big(const InvArgs& a, cudaStream_t st) {
   if (a.g.bw > kBigMax || a.g.bh > kBigMax || !a.twr || !a.twc || !a.work) return cudaErrorInvalidValue;
   if (a.g.nb == 0) return cudaSuccess;
-  return launch_kernel(k_inverse_big, a.g.nb, kBigThreads, kBigSmem, st, a);
+  return launch_kernel(k_inverse_big, a.g.nb, kBigThreads, kBigSmem, st, a, false);
 }
 
 }  // namespace f3d

@@ -285,8 +285,8 @@ int sm_count();
 void count_launch();
 
 // Launches a kernel of this library and counts it. Where the stream's previous
-// operation is a kernel, this one may start before that has ended: every kernel
-// waits for its predecessor (grid_wait) before it reads or writes anything that
+// operation is a kernel, this one may start before that has ended (overlap; with
+// false it starts then): every kernel waits for its predecessor (grid_wait) before it reads or writes anything that
 // another kernel may touch, and lets its successor start (grid_go) once each of
 // its CTAs runs and holds the tensor memory it needs: whatever has started can
 // end without a place that a waiting CTA holds. Launch latency and set-up then
