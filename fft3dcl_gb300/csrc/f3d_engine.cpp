@@ -21,10 +21,12 @@
 #include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <string>
 #include <thread>
+#include <utility>
 #include <vector>
 
 namespace f3d {
@@ -109,7 +111,7 @@ struct f3d_engine {
   KernelClock* d_clk = nullptr;
   uint64_t clk_runs[3] = {};  // launches of each so far
   bool fwd_timed = false, proc_timed = false;
-  cudaStream_t side = nullptr;  // for work beside the caller's stream (zero_now, read_clocks)
+  cudaStream_t side = nullptr;  // for work beside the caller's stream (zeroed, read_clocks)
 
   int fail(int code, const std::string& msg) {
     err = msg;
@@ -368,12 +370,15 @@ int run_process(f3d_engine* e, const int* window, int n, uint8_t* ddst, long lon
   return F3D_OK;
 }
 
-// Zeroes n bytes before it returns, on a stream without other work: neither the
-// legacy stream, which a non-blocking stream's first launch does not wait for,
-// nor the caller's, which may be recording a graph.
-cudaError_t zero_now(void* p, size_t n, cudaStream_t side) {
-  const cudaError_t e = cudaMemsetAsync(p, 0, n, side);
-  return e == cudaSuccess ? cudaStreamSynchronize(side) : e;
+// Zeroes the buffers that are there before it returns, on a stream without other
+// work, *side, that it creates: neither the legacy stream, which a non-blocking
+// stream's first launch does not wait for, nor the caller's, which may be
+// recording a graph.
+cudaError_t zeroed(cudaStream_t* side, std::initializer_list<std::pair<void*, size_t>> buffers) {
+  cudaError_t e = cudaStreamCreateWithFlags(side, cudaStreamNonBlocking);
+  for (const auto& b : buffers)
+    if (e == cudaSuccess && b.first) e = cudaMemsetAsync(b.first, 0, b.second, *side);
+  return e == cudaSuccess ? cudaStreamSynchronize(*side) : e;
 }
 
 constexpr int kClocks = 3;
@@ -548,8 +553,6 @@ int f3d_engine_create(const f3d_script_params* sp, const f3d_plane_geom* geom,
     if (ce != cudaSuccess) return finish_fail(e->cuda_fail(ce, "stream creation"));
     e->own_stream = true;
   }
-  ce = cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking);
-  if (ce != cudaSuccess) return finish_fail(e->cuda_fail(ce, "stream creation"));
   const size_t bwbh = (size_t)ip.bw * ip.bh;
   const size_t plane_bytes = (size_t)g.width * g.height * 4;
   auto up = [&](float** d, const std::vector<float>& h) -> cudaError_t {
@@ -571,15 +574,13 @@ int f3d_engine_create(const f3d_script_params* sp, const f3d_plane_geom* geom,
     e->tc_bytes = tab.size();
     if ((ce = e->alloc(&e->d_tc, e->tc_bytes)) != cudaSuccess ||
         (ce = cudaMemcpy(e->d_tc, tab.data(), tab.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (ce = e->alloc(&e->d_err, sizeof(int))) != cudaSuccess || (ce = zero_now(e->d_err, sizeof(int), e->side)) != cudaSuccess)
+        (ce = e->alloc(&e->d_err, sizeof(int))) != cudaSuccess)
       return finish_fail(e->cuda_fail(ce, "tensor-core table upload"));
   }
   // The clocks stand behind the input plane.
   if ((ce = e->alloc(&e->d_in, in_bytes(g))) != cudaSuccess || (ce = e->alloc(&e->d_out, plane_bytes)) != cudaSuccess)
     return finish_fail(e->cuda_fail(ce, "buffer allocation"));
   e->d_clk = reinterpret_cast<KernelClock*>(e->d_in + in_bytes(g) - kClockBytes);
-  if ((ce = zero_now(e->d_clk, kClockBytes, e->side)) != cudaSuccess)
-    return finish_fail(e->cuda_fail(ce, "buffer allocation"));
   if (ip.bm == 0) {
     const size_t nbin = (size_t)e->grid.nb * e->ps;
     if ((ce = e->alloc(&e->d_klast, sizeof(float2) * nbin)) != cudaSuccess ||
@@ -593,8 +594,7 @@ int f3d_engine_create(const f3d_script_params* sp, const f3d_plane_geom* geom,
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     sweep_plan(e->inv_form, geo, sms > 0 ? sms : 1, &e->sweep_strips, &e->sweep_segs);
     e->seam_floats = sweep_seam_floats(geo, e->sweep_strips, e->sweep_segs);
-    if (e->seam_floats && ((ce = e->alloc(&e->d_seam, sizeof(float) * e->seam_floats)) != cudaSuccess ||
-                           (ce = zero_now(e->d_seam, sizeof(float) * e->seam_floats, e->side)) != cudaSuccess))
+    if (e->seam_floats && (ce = e->alloc(&e->d_seam, sizeof(float) * e->seam_floats)) != cudaSuccess)
       return finish_fail(e->cuda_fail(ce, "seam buffer allocation"));
     if (e->inv_form == F3D_FORM_TC) {
       e->img_bytes = tc_image_bytes(geo);
@@ -621,6 +621,8 @@ int f3d_engine_create(const f3d_script_params* sp, const f3d_plane_geom* geom,
         (ce = e->alloc(&e->d_work, sizeof(float2) * bwbh * e->grid.nb)) != cudaSuccess)
       return finish_fail(e->cuda_fail(ce, "large-block buffer allocation"));
   }
+  ce = zeroed(&e->side, {{e->d_clk, kClockBytes}, {e->d_err, sizeof(int)}, {e->d_seam, sizeof(float) * e->seam_floats}});
+  if (ce != cudaSuccess) return finish_fail(e->cuda_fail(ce, "the buffers' clearing"));
   *out = e;
   return F3D_OK;
 }
@@ -952,14 +954,6 @@ int f3d_batch_create(f3d_engine* const* engines, int n, int flags, f3d_batch** o
   b->seam_bytes.assign(n, 0);
   b->repeat.assign(n, false);
   b->fast = e0->form == F3D_FORM_FAST;
-  if (cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming) != cudaSuccess ||
-      cudaMalloc(&b->clk, kClockBytes) != cudaSuccess || zero_now(b->clk, kClockBytes, b->side) != cudaSuccess) {
-    cudaGetLastError();
-    f3d_batch_destroy(b);
-    return fail_thread(F3D_E_CUDA, "FFT3DCL: batch stream creation failed");
-  }
   for (int i = 0; i < n; i++) {
     // An engine that appears k times enters k frames per step.
     int k = 0;
@@ -976,12 +970,22 @@ int f3d_batch_create(f3d_engine* const* engines, int n, int flags, f3d_batch** o
     b->img_bytes[i] = b->fast ? 0 : e->img_bytes;  // the fast sweep has no block images
     b->seam_bytes[i] = sizeof(float) * e->seam_floats;
     if ((b->img_bytes[i] && cudaMalloc(&b->img[i], b->img_bytes[i]) != cudaSuccess) ||
-        (b->seam_bytes[i] && (cudaMalloc(&b->seam[i], b->seam_bytes[i]) != cudaSuccess ||
-                              zero_now(b->seam[i], b->seam_bytes[i], b->side) != cudaSuccess))) {
+        (b->seam_bytes[i] && cudaMalloc(&b->seam[i], b->seam_bytes[i]) != cudaSuccess)) {
       cudaGetLastError();
       f3d_batch_destroy(b);
       return fail_thread(F3D_E_NOMEM, "FFT3DCL: batch output buffers could not be allocated");
     }
+  }
+  cudaError_t ce = cudaMalloc(&b->clk, kClockBytes);
+  if (ce == cudaSuccess) ce = zeroed(&b->side, {{b->clk, kClockBytes}});
+  for (int i = 0; i < n && ce == cudaSuccess; i++)
+    if (b->seam[i]) ce = cudaMemsetAsync(b->seam[i], 0, b->seam_bytes[i], b->side);
+  if (ce == cudaSuccess) ce = cudaStreamSynchronize(b->side);
+  if (ce != cudaSuccess || cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming) != cudaSuccess) {
+    cudaGetLastError();
+    f3d_batch_destroy(b);
+    return fail_thread(F3D_E_CUDA, "FFT3DCL: batch stream creation failed");
   }
   if (!b->fast) {  // the fast form has no launch shapes to tune
     std::lock_guard<std::mutex> lk(g_tune_mtx);
