@@ -47,16 +47,24 @@ __device__ __forceinline__ unsigned long long device_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
+// Reductions for the stamps; atomicAdd and atomicMax in their place cost a pass of
+// many CTAs more (4K fast, 16,900 of them: 264 us against 261).
+__device__ __forceinline__ void red_add(unsigned long long* p, unsigned long long v) {
+  asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void red_max(unsigned long long* p, unsigned long long v) {
+  asm volatile("red.relaxed.gpu.global.max.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 __device__ __forceinline__ void stamp_start(KernelClock* clk) {  // after grid_wait
   if (clk && (blockIdx.x | blockIdx.y | threadIdx.x) == 0) {
     clk->start = device_ns();
-    atomicAdd(&clk->runs, (1ull << 32) + gridDim.x * gridDim.y);
+    red_add(&clk->runs, (1ull << 32) + gridDim.x * gridDim.y);
   }
 }
 __device__ __forceinline__ void stamp_end(KernelClock* clk) {
   if (clk && threadIdx.x == 0) {
-    atomicMax(&clk->end, device_ns());
-    atomicAdd(&clk->runs, ~0ull);
+    red_max(&clk->end, device_ns());
+    red_add(&clk->runs, ~0ull);
   }
 }
 
