@@ -24,8 +24,8 @@ struct Geo {
 // far it is: the launches that have started, in the high 32 bits, plus the CTAs
 // still to end, so that the low bits are 0 when none of it runs. Null: not timed.
 struct KernelClock {
-  unsigned long long start;  // its first CTA past the wait for the kernel ahead
-  unsigned long long end;    // thread 0 of its last CTA done
+  unsigned long long start;  // its first CTA past its set-up and the wait for the kernel ahead
+  unsigned long long end;    // thread 0 of its last CTA done, bulk stores read but not yet written
   unsigned long long runs;
 };
 
@@ -215,7 +215,7 @@ cudaError_t launch_forward_tc(const TcFwdArgs& a, cudaStream_t st);
 // the prefix of per-plane CTA (forward: block-group) counts. Passed by value
 // as kernel parameters, so a captured CUDA graph is re-pointed at the next
 // frame's buffers by updating its kernel nodes' parameters. At 16 planes a
-// SweepBatch is about 13.5 KB: above the classic 4 KB parameter limit, within
+// SweepBatch is about 14.5 KB: above the classic 4 KB parameter limit, within
 // the 32 KB that CUDA 12.1+ allows for __grid_constant__ parameters.
 constexpr int kMaxBatch = 16;
 struct TcFwdBatch {
@@ -252,7 +252,9 @@ struct FilterBatch {
 // Launch shape of the tensor-core kernels, picked by the autotuner.
 struct TcTune {
   int fwd_ctas_per_sm = 3;  // persistent forward grid: CTAs per SM (1 to 3; 2 at most with the split)
-  int filter_minb = 5;      // filter kernel variant: spectra loads of one block in flight, or (4, 3) of two
+  // Filter CTAs per SM: 5, the spectra loads of one block in flight, or 4 (and 3, a
+  // shape without a kernel of its own), of two; 16 x 16 blocks differ in registers only.
+  int filter_minb = 5;
 };
 cudaError_t launch_forward_tc_batch(const TcFwdArgs* planes, int n, const TcTune& t, cudaStream_t st);
 // after_filter (may be null) is recorded on st between the filter and the

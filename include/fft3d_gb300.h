@@ -210,7 +210,11 @@ int f3d_prune(f3d_engine* e, int lo, int hi);
 int f3d_synchronize(f3d_engine* e);
 /* Device time of the kernels of the last forward / process calls in ms,
  * taken by the kernels on the GPU's global timer (-1 for a kernel that has not
- * run or not ended; other work queued on the engine's stream does not matter):
+ * run or not ended; other work queued on the engine's stream does not matter).
+ * A time runs from the kernel's first CTA, once the kernel ahead has ended and
+ * its own set-up is done, to the last instruction of the first thread of its
+ * last CTA: a few microseconds less than events on either side would give,
+ * without the launch and the last stores' way to memory.
  * ms[0] forward transform;
  * ms[1] filter + inverse (separate kernels), the whole sweep (fused fast
  *       form) or the filter kernel (tensor-core form);
@@ -296,13 +300,14 @@ int f3d_batch_step(f3d_batch* b, const int* fns, const void* const* dev_src, con
 /* Launch shape in use; returns 1 when the autotuner has chosen it. */
 int f3d_batch_tune(f3d_batch* b, int* fwd_ctas_per_sm, int* filter_minb);
 /* Pins the launch shape (the autotuner then keeps it): fwd_ctas_per_sm 1 to
- * 3 forward CTAs per SM, filter_minb 3..5 filter CTAs per SM. Every shape gives the same
- * results. F3D_E_PARAM for any other shape. */
+ * 3 forward CTAs per SM, filter_minb 4 or 5 filter CTAs per SM (3 is accepted, and
+ * reported by f3d_batch_tune as it was set, and runs the kernel of 4). Every shape
+ * gives the same results. F3D_E_PARAM for any other shape. */
 int f3d_batch_set_tune(f3d_batch* b, int fwd_ctas_per_sm, int filter_minb);
 /* Device times (ms) of the last step with outputs that ran outside a CUDA
  * graph (steps replayed as a graph are not timed): ms[0] the filter kernel,
  * ms[1] the inverse + overlap-add kernel (fast form: ms[0] the fused sweep,
- * ms[1] 0). Waits for that step.
+ * ms[1] 0), as f3d_last_kernel_ms counts them. Waits for that step.
  * F3D_E_STATE when no such step ran. */
 int f3d_batch_last_kernel_ms(f3d_batch* b, float* ms);
 
