@@ -221,8 +221,11 @@ __device__ __forceinline__ BinTables bin_tables(const FilterArgs& a, int i) {
 // Fixes a kernel's copy of the filter arguments to the switches it is built
 // for. Read at run time they cost about ten instructions of branches per bin,
 // and table loads behind a branch cannot be issued with the spectra's.
-// Products that are added later are rounded by themselves (prod), so the bits
-// are the same.
+// The bits are the same: the products of the degrid sample and of the gains are
+// rounded by themselves (prod) or are those of an explicit fmaf; the others that
+// are added later (3 * d, the factors of the 3-point temporal transform, the
+// sharpening's factor * root) the compiler fuses in every set alike, which the
+// tests hold it to, comparing the sets bit for bit.
 template <int SW>
 __device__ __forceinline__ void fix_switches(FilterArgs& f) {
   if constexpr (SW != kSwAny) {
