@@ -42,17 +42,16 @@ WORKLOAD = ("3840x2160 YUV420P10 luma, sigma=3 bt=4 bw=bh=32 ow=oh=16 sharpen=0.
             "48-frame seeded clip, one output frame per step")
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant
-# kernel from one ncu capture of this workload (launch list of
-# `bench.py --steps 2 --warmup 3`), keyed by form; None until captured.
-NCU_TRAFFIC = {"tc": 571806464 + 130638592}
+# kernel from one ncu capture of this workload, one output per launch
+# (profiles/kernels_of_the_cases.md), keyed by form; None until captured.
+NCU_TRAFFIC = {"tc": 679800000 + 107300000}
 # The same for the filter launch of a batch step of k consecutive outputs
 # (k -> bytes): captured on the 1920x1080 case of this workload (`--size
 # 1920x1080 --steps 1 --warmup 3 --no-cpu --serve-streams 0 --no-yuv
-# --compare tc --outputs-per-step k`, mean of the k-output launches; k=4:
-# 260.2 MB read + 124.4 MB written, k=8: 410.5 + 286.0 MB, k=10 (with the
-# filter's block images): 495.5 + 305.5 MB) and scaled to
-# 3840x2160 by the block count (32912 / 8540).
-NCU_TRAFFIC_BATCH = {4: 1002927925 + 479516689, 8: 1581975962 + 1102231724, 10: 1909589696 + 1177355504}
+# --no-configs --compare tc --outputs-per-step k`, mean of the k-output launches
+# of the 5-CTA kernel; k=4: 259.9 MB read + 103.3 MB written, k=8: 408.4 + 236.3,
+# k=10: 482.4 + 304.5) and scaled to 3840x2160 by the block count (32912 / 8540).
+NCU_TRAFFIC_BATCH = {4: 1001773452 + 398258323, 8: 1574033742 + 910706642, 10: 1859026998 + 1173501639}
 # Consecutive outputs per batch step of the tensor-core headline (4K sweeps:
 # ten beat eight and twelve); its traffic must be in NCU_TRAFFIC_BATCH.
 DEFAULT_OUTPUTS_PER_STEP = 10
@@ -599,7 +598,7 @@ def run_gpu(args, rank, world, local_rank):
         clk = clocks.stop() if clocks else None
         ms = e0.elapsed_time(e1)
         # Per-kernel device time over the same number of steps (a synchronize
-        # after each step so that the engine's events can be read).
+        # after each step: the times are those of the last one).
         kt = np.zeros(3)
         for _ in range(args.steps):
             step_engine(n)
@@ -612,8 +611,8 @@ def run_gpu(args, rank, world, local_rank):
             forms_extra["tune"] = tune
             batch.close()
             # The batch step's own filter and inverse launches (k outputs per
-            # launch), same launch shape, without a graph so that events
-            # bracket them, and with the forwards outside the step so that no
+            # launch), same launch shape, without a graph so that they are
+            # timed, and with the forwards outside the step so that no
             # concurrent kernel shares the GPU while they run.
             tb = F.Batch([eng] * k, graph=False, autotune=False)
             tb.set_tune(tune["fwd_ctas_per_sm"], tune["filter_minb"])
@@ -756,7 +755,9 @@ def run_gpu(args, rank, world, local_rank):
     ab = algorithmic_bytes(info.nblocks, info.fbw, ip.bh, bt)
     peak, peak_kind = load_peaks()
     inv_ms = float(kt[1])
-    # The dominant kernel, timed by itself on the GPU: the tensor-core
+    # The dominant kernel, by its own stamps (from its first CTA past the wait
+    # for the kernel ahead to thread 0 of its last CTA, copies still under way
+    # and set-up not counted: some us less than an event on either side): the tensor-core
     # filter (window spectra in; its block images are an intermediate), the
     # fused fast-form sweep (window spectra in, packed plane out) or, unfused,
     # the filter+inverse kernel (window spectra in).
@@ -765,7 +766,7 @@ def run_gpu(args, rank, world, local_rank):
         kt_names = ("forward", "filter", "inverse_overlap_add")
     elif info.fused:
         kname, kbytes = "k_sweep_fast (filter+inverse+overlap-add+pack)", ab["filter_inverse"] + ab["plane"]
-        kt_names = ("forward", "sweep", "seam_merge")
+        kt_names = ("forward", "sweep")
     else:
         kname, kbytes = "k_inverse (filter+inverse)", ab["filter_inverse"]
         kt_names = ("forward", "filter_inverse", "overlap_add")
@@ -796,8 +797,8 @@ def run_gpu(args, rank, world, local_rank):
                    "form": args.form, "parallelism": f"replicas x{world}",
                    "inputs": f"clip resident in HBM ({len(frames)} x 16.6 MB)",
                    "l2": "working set per step ~750 MB: four 143 MB window spectra, larger than the 129 MB L2"},
-        "kernel_ms": {kt_names[i]: round(float(kt[i]), 4) for i in range(3)},
-        "batch_kernel_ms": bkt and {"filter": round(bkt[0], 4), "inverse_overlap_add_merge": round(bkt[1], 4),
+        "kernel_ms": {name: round(float(t), 4) for name, t in zip(kt_names, kt)},
+        "batch_kernel_ms": bkt and {"filter": round(bkt[0], 4), "inverse_overlap_add": round(bkt[1], 4),
                                     "outputs_per_launch": kframes},
         "forms": forms,
         "roofline": roof,
