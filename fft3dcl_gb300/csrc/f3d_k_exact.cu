@@ -10,8 +10,9 @@
 // one thread per kept column; the inverse one thread per column (Hermitian
 // completion on the fly), then one thread per row. Shared memory carries the
 // transposes; a CTA of 128 threads works on 128/TPB blocks.
-// 64 x 64 blocks run their 64-point transforms on lane pairs instead
-// (k_forward_exact64, k_inverse_exact64: 128 threads per block).
+// 64 x 64 blocks run their 64-point transforms on lane pairs and groups of four
+// instead (k_forward_exact64, 128 threads per block; k_inverse_lanes, 256), the
+// inverse of 32 x 32 blocks on pairs (k_inverse_lanes, 64).
 #include "f3d_device.cuh"
 
 #ifndef F3D_BW

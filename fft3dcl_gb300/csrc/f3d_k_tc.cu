@@ -129,8 +129,9 @@ struct FwdSmem {
 };
 // CTAs per SM of the forward kernel: three fit in shared memory without the
 // split, two with it; the words of unaligned rows do not fit in the registers
-// of three (spilled registers cost more than the third CTA: 4K 10-bit 52 -> 60
-// us with 30 bytes of them).
+// of three (30 bytes spilled per thread cost more than the third CTA gave: 4K
+// 10-bit 52 -> 60 us). Aligned 16-bit rows of 32 x 32 blocks spill 16 bytes at
+// three, the other kernels none.
 constexpr int kFwdMaxCtasPerSm = 3;
 constexpr int fwd_ctas(bool split, bool aligned, int bps) { return split || (!aligned && bps == 2) ? 2 : kFwdMaxCtasPerSm; }
 
@@ -858,7 +859,10 @@ __global__ void __launch_bounds__(kTcThreads, MINB) k_filter_tc(const __grid_con
   const int b0 = local / rl * C::G, nvb = min(C::G, P.nblk - b0);
   const size_t gb0 = (size_t)b0 * C::PS;
   // The window spectra begin moving into L2 as whole runs (of shifted
-  // windows, only the newest frame: the others are an earlier output's).
+  // windows, only the newest frame: the others are an earlier output's). With
+  // one output of a large plane a fifth is read twice (4K bt=4: 680 MB of 573),
+  // probably because that is more than L2 keeps: five CTAs on 152 SMs ask for
+  // 106 MB beside 25 MB of images.
   if (tid < NF && (!((B.shifted >> pl) & 1) || tid == NF - 1))
     tc::prefetch_l2(reinterpret_cast<const uint8_t*>(P.f.s[tid]) + b0 * (size_t)BLK, nvb * BLK);
   // The current frame's DC of each block (the degrid correction's scale).
@@ -1408,8 +1412,9 @@ cudaError_t launch_sweep_n(const SweepBatch& B, int n, const TcTune& t, cudaStre
   if (after_filter && (e = cudaEventRecord(after_filter, st)) != cudaSuccess) return e;
   // Inverse + overlap-add: one CTA per (strip, segment) of every plane. It
   // starts within the filter but behind a batch's long one, where what is saved
-  // is little and its waiting CTAs cost more (ten 10-bit 4K outputs, 82,000
-  // filter CTAs: 1404 us, else 1388; three 1080p planes, 3,150: 106, else 108).
+  // is little and its waiting CTAs cost more (ten 10-bit 4K outputs, 41,140
+  // filter CTAs: 1404 us, else 1388; three 1080p planes, 1,597: 106, else 108;
+  // nothing between them was measured, so the line at eight waves is a choice).
   const bool overlap = n == 1 || l.grid <= 8 * 5 * sm_count();
   e = prepare(k_sweep_tc<N>, smem);
   if (e != cudaSuccess) return e;
