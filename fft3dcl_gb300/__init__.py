@@ -648,6 +648,8 @@ class Batch:
         if not n == len(lens) == len(fns) == len(srcs) == len(src_pitches) == len(dsts) == len(dst_pitches):
             return None
         wins = array("i", chain.from_iterable(windows))
+        if len(wins) != sum(lens):  # windows that can be gone through once
+            return None
         starts, at = [], wins.buffer_info()[0]
         for k in lens:
             starts.append(at)
