@@ -61,10 +61,20 @@ __device__ __forceinline__ void stamp_start(KernelClock* clk) {  // after grid_w
     red_add(&clk->runs, (1ull << 32) + gridDim.x * gridDim.y);
   }
 }
+// The CTA's number is read again in here: kept from the kernel's start for the
+// slot, it cost registers, and CTAs on an SM, in a dozen kernels. SPREAD: whether
+// the kernel's CTAs count in all slots (k_ola: in one, 4K 24 us, else 28).
+template <bool SPREAD = true>
 __device__ __forceinline__ void stamp_end(KernelClock* clk) {
   if (clk && threadIdx.x == 0) {
-    red_max(&clk->end, device_ns());
-    red_add(&clk->runs, ~0ull);
+    KernelClock::Slot* s = clk->slot;
+    if constexpr (SPREAD) {
+      uint32_t x;
+      asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(x));
+      s += x % KernelClock::kSlots;
+    }
+    red_max(&s->end, device_ns());
+    red_add(&s->done, 1);
   }
 }
 

@@ -384,7 +384,7 @@ cudaError_t zeroed(cudaStream_t* side, std::initializer_list<std::pair<void*, si
 constexpr int kClocks = 3;
 constexpr size_t kClockBytes = kClocks * sizeof(KernelClock);
 // Bytes of an engine's input plane and its clocks.
-size_t in_bytes(const f3d_plane_geom& g) { return ((size_t)g.width * g.height * 4 + 15) / 16 * 16 + kClockBytes; }
+size_t in_bytes(const f3d_plane_geom& g) { return ((size_t)g.width * g.height * 4 + 127) / 128 * 128 + kClockBytes; }
 
 // Milliseconds of n kernels from their clocks, runs[i] of whose launches have
 // been queued on st: -1 where one has not run, or where the last has not ended,
@@ -408,9 +408,14 @@ bool read_clocks(const KernelClock* d, int n, uint64_t* runs, cudaStream_t st, c
       return false;
     }
   for (int i = 0; i < n; i++) {
-    if (idle) runs[i] = first[i].runs >> 32;
-    const bool ended = first[i].runs == runs[i] << 32;
-    ms[i] = ended && t[i].start && t[i].end >= t[i].start ? (t[i].end - t[i].start) * 1e-6f : -1.0f;
+    unsigned long long done = 0, end = 0;
+    for (int s = 0; s < KernelClock::kSlots; s++) {
+      done += first[i].slot[s].done;
+      end = std::max(end, t[i].slot[s].end);
+    }
+    if (idle) runs[i] = (first[i].runs - done) >> 32;
+    const bool ended = first[i].runs - done == runs[i] << 32;
+    ms[i] = ended && t[i].start && end >= t[i].start ? (end - t[i].start) * 1e-6f : -1.0f;
   }
   return true;
 }

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(256) k_ola(const __grid_constant__ OlaArgs a) 
     for (int k = 0; k < V; k++) sum[k] += a.chroma_norm;
   if constexpr (V == 4) store_quad(a.dst + (long long)y * a.pitch, x, g.W, sum, a.fmt, a.inv_norm, a.max_pix);
   else store_sample(a.dst + (long long)y * a.pitch, x, sum[0], a.fmt, a.inv_norm, a.max_pix);
-  stamp_end(a.clk);
+  stamp_end<false>(a.clk);
 }
 
 }  // namespace
