@@ -181,6 +181,12 @@ __device__ __forceinline__ void filter_block(const InvArgs& a, int b, int t, flo
   }
 }
 
+// Blocks four wide or high (PS bins, TPB threads): at most three bins a thread,
+// all loaded together, and no prefetch of runs as short as 96 bytes (inverse, 4K
+// 10-bit bt=4, both / one bin at a time and prefetched / neither prefetched: 4 x 8
+// 225, 285, 260 us, 8 x 4 223, 272, 235, 4 x 32 410, 455, 466).
+constexpr bool small_block(int ps, int tpb) { return ps <= 3 * tpb; }
+
 // The temporal mode as a template argument (square blocks: one copy of the
 // filter for each mode, of which a launch runs one) or read per bin.
 template <bool KALMAN, bool BY_MODE, int PS, int TPB, int KB>
@@ -190,7 +196,7 @@ __device__ __forceinline__ void filter_block_any(const InvArgs& a, int b, int t,
   // with 1, 2, 3, 4 in flight: 32x32 bt=4 97.4, 97.6, 97.6, 104 us, bt=1 78, 76,
   // 75, 76; bt=3 64x64 on pairs 129.5, 129.6, 132, 137, 16x16 79, 81, 84, 86, 8x8 85, 86,
   // 89, 95).
-  constexpr int KN = TPB == 64 ? 3 : 1;
+  constexpr int KN = TPB == 64 ? 3 : (small_block(PS, TPB) ? 4 : 1);
   if constexpr (KALMAN) {
     filter_block<0, PS, TPB, KB>(a, b, t, F);
   } else if constexpr (BY_MODE) {
@@ -253,7 +259,7 @@ __global__ void __launch_bounds__(Cfg<BW, BH>::THREADS, Cfg<BW, BH>::INV_CTAS - 
   grid_go();
   grid_wait();
   stamp_start(a.clk);
-  if (!KALMAN && valid && t == 0) prefetch_window<C::PS>(a, b);
+  if (!KALMAN && !small_block(C::PS, C::TPB) && valid && t == 0) prefetch_window<C::PS>(a, b);
   if (valid) filter_block_any<KALMAN, BW == BH, C::PS, C::TPB, C::KB>(a, b, t, F);
   block_sync<C::TPB>();
   {
