@@ -1300,6 +1300,26 @@ struct FwdLaunch {
   size_t smem = 0;
   int ctas = 0;  // per SM
 };
+// Shared memory of which no more than `ctas` CTAs fit on an SM (228 KB, 1 KB of
+// it for each CTA).
+constexpr size_t smem_for_ctas(int ctas) { return 228 * 1024 / (ctas + 1) - 1024 + 128; }
+
+// Whether one plane's forward of 16 x 16 blocks asks for that much: its
+// persistent CTAs are placed where the kernel ahead leaves room first, and where
+// an SM holds more of them than the grid is meant to put there (8-bit 4 for 3,
+// 16-bit at two an SM 3; 10-bit and float no more), the first SMs to come free took
+// more and others were left with fewer. It pays once a CTA has a group and a
+// half: queued passes, bt=4, before the kernels overlapped / overlapped / now: 4K
+// 16-bit 293, 292, 266 us, 8-bit 327, 275, 256; 7680x4320 16-bit 1004, 1058, 940;
+// 1080p 16-bit 111, 93, 87; 720p 8-bit 74, 49.3, 48.3 (932 groups for 456 CTAs).
+// With fewer groups each has one and crowding costs nothing (960x540 8-bit, 534:
+// 33.2 us, else 34.1). In a batch of several planes the forward shares the SMs
+// with another kernel and takes what is there (8-bit 1080p, sixteen outputs: 769
+// us, else 784).
+bool spread_ctas(int n_planes, int fmt, int ctas, int groups) {
+  return n_planes == 1 && (fmt == FMT_U8 || (fmt == FMT_U16 && ctas == 2)) && 2 * groups >= 3 * ctas * sm_count();
+}
+
 template <int N>
 FwdLaunch forward_launch_n(const TcFwdArgs* planes, int n) {
   FwdLaunch l;
@@ -1311,6 +1331,8 @@ FwdLaunch forward_launch_n(const TcFwdArgs* planes, int n) {
   l.kernel = aligned ? forward_kernel<N, true>(fmt, split) : forward_kernel<N, false>(fmt, split);
   l.smem = split ? FwdSmem<N, true>::BYTES : FwdSmem<N, false>::BYTES;
   l.ctas = fwd_ctas(split, aligned, fmt == FMT_U16 ? 2 : 1);
+  if (N == 16 && spread_ctas(n, fmt, l.ctas, (planes[0].g.nb + TcCfg<N>::G - 1) / TcCfg<N>::G))
+    l.smem = std::max(l.smem, smem_for_ctas(l.ctas));
   return l;
 }
 FwdLaunch forward_launch(const TcFwdArgs* planes, int n) {
